@@ -5,9 +5,11 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 
 #include "field_kernels.cuh"
 #include "fields.hpp"
+#include "line_tables.hpp"
 
 namespace pmg {
 namespace {
@@ -22,7 +24,7 @@ template <int N, typename T> kern::Tab<N, T> tab_of(const Tables1D &t) {
     k.D[a] = (T)t.D[a];
   }
   for (int a = 0; a < N; ++a) k.W[a] = (T)t.W[a];
-  kern::fill_even_odd(k, t.S.data(), t.SD.data());
+  kern::fill_even_odd<N>(k, t.S.data(), t.SD.data());
   return k;
 }
 
@@ -63,8 +65,32 @@ template <typename K> int resident_grid(K kernel, int threads, size_t smem, int6
   return (int)std::max<int64_t>(1, std::min<int64_t>(work_blocks, resident));
 }
 
+// cells per block of the line kernels here: as the Laplace kernels (Q3 a warp per pair of cells,
+// elsewhere the lines of 5 or 3 cells in 4 or 5 warps)
+template <int N, bool WARP> using FieldShape =
+    std::conditional_t<N == 4 && WARP, kern::LineShape<4, 2, 8>,
+                       std::conditional_t<(N <= 5), kern::LineShape<N == 4 ? 8 : 5, 0, 4>, kern::LineShape<3, 0, 3>>>;
+
+template <int N, typename T, int MG> void mass_line_launch(const pmg_operator &op, const void *src, void *dst,
+                                                           cudaStream_t s) {
+  using SH = FieldShape<N, true>;
+  constexpr size_t smem = kern::mass_line_smem<N, T, SH>();
+  static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
+  const int64_t blocks = (op.n_cells + SH::CPB - 1) / SH::CPB;
+  kern::mass_line_kernel<N, T, MG, SH><<<(unsigned)blocks, kern::line_threads<N, SH>(), smem, s>>>(
+      line_tables<N, T>(), static_cast<const T *>(src), static_cast<T *>(dst), op.idx.as<uint32_t>(), op.geo.as<T>(),
+      op.coef.as<T>(), op.n_cells);
+  PMG_LAUNCH_CHECK();
+  op.launch_units[PMG_KERNEL_MASS] = op.n_cells;
+  op.launch_par[PMG_KERNEL_MASS] = blocks;
+}
+
 template <int N, typename T> void mass_launch(const pmg_operator &op, const void *src, void *dst,
                                               cudaStream_t s) {
+  if constexpr (kern::mass_line_layout(N)) {
+    if (op.mass_geom == 1) mass_line_launch<N, T, 1>(op, src, dst, s);
+    else mass_line_launch<N, T, 0>(op, src, dst, s);
+  } else {
   constexpr int CPW = kern::Layout<N>::CPW, CS = kern::Stride<N>::CELL;
   const size_t smem = size_t(kWarps) * CPW * CS * sizeof(T);
   const int64_t blocks = (op.n_groups + kWarps - 1) / kWarps;
@@ -84,6 +110,7 @@ template <int N, typename T> void mass_launch(const pmg_operator &op, const void
   }
   op.launch_units[PMG_KERNEL_MASS] = op.n_groups;
   PMG_LAUNCH_CHECK();
+  }
 }
 
 template <int N, typename T> void mass_diag_launch(const pmg_operator &op, void *diag, cudaStream_t s) {
@@ -108,17 +135,30 @@ template <int N, typename T> void mass_diag_launch(const pmg_operator &op, void 
 template <int N, typename T, int GEOM>
 void qp_form_geom(const pmg_operator &op, const void *u, const void *v, double alpha, double *out,
                   cudaStream_t s) {
-  constexpr int CPW = kern::Layout<N>::CPW, CS = kern::Stride<N>::CELL;
-  constexpr int W = 2; // warps per block
-  const size_t smem = size_t(W) * 6 * CPW * CS * sizeof(T);
-  auto k = kern::qp_form_slab_kernel<N, T, GEOM>;
-  const int grid = resident_grid(k, 32 * W, smem, (op.n_groups + W - 1) / W);
-  k<<<grid, 32 * W, smem, s>>>(tab_of<N, T>(cached_tables(op.degree)), static_cast<const T *>(u),
-                               static_cast<const T *>(v), out, op.idx.as<uint32_t>(), op.geo.as<T>(),
-                               op.coef.as<T>(), op.n_groups, op.n_cells, alpha);
-  PMG_LAUNCH_CHECK();
-  op.launch_units[PMG_KERNEL_QP_FORM] = op.n_groups;
-  op.launch_par[PMG_KERNEL_QP_FORM] = (int64_t)grid * W;
+  if constexpr (N >= 4) {
+    using SH = FieldShape<N, false>;
+    constexpr size_t smem = kern::line_smem<N, T, SH>();
+    static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
+    const int64_t blocks = (op.n_cells + SH::CPB - 1) / SH::CPB;
+    kern::qp_form_line_kernel<N, T, GEOM, SH><<<(unsigned)blocks, kern::line_threads<N, SH>(), smem, s>>>(
+        line_tables<N, T>(), static_cast<const T *>(u), static_cast<const T *>(v), out, op.idx.as<uint32_t>(),
+        op.geo.as<T>(), op.coef.as<T>(), (T)op.affine[0], (T)op.affine[1], (T)op.affine[2], op.n_cells, alpha);
+    PMG_LAUNCH_CHECK();
+    op.launch_units[PMG_KERNEL_QP_FORM] = op.n_cells;
+    op.launch_par[PMG_KERNEL_QP_FORM] = blocks;
+  } else {
+    constexpr int CPW = kern::Layout<N>::CPW, CS = kern::Stride<N>::CELL;
+    constexpr int W = 2; // warps per block
+    const size_t smem = size_t(W) * 6 * CPW * CS * sizeof(T);
+    auto k = kern::qp_form_slab_kernel<N, T, GEOM>;
+    const int grid = resident_grid(k, 32 * W, smem, (op.n_groups + W - 1) / W);
+    k<<<grid, 32 * W, smem, s>>>(tab_of<N, T>(cached_tables(op.degree)), static_cast<const T *>(u),
+                                 static_cast<const T *>(v), out, op.idx.as<uint32_t>(), op.geo.as<T>(),
+                                 op.coef.as<T>(), op.n_groups, op.n_cells, alpha);
+    PMG_LAUNCH_CHECK();
+    op.launch_units[PMG_KERNEL_QP_FORM] = op.n_groups;
+    op.launch_par[PMG_KERNEL_QP_FORM] = (int64_t)grid * W;
+  }
 }
 
 template <int N, typename T>

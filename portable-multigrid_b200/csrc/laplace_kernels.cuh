@@ -1,10 +1,13 @@
-// Sum-factorized cell kernels of the continuous Q_p Laplace operator for sm_100a.
+// Slab kernels of the continuous Q_p Laplace operator for sm_100a: the vmult at degrees 1 and 2
+// with stored geometry or a coefficient, and the diagonal at every degree.  (The vmult at
+// degrees 3 to 6, and of axis-aligned cells without a coefficient at every degree, is in
+// line_kernels.cuh: one lane per line of a cell.  At degrees 1 and 2 a line is too short: full
+// geometry at 64^3, FP64 Q2 82 against 101 us, FP32 Q2 48 against 62 us with lines.)
 //
 // What they compute is the BK3 cell operator of the reference
 // (include/kernels/bk3_kokkos_kernel.h:25-746): per cell gather the nodal values (Dirichlet
 // entries read as 0), interpolate to the Gauss points, take collocation gradients, apply
-// the symmetric geometry tensor G, integrate against the gradients and scatter-add.  How
-// they compute it is laid out for the B200:
+// the symmetric geometry tensor G, integrate against the gradients and scatter-add.
 //
 //  * A warp owns a group of CPW = floor(32/N) consecutive cells (N = p+1 nodes per
 //    direction), N lanes per cell.  Lane s of a cell works on a slab of the cell: the
@@ -18,8 +21,8 @@
 //                 a = Sy^T SDx^T fx + SDy^T Sx^T fy,  c = Sy^T Sx^T fz
 //        Y-slab:  out = Sz^T a + SDz^T c
 //    No block-wide barrier is used; warps are independent.
-//  * The index map and G are stored lane-contiguous per group ([group][point][lane]), so
-//    every load of them is a fully coalesced warp access; G is column-major per group (one
+//  * The index map and the geometry are stored lane-contiguous per group ([group][point][lane]),
+//    so every load of them is a fully coalesced warp access; G is column-major per group (one
 //    contiguous chunk per x point). The ring variant streams the columns of the current
 //    group through a two-slot shared-memory ring filled by TMA bulk copies one column ahead;
 //    the direct-load variant bulk-prefetches the next group's G into L2
@@ -58,21 +61,22 @@ template <int N, typename T> struct Tab {
   EvenOdd<N, T> eST, eSDT; // their transposes (input point q, output node i)
 };
 
-// fill the even/odd tables of `tab` from the row-major N x N tables S and SD (host)
-template <int N, typename T> inline void fill_even_odd(Tab<N, T> &tab, const double *S, const double *SD) {
+// even/odd table of the matrix M(i, q) (host)
+template <int N, typename T, typename F> inline void fill_even_odd(EvenOdd<N, T> &e, F &&M) {
   constexpr int H = N / 2, Q = (N + 1) / 2;
-  auto fill = [&](EvenOdd<N, T> &e, auto M) {
-    for (int i = 0; i < H; ++i)
-      for (int q = 0; q < Q; ++q) {
-        e.A[i * Q + q] = (T)(0.5 * (M(i, q) + M(N - 1 - i, q)));
-        e.B[i * Q + q] = (T)(0.5 * (M(i, q) - M(N - 1 - i, q)));
-      }
-    for (int q = 0; q < Q; ++q) e.C[q] = (N & 1) ? (T)M(H, q) : T(0);
-  };
-  fill(tab.eS, [&](int i, int q) { return S[i * N + q]; });
-  fill(tab.eSD, [&](int i, int q) { return SD[i * N + q]; });
-  fill(tab.eST, [&](int r, int k) { return S[k * N + r]; });
-  fill(tab.eSDT, [&](int r, int k) { return SD[k * N + r]; });
+  for (int i = 0; i < H; ++i)
+    for (int q = 0; q < Q; ++q) {
+      e.A[i * Q + q] = (T)(0.5 * (M(i, q) + M(N - 1 - i, q)));
+      e.B[i * Q + q] = (T)(0.5 * (M(i, q) - M(N - 1 - i, q)));
+    }
+  for (int q = 0; q < Q; ++q) e.C[q] = (N & 1) ? (T)M(H, q) : T(0);
+}
+// those of S and SD (row-major N x N) and their transposes into tab.eS, eSD, eST, eSDT
+template <int N, typename TAB> inline void fill_even_odd(TAB &tab, const double *S, const double *SD) {
+  fill_even_odd(tab.eS, [&](int i, int q) { return S[i * N + q]; });
+  fill_even_odd(tab.eSD, [&](int i, int q) { return SD[i * N + q]; });
+  fill_even_odd(tab.eST, [&](int r, int k) { return S[k * N + r]; });
+  fill_even_odd(tab.eSDT, [&](int r, int k) { return SD[k * N + r]; });
 }
 
 // out_q = sum_i M(i, q) in_i by the even/odd form; f(q, out_q) is called once for every q
@@ -126,6 +130,46 @@ template <int N> struct Layout {
   static constexpr int N3 = N * N * N;
 };
 
+// elements of a cell's geometry in the line layout, [N][ncomp][N^2], padded to 16 bytes (the
+// unit of the bulk prefetch)
+template <int N, typename T> __host__ __device__ constexpr int geo_cell_elems(int ncomp) {
+  return (ncomp * N * N * N * (int)sizeof(T) + 15) / 16 * 16 / (int)sizeof(T);
+}
+
+// whether a Laplace operator of geometry code GEOM (0 full, 1 axis-aligned, 2 with a coefficient,
+// 3 inverse Jacobian) is applied by the line kernels and keeps its cell data in the line layout:
+// degrees >= 3, axis-aligned cells at every degree, and degree 1 with a coefficient (64^3 cells,
+// FP64 / FP32: 18.8 / 12.5 us against 25.5 / 16.5 us with slabs; degree 2: 76 / 43 against 66 / 43)
+__host__ __device__ constexpr bool line_layout(int N, int geom) {
+  return N >= 4 || geom == 1 || (N == 2 && geom == 2);
+}
+// the same for mass matrices
+__host__ __device__ constexpr bool mass_line_layout(int N) { return N >= 4; }
+
+// Where an operator's cell data lie.  LINE: cell by cell, the index map lexicographic, a value per point as [x point][z point,
+// y point].  Otherwise by warp group: the index map as [group][k*N + i][e*N + j], a full geometry
+// as [group][x point][y point][component][e*N + z point], a value per point as
+// [group][y point, x point][e*N + z point].
+template <int N, bool LINE> struct CellData {
+  using Lo = Layout<N>;
+  static __device__ __forceinline__ int64_t idx(int64_t c, int i, int j, int k) {
+    if (LINE) return c * Lo::N3 + (k * N + j) * N + i;
+    const int64_t g = c / Lo::CPW;
+    return (g * Lo::N2 + k * N + i) * Lo::LANES + int(c - g * Lo::CPW) * N + j;
+  }
+  // value m of the `ncomp` values of point (p, q, r)
+  template <typename T> static __device__ __forceinline__ int64_t geo(int64_t c, int p, int q, int r, int m, int ncomp) {
+    if (LINE) return c * geo_cell_elems<N, T>(ncomp) + (p * ncomp + m) * Lo::N2 + r * N + q;
+    const int64_t g = c / Lo::CPW;
+    return ((g * Lo::N2 + p * N + q) * ncomp + m) * Lo::LANES + int(c - g * Lo::CPW) * N + r;
+  }
+  static __device__ __forceinline__ int64_t point(int64_t c, int p, int q, int r) {
+    if (LINE) return c * Lo::N3 + p * Lo::N2 + r * N + q;
+    const int64_t g = c / Lo::CPW;
+    return (g * Lo::N2 + q * N + p) * Lo::LANES + int(c - g * Lo::CPW) * N + r;
+  }
+};
+
 // L2 eviction policies: the geometry and index streams are read once and should not push
 // the reused src/dst lines out of L2; src gathers and dst atomics should stay.
 __device__ __forceinline__ uint64_t policy_evict_first() {
@@ -136,12 +180,6 @@ __device__ __forceinline__ uint64_t policy_evict_first() {
 __device__ __forceinline__ uint64_t policy_evict_last() {
   uint64_t p;
   asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-
-__device__ __forceinline__ uint64_t policy_evict_normal() {
-  uint64_t p;
-  asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
 
@@ -167,13 +205,8 @@ __device__ __forceinline__ uint32_t ld_stream(const uint32_t *p, uint64_t pol) {
   asm("ld.global.nc.L1::no_allocate.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
   return v;
 }
-// the same loads as volatile asm: issued where they stand in the program, not sunk towards
-// their first use (the register pipeline of vmult_slab_kernel issues them a phase early)
-__device__ __forceinline__ uint32_t ld_stream_early(const uint32_t *p, uint64_t pol) {
-  uint32_t v;
-  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
-  return v;
-}
+// gathered or streamed loads as volatile asm: issued where they stand in the program, not sunk
+// towards their first use
 __device__ __forceinline__ double ld_keep_early(const double *p, uint64_t pol) {
   double v;
   asm volatile("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
@@ -183,6 +216,19 @@ __device__ __forceinline__ float ld_keep_early(const float *p, uint64_t pol) {
   float v;
   asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
   return v;
+}
+__device__ __forceinline__ uint32_t ld_keep_early(const uint32_t *p, uint64_t pol) {
+  uint32_t v;
+  asm volatile("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+  return v;
+}
+// W[s] for a runtime s without a divergent constant-bank access
+template <int N, typename T> __device__ __forceinline__ T line_weight(const T (&W)[N], int s) {
+  T w = W[0];
+#pragma unroll
+  for (int r = 1; r < N; ++r)
+    if (s == r) w = W[r];
+  return w;
 }
 // gathered loads that are reused by neighbouring cells
 __device__ __forceinline__ double ld_keep(const double *p, uint64_t pol) {
@@ -274,31 +320,6 @@ template <int PENDING> __device__ __forceinline__ void cp_async_wait() {
 //   phase 3 (Y-slab), per x node i:        out = Sz^T a + SDz^T c, scatter
 // Each lane overwrites only its own slab's region of the buffers between the two
 // exchanges, so only the two exchanges (and the end of a group) need a __syncwarp.
-// compile-time overrides of the tuned choices in vmult_slab_kernel (-1: the tuned default,
-// 0: off, 1: on): even/odd phase-2 contractions (EO2), rolled deferred passes and phase 3
-// (TUNR), phase 2 without accumulators (DEFER), paired-point x contractions (EO1X)
-#ifndef PMG_VMULT_EO_PHASE2
-#define PMG_VMULT_EO_PHASE2 -1
-#endif
-#ifndef PMG_VMULT_ROLL_TAIL
-#define PMG_VMULT_ROLL_TAIL -1
-#endif
-#ifndef PMG_VMULT_DEFER
-#define PMG_VMULT_DEFER -1
-#endif
-#ifndef PMG_VMULT_EO_PHASE1X
-#define PMG_VMULT_EO_PHASE1X -1
-#endif
-// L2 prefetch of the next group's geometry (full and inverse-Jacobian layouts): -1 the tuned
-// default, 1 evict-first, 0 none, 2 evict-normal.  The default prefetches (evict-first) for the
-// direct-load variants only: the ring variant streams each column through its TMA ring
-// already, and the extra prefetch only added L2 traffic (deformed cube on B200, FP64 128^3:
-// Q4 3914-3968 -> 3721-3737 us, Q5 at 64^3 1188 -> 1157 us, Q3 unchanged without it; FP32
-// ring variants Q3 972 -> 914 us, Q2 398 -> 381 us; FP32 Q4 with direct loads 2156 ->
-// 2430-2497 us without it)
-#ifndef PMG_VMULT_PREFETCH
-#define PMG_VMULT_PREFETCH -1
-#endif
 template <int N> struct Stride {
   // per-cell stride of the exchange buffers, padded where that lowers bank conflicts of
   // the two exchange patterns (offsets N*s and N*N*s within a cell)
@@ -324,76 +345,30 @@ __device__ __forceinline__ void invjac_flux(const T *__restrict__ geo, int64_t g
   for (int d = 0; d < 3; ++d) f[d] = iv[3 * d] * gx[0] + iv[3 * d + 1] * gx[1] + iv[3 * d + 2] * gx[2];
 }
 
-template <int N, typename T, int GEOM, bool SMEM_G>
-__device__ __forceinline__ void load_g6(const T *__restrict__ geo, const T *gs,
-                                        const T *__restrict__ coef, const Tab<N, T> &tab,
-                                        int64_t g, int lane, int e, int q, int p, T wr,
-                                        uint64_t pol, T (&c)[6]) {
-  using Lo = Layout<N>;
-  constexpr int LANES = Lo::LANES, N2 = Lo::N2, CPW = Lo::CPW;
-  if (GEOM == 0 && SMEM_G) {
-    const T *gp = gs + q * 6 * LANES + lane; // the staged x column p
+// the six components of the tensor at point (p, q, r) of cell c
+template <int N, typename T, int GEOM>
+__device__ __forceinline__ void load_g6(const T *__restrict__ geo, const T *__restrict__ coef, const Tab<N, T> &tab,
+                                        int64_t cell, int r, int q, int p, T wr, T (&c)[6]) {
+  using CD = CellData<N, line_layout(N, GEOM)>;
+  if (GEOM == 0) {
 #pragma unroll
-    for (int m = 0; m < 6; ++m) c[m] = gp[m * LANES];
-  } else if (GEOM == 0) {
-    const T *gp = geo + g * (N2 * 6 * LANES) + (p * N + q) * 6 * LANES + lane;
-#pragma unroll
-    for (int m = 0; m < 6; ++m) c[m] = ld_stream(gp + m * LANES, pol);
+    for (int m = 0; m < 6; ++m) c[m] = __ldg(geo + CD::template geo<T>(cell, p, q, r, m, 6));
   } else {
-    const T *cg = geo + (g * CPW + e) * 8;
     T w = wr * tab.W[q] * tab.W[p];
-    if (GEOM == 2) w *= ld_stream(coef + g * (N2 * LANES) + (q * N + p) * LANES + lane, pol);
+    if (GEOM == 2) w *= __ldg(coef + CD::point(cell, p, q, r));
 #pragma unroll
-    for (int m = 0; m < 6; ++m) c[m] = w * __ldg(cg + m);
+    for (int m = 0; m < 6; ++m) c[m] = w * __ldg(geo + cell * 8 + m);
   }
 }
 
-// resident blocks of 128 threads per SM the register allocation is sized for; matches the
-// shared-memory footprint (3 exchange buffers per warp) of each degree and type
-// FP64 affine kernels at 3 <= N <= 5: 0 plain runtime loops, 1 with even/odd z contractions,
-// 2 (default) unrolled with every even/odd form at up to 255 registers, which measured fastest
-// on B200 despite some spills (64^3 / 48^3 with kappa: Q4 217 -> 174 us, Q3 205 -> 200 us,
-// Q2 74 -> 67 us; mode 1: 210, 199, 72 us)
-// (at N = 6 and 7 the unrolled FP64 form spills 0.5-1.4 KB and measured 1.6-2.1x slower)
-#ifndef PMG_VMULT_F64_AFFINE_NMAX
-#define PMG_VMULT_F64_AFFINE_NMAX 5
-#endif
-#ifndef PMG_VMULT_F64_AFFINE_MODE
-#define PMG_VMULT_F64_AFFINE_MODE 2
-#endif
-template <int N, typename T, int GEOM> constexpr int f64_affine_mode_v =
-    (sizeof(T) == 8 && N <= PMG_VMULT_F64_AFFINE_NMAX && N >= 3 && (GEOM == 1 || GEOM == 2)) ? PMG_VMULT_F64_AFFINE_MODE : 0;
-template <int N, typename T, int GEOM = 1> struct MinBlocks {
-  static constexpr int value =
-      f64_affine_mode_v<N, T, GEOM> == 2
-          ? 2
-          : (sizeof(T) == 8 ? (N >= 6 ? 2 : 3) : ((N == 7 && (GEOM == 0 || GEOM == 3)) ? 3 : 2));
-};
-// outer streaming loops: runtime loops for FP64 (bounded live registers), unrolled for FP32
-// (registers are cheap at 4 bytes and unrolling keeps the tables as immediate operands),
-// except FP32 Q6 with full geometry, where runtime loops at 170 registers (12 warps/SM)
-// measured 1.4x faster on B200 than the unrolled form at 255
-// (FP32 Q6 affine in runtime loops at 142 registers, 12 warps/SM, measured no faster than the
-// unrolled form at 8 warps/SM)
-template <int N, typename T, int GEOM = 1> struct Unroll {
-  static constexpr int value = f64_affine_mode_v<N, T, GEOM> == 2
-                                   ? N
-                                   : ((sizeof(T) == 8 || (N == 7 && (GEOM == 0 || GEOM == 3))) ? 1 : N);
-};
-
 // Shared memory per warp of vmult_slab_kernel: 3 exchange buffers, plus (SMEM_G) the
-// geometry column ring and its two mbarriers, plus the gather pipeline (PIPE): 1 = one
-// group's index block, 2 = one group's gathered src values and two index blocks, 3 (the
-// register pipeline) nothing.
+// geometry column ring and its two mbarriers, plus (PIPE) one group's index block.
 template <int N, typename T, bool SMEM_G, int PIPE = 0> struct SlabSmem {
   static constexpr size_t XCHG = size_t(3) * Layout<N>::CPW * Stride<N>::CELL * sizeof(T);
   static constexpr size_t CHUNK = size_t(N) * 6 * Layout<N>::LANES * sizeof(T); // one x column
   static constexpr size_t GEO = SMEM_G ? 2 * CHUNK : 0;                         // two-slot ring
-  static constexpr size_t IDXB = size_t(Layout<N>::N2) * Layout<N>::LANES * 4;   // one index block
-  static constexpr size_t SRC = PIPE == 2 ? size_t(Layout<N>::N2) * Layout<N>::LANES * sizeof(T) : 0;
-  static constexpr size_t IDX = (PIPE == 0 || PIPE == 3) ? 0 : (PIPE == 1 ? 1 : 2) * IDXB;
-  static constexpr size_t OFF_SRC = ((GEO + XCHG + 15) / 16) * 16;
-  static constexpr size_t OFF_IDX = OFF_SRC + ((SRC + 15) / 16) * 16;
+  static constexpr size_t IDX = PIPE ? size_t(Layout<N>::N2) * Layout<N>::LANES * 4 : 0; // one index block
+  static constexpr size_t OFF_IDX = ((GEO + XCHG + 15) / 16) * 16;
   static constexpr size_t PER_WARP = OFF_IDX + ((IDX + 15) / 16) * 16 + (SMEM_G ? 16 : 0);
 };
 
@@ -401,58 +376,25 @@ template <int N, typename T, bool SMEM_G, int PIPE = 0> struct SlabSmem {
 // two-slot shared-memory ring; the copy of the next column (or of the next group's first
 // column) is issued when a column starts, so it overlaps with that column's work.
 // Warps share nothing (each has its own ring, barriers and buffers): any warps per block.
-// PIPE: the dependent index -> src gather is taken off the critical path by per-thread
-// cp.async copies one group ahead (each lane copies exactly the entries it later reads, so
-// cp.async.wait_group alone orders them):
-//   1: the next group's index block is copied once the current gather has read its own;
-//   2: the next group's src values are copied (zero-filled at Dirichlet entries) right after
-//      the current group's first phase, from an index block copied a group earlier still;
-//      the scatter reads its indices from shared memory as well;
-//   3: a register pipeline without shared memory: the next group's index block is loaded
-//      into registers when phase 2 starts (it lands during phase 2) and its src values when
-//      phase 3 starts (they land during the scatter); phase 1 then starts with the gathered
-//      values in registers.  It costs N^2 index registers through phase 2 and N^2 values
-//      through phase 3, which the shared-memory-bound ring variant has to spare.
+// PIPE 1: the next group's index block is copied into shared memory one group ahead by
+// per-thread cp.async copies (each lane copies exactly the entries it later reads, so
+// cp.async.wait_group alone orders them).
 template <int N, typename T, int GEOM, bool SMEM_G, int PIPE = 0>
-__global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N, T, GEOM>::value))
+__global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : (sizeof(T) == 8 && !(GEOM == 2 && N == 3) ? 3 : 2)))
     vmult_slab_kernel(const __grid_constant__ Tab<N, T> tab, const T *__restrict__ src, T *__restrict__ dst,
                       const uint32_t *__restrict__ idx, const T *__restrict__ geo,
                       const T *__restrict__ coef, int64_t n_groups, unsigned int *err) {
+  static_assert(N == 2 || N == 3, "degrees 1 and 2; line_kernels.cuh has the others");
+  static_assert(GEOM == 0 || GEOM == 2 || GEOM == 3, "axis-aligned cells without a coefficient: vmult_box_kernel");
   using Lo = Layout<N>;
   constexpr int CPW = Lo::CPW, LANES = Lo::LANES, N2 = Lo::N2;
   constexpr int CS = Stride<N>::CELL;
   constexpr unsigned MASK = Lo::MASK;
-  constexpr int UNR = SMEM_G ? N : Unroll<N, T, GEOM>::value;
-  // even/odd contractions where they measured faster on B200 (the FP64 runtime-loop
-  // variants spill with the extra live values; N = 2 gains nothing):
-  //  EO   z contractions of phases 1 and 3: the ring variants, the FP32 direct variants
-  //       other than N = 6 and N = 7 full geometry, and the FP64 affine kernels at N <= 5
-  //  EO2  phase 2 (the y contractions of the columns, the x contraction of fz): the ring
-  //       variants, FP32 N <= 5, every N = 7 variant and the unrolled FP64 affine kernels
-  //  EO1X x contractions of phase 1 by mirrored pairs of points (the point loop unrolled):
-  //       with EO except at N = 6
-  //  DEFER (below) phase 2 without register accumulators, at N = 7
-  constexpr bool EO =
-      N >= 3 && (SMEM_G || (sizeof(T) == 4 && N != 6 && !(N == 7 && (GEOM == 0 || GEOM == 3))) ||
-                 f64_affine_mode_v<N, T, GEOM> >= 1);
-  constexpr bool EO2 =
-      PMG_VMULT_EO_PHASE2 >= 0
-          ? (PMG_VMULT_EO_PHASE2 == 1 && N >= 3)
-          : N >= 3 && (SMEM_G || (sizeof(T) == 4 && N <= 5) || N == 7 || f64_affine_mode_v<N, T, GEOM> == 2);
-  // DEFER: phase 2 keeps no accumulators; y1, y2 and x3 are parked in the lane's own plane and
-  // contracted along x (and y) afterwards in even/odd form (N = 7: 8-35 % faster on B200,
-  // the runtime-loop FP64 variants lose their spills; slower at N <= 6)
-  constexpr bool DEFER = EO2 && (PMG_VMULT_DEFER >= 0 ? PMG_VMULT_DEFER == 1 : N == 7);
-  // the deferred passes and phase 3 index the tables by their inner loops only, so their
-  // outer loops can stay rolled (smaller code) at no table-load cost: FP32 Q4 affine falls
-  // from ~205 to 128 registers and runs 21 % faster on B200; every other variant measured
-  // 1-15 % slower rolled
-  constexpr int TUNR = PMG_VMULT_ROLL_TAIL >= 0 ? (PMG_VMULT_ROLL_TAIL == 1 ? 1 : UNR)
-                                                : ((sizeof(T) == 4 && N == 5 && (GEOM == 1 || GEOM == 2)) ? 1 : UNR);
-  constexpr bool EO1X = PMG_VMULT_EO_PHASE1X >= 0 ? (PMG_VMULT_EO_PHASE1X == 1 && EO && UNR == N)
-                                                  : (EO && UNR == N && N != 6);
+  // even/odd contractions where they measured faster on B200 (N = 2 gains nothing, the FP64
+  // runtime-loop variants spill); outer streaming loops in runtime form for FP64 direct loads
+  constexpr bool EO = N == 3 && (SMEM_G || sizeof(T) == 4 || GEOM == 2);
+  constexpr int UNR = (SMEM_G || sizeof(T) == 4 || EO) ? N : 1;
   using SM = SlabSmem<N, T, SMEM_G, PIPE>;
-  static_assert(!(SMEM_G && PIPE == 2), "src staging is not combined with the geometry ring");
   constexpr int NCOMP = GEOM == 3 ? 10 : 6; // geometry values per quadrature point
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
@@ -465,8 +407,7 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
   T *bufZ = bufW + CPW * CS;
   T *bufX = bufZ + CPW * CS;
   uint64_t *bars = reinterpret_cast<uint64_t *>(wsm + SM::PER_WARP - 16);
-  T *sbuf = reinterpret_cast<T *>(wsm + SM::OFF_SRC) + lane;               // [N2][LANES] (PIPE 2)
-  uint32_t *ibuf = reinterpret_cast<uint32_t *>(wsm + SM::OFF_IDX) + lane; // [slot][N2][LANES]
+  uint32_t *ibuf = reinterpret_cast<uint32_t *>(wsm + SM::OFF_IDX) + lane; // [N2][LANES]
   constexpr int CHUNK_ELEMS = N * 6 * LANES;
   uint32_t chunk = 0; // columns consumed so far; slot = chunk & 1, parity = (chunk >> 1) & 1
   const int64_t warp0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -481,108 +422,38 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
     }
     __syncwarp(MASK);
   }
-  T wr = tab.W[0]; // Gauss weight of this lane's z point (affine geometry)
-#pragma unroll
-  for (int r = 1; r < N; ++r)
-    if (s == r) wr = tab.W[r];
+  const T wr = line_weight<N, T>(tab.W, s); // Gauss weight of this lane's z point (coefficient geometry)
 
-  // gather pipeline: copy the index block of group gg into slot `slot` / the src values
-  // named by slot `slot` into sbuf; every call commits exactly one cp.async group
-  auto issue_idx = [&](int64_t gg, int slot) {
+  // copy the index block of group gg; every call commits exactly one cp.async group
+  auto issue_idx = [&](int64_t gg) {
     if (gg < n_groups) {
       const uint32_t *ip = idx + gg * (N2 * LANES) + lane;
 #pragma unroll
-      for (int a = 0; a < N2; ++a) cp_async(ibuf + (slot * N2 + a) * LANES, ip + a * LANES, 4, 4, pol_first);
+      for (int a = 0; a < N2; ++a) cp_async(ibuf + a * LANES, ip + a * LANES, 4, 4, pol_first);
     }
     cp_async_commit();
   };
-  auto issue_src = [&](bool valid, int slot) {
-    if (valid) {
-#pragma unroll
-      for (int a = 0; a < N2; ++a) {
-        const uint32_t id = ibuf[(slot * N2 + a) * LANES];
-        const bool ok = id != kInvalidIdx;
-        cp_async(sbuf + a * LANES, ok ? src + id : src, (int)sizeof(T), ok ? (int)sizeof(T) : 0, pol_last);
-      }
-    }
-    cp_async_commit();
-  };
-  int it = 0; // groups done by this warp (PIPE 2: index slot of group g = it & 1)
-  // PIPE 3: the next group's index block and gathered src values, carried in registers
-  constexpr int RP = PIPE == 3 ? N : 1;
-  uint32_t nidx[RP][RP];
-  T nsrc[RP][RP];
-  auto load_next_idx = [&](int64_t gg) {
-    if (PIPE == 3 && gg < n_groups) {
-      const uint32_t *ip = idx + gg * (N2 * LANES) + lane;
-#pragma unroll
-      for (int k = 0; k < RP; ++k)
-#pragma unroll
-        for (int i = 0; i < RP; ++i) nidx[k][i] = ld_stream_early(ip + (k * N + i) * LANES, pol_first);
-    }
-  };
-  auto load_next_src = [&](int64_t gg) {
-    if (PIPE == 3 && gg < n_groups) {
-#pragma unroll
-      for (int k = 0; k < RP; ++k)
-#pragma unroll
-        for (int i = 0; i < RP; ++i)
-          nsrc[k][i] = nidx[k][i] != kInvalidIdx ? ld_keep_early(src + nidx[k][i], pol_last) : T(0);
-    }
-  };
-  if (PIPE == 3) {
-    load_next_idx(warp0);
-    load_next_src(warp0);
-  }
-  if (PIPE == 1) issue_idx(warp0, 0);
-  if (PIPE == 2) {
-    issue_idx(warp0, 0);
-    cp_async_wait<0>();
-    issue_src(warp0 < n_groups, 0);
-    issue_idx(warp0 + nwarps, 1);
-  }
+  if (PIPE == 1) issue_idx(warp0);
 
-  for (int64_t g = warp0; g < n_groups; g += nwarps, ++it) {
-    constexpr bool PREFETCH = PMG_VMULT_PREFETCH == -1 ? !SMEM_G : PMG_VMULT_PREFETCH != 0;
-    if ((GEOM == 0 || GEOM == 3) && PREFETCH && lane == 0 && g + nwarps < n_groups)
-      prefetch_l2(geo + (g + nwarps) * (N2 * NCOMP * LANES), N2 * NCOMP * LANES * sizeof(T),
-                  PMG_VMULT_PREFETCH == 2 ? policy_evict_normal() : pol_first);
+  for (int64_t g = warp0; g < n_groups; g += nwarps) {
+    // the ring streams each column ahead already: an L2 prefetch as well only added traffic
+    // (FP32 Q2 at 128^3 398 against 381 us)
+    if ((GEOM == 0 || GEOM == 3) && !SMEM_G && lane == 0 && g + nwarps < n_groups)
+      prefetch_l2(geo + (g + nwarps) * (N2 * NCOMP * LANES), N2 * NCOMP * LANES * sizeof(T), pol_first);
     const uint32_t *ig = idx + g * (N2 * LANES) + lane;
-    const int slot = it & 1;
 
     // ---- phase 1: gather the Y-slab y = s, u[k][i] = src at node (i, s, k) ----
     {
       T u[N][N];
-      if (PIPE == 3) {
+      if (PIPE == 1) cp_async_wait<0>(); // this group's index block
 #pragma unroll
-        for (int k = 0; k < N; ++k)
+      for (int k = 0; k < N; ++k)
 #pragma unroll
-          for (int i = 0; i < N; ++i) u[k][i] = nsrc[k < RP ? k : 0][i < RP ? i : 0];
-      } else if (PIPE == 2) {
-        cp_async_wait<1>(); // this group's src values (the next index block may be in flight)
-#pragma unroll
-        for (int k = 0; k < N; ++k)
-#pragma unroll
-          for (int i = 0; i < N; ++i) u[k][i] = sbuf[(k * N + i) * LANES];
-      } else if (PIPE == 1) {
-        cp_async_wait<0>(); // this group's index block
-#pragma unroll
-        for (int k = 0; k < N; ++k)
-#pragma unroll
-          for (int i = 0; i < N; ++i) {
-            const uint32_t id = ibuf[(k * N + i) * LANES];
-            u[k][i] = (id != kInvalidIdx) ? ld_keep(src + id, pol_last) : T(0);
-          }
-      } else {
-#pragma unroll
-        for (int k = 0; k < N; ++k)
-#pragma unroll
-          for (int i = 0; i < N; ++i) {
-            const uint32_t id = ld_stream(ig + (k * N + i) * LANES, pol_first);
-            u[k][i] = (id != kInvalidIdx) ? ld_keep(src + id, pol_last) : T(0);
-          }
-      }
-      if constexpr (EO1X) {
+        for (int i = 0; i < N; ++i) {
+          const uint32_t id = PIPE == 1 ? ibuf[(k * N + i) * LANES] : ld_stream(ig + (k * N + i) * LANES, pol_first);
+          u[k][i] = (id != kInvalidIdx) ? ld_keep(src + id, pol_last) : T(0);
+        }
+      if constexpr (EO) {
         // x contractions t = Sx u, tx = SDx u by mirrored pairs of points (p, N-1-p): the
         // sums and differences of mirrored nodes replace u in place (u[k][i] = e_i and
         // u[k][N-1-i] = o_i for i < H)
@@ -654,11 +525,6 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
             tx[k] = b;
           }
           // z contraction: w = Sz t, wz = SDz t, wx = Sz tx at (z = r, y = s, x = p)
-          if constexpr (EO) {
-            eo_apply<N, T, 1>(tab.eS, t, [&](int r, T v) { bufW[(r * N + s) * N + p] = v; });
-            eo_apply<N, T, -1>(tab.eSD, t, [&](int r, T v) { bufZ[(r * N + s) * N + p] = v; });
-            eo_apply<N, T, 1>(tab.eS, tx, [&](int r, T v) { bufX[(r * N + s) * N + p] = v; });
-          } else {
 #pragma unroll
             for (int r = 0; r < N; ++r) {
               T w = T(0), wz = T(0), wx = T(0);
@@ -673,22 +539,15 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
               bufZ[o] = wz;
               bufX[o] = wx;
             }
-          }
         }
       }
     }
-    // the gather's shared-memory entries are consumed: refill them for the next group
-    if (PIPE == 1) issue_idx(g + nwarps, 0);
-    if (PIPE == 3) load_next_idx(g + nwarps); // lands during phase 2
-    if (PIPE == 2) {
-      cp_async_wait<0>(); // the next group's index block
-      issue_src(g + nwarps < n_groups, slot ^ 1);
-    }
+    if (PIPE == 1) issue_idx(g + nwarps); // the index block is consumed: refill it for the next group
     __syncwarp(MASK);
 
     // ---- phase 2: Z-slab z = s, streamed over the x point p ----
     T cd0 = T(0), cd3 = T(0), cd5 = T(0); // diagonal of the affine cell tensor
-    if (GEOM == 1 || GEOM == 2) {
+    if (GEOM == 2) {
       const T *cg = geo + (g * CPW + e) * 8;
       cd0 = __ldg(cg);
       cd3 = __ldg(cg + 3);
@@ -716,7 +575,7 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
           }
           if (!mbar_wait_bounded(&bars[chunk & 1], (chunk >> 1) & 1, err, 1u << 24)) {
             if (lane == 0) mbar_wait_bounded(&bars[(chunk + 1) & 1], ((chunk + 1) >> 1) & 1, err, 1u << 24);
-            if (PIPE == 1 || PIPE == 2) cp_async_wait<0>();
+            if (PIPE == 1) cp_async_wait<0>();
             return; // the error flag is set; let copies in flight land before leaving
           }
           gcol = ring + (chunk & 1) * CHUNK_ELEMS;
@@ -730,12 +589,15 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
           Xc[j] = bufX[o];
         }
         T fx[N], fy[N];
-        if constexpr (EO2) {
+        if constexpr (EO) {
           // f = G grad u at the point (p, q) of this slab: fx, fy kept, fz -> own bufX region
           auto point = [&](int q, T dx, T dy, T dz) {
             if (GEOM == 0) {
               T gc[6];
-              load_g6<N, T, GEOM, SMEM_G>(geo, gcol, coef, tab, g, lane, e, q, p, wr, pol_first, gc);
+              const T *gp = SMEM_G ? gcol + q * 6 * LANES + lane // the staged x column p
+                                   : geo + g * (N2 * 6 * LANES) + (p * N + q) * 6 * LANES + lane;
+#pragma unroll
+              for (int m = 0; m < 6; ++m) gc[m] = SMEM_G ? gp[m * LANES] : ld_stream(gp + m * LANES, pol_first);
               fx[q] = gc[0] * dx + gc[1] * dy + gc[2] * dz;
               fy[q] = gc[1] * dx + gc[3] * dy + gc[4] * dz;
               bufX[(s * N + q) * N + p] = gc[2] * dx + gc[4] * dy + gc[5] * dz; // fz
@@ -748,7 +610,7 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
             } else {
               // affine cells are axis-aligned boxes: the cell tensor is diagonal (rr, ss, tt)
               T w = wr * tab.W[q] * tab.W[p];
-              if (GEOM == 2) w *= ld_stream(coef + g * (N2 * LANES) + (q * N + p) * LANES + lane, pol_first);
+              w *= ld_stream(coef + g * (N2 * LANES) + (q * N + p) * LANES + lane, pol_first);
               fx[q] = (w * cd0) * dx;
               fy[q] = (w * cd3) * dy;
               bufX[(s * N + q) * N + p] = (w * cd5) * dz; // fz
@@ -763,22 +625,13 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
           for (int q = 0; q < N; ++q) point(q, dxv[q], dyv[q], dzv[q]);
           eo_apply<N, T, 1>(tab.eST, fx, [&](int j, T v) { y1v[j] = v; });
           eo_apply<N, T, -1>(tab.eSDT, fy, [&](int j, T v) { y2v[j] = v; });
-          if constexpr (DEFER) {
-            // park y1, y2 over the consumed column p of this lane's plane (bufW, bufZ)
 #pragma unroll
-            for (int j = 0; j < N; ++j) {
-              bufW[(s * N + j) * N + p] = y1v[j];
-              bufZ[(s * N + j) * N + p] = y2v[j];
+          for (int j = 0; j < N; ++j)
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+              a[j][i] = fma(tab.SD[i * N + p], y1v[j], a[j][i]);
+              a[j][i] = fma(tab.S[i * N + p], y2v[j], a[j][i]);
             }
-          } else {
-#pragma unroll
-            for (int j = 0; j < N; ++j)
-#pragma unroll
-              for (int i = 0; i < N; ++i) {
-                a[j][i] = fma(tab.SD[i * N + p], y1v[j], a[j][i]);
-                a[j][i] = fma(tab.S[i * N + p], y2v[j], a[j][i]);
-              }
-          }
         } else {
 #pragma unroll
           for (int q = 0; q < N; ++q) {
@@ -792,7 +645,10 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
             // f = G grad u at the point (p, q) of this slab: fx, fy kept, fz -> own bufX region
             if (GEOM == 0) {
               T gc[6];
-              load_g6<N, T, GEOM, SMEM_G>(geo, gcol, coef, tab, g, lane, e, q, p, wr, pol_first, gc);
+              const T *gp = SMEM_G ? gcol + q * 6 * LANES + lane // the staged x column p
+                                   : geo + g * (N2 * 6 * LANES) + (p * N + q) * 6 * LANES + lane;
+#pragma unroll
+              for (int m = 0; m < 6; ++m) gc[m] = SMEM_G ? gp[m * LANES] : ld_stream(gp + m * LANES, pol_first);
               fx[q] = gc[0] * dx + gc[1] * dy + gc[2] * dz;
               fy[q] = gc[1] * dx + gc[3] * dy + gc[4] * dz;
               bufX[(s * N + q) * N + p] = gc[2] * dx + gc[4] * dy + gc[5] * dz; // fz
@@ -804,7 +660,7 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
               bufX[(s * N + q) * N + p] = f3[2]; // fz
             } else {
               T w = wr * tab.W[q] * tab.W[p];
-              if (GEOM == 2) w *= ld_stream(coef + g * (N2 * LANES) + (q * N + p) * LANES + lane, pol_first);
+              w *= ld_stream(coef + g * (N2 * LANES) + (q * N + p) * LANES + lane, pol_first);
               fx[q] = (w * cd0) * dx;
               fy[q] = (w * cd3) * dy;
               bufX[(s * N + q) * N + p] = (w * cd5) * dz; // fz
@@ -830,47 +686,13 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
           ++chunk;
         }
       }
-      if constexpr (DEFER) {
-        // a(j, .) = SDx^T y1(j, .) + Sx^T y2(j, .), row by row in place over y1 (bufW)
-#pragma unroll TUNR
-        for (int j = 0; j < N; ++j) {
-          T y1[N], y2[N], v[N];
+      // a -> own slab region of bufW (all of this lane's reads of it are done)
 #pragma unroll
-          for (int p = 0; p < N; ++p) {
-            y1[p] = bufW[(s * N + j) * N + p];
-            y2[p] = bufZ[(s * N + j) * N + p];
-          }
-          eo_apply<N, T, -1>(tab.eSDT, y1, [&](int i, T x) { v[i] = x; });
-          eo_apply<N, T, 1>(tab.eST, y2, [&](int i, T x) { v[i] += x; });
+      for (int j = 0; j < N; ++j)
 #pragma unroll
-          for (int i = 0; i < N; ++i) bufW[(s * N + j) * N + i] = v[i];
-        }
-      } else {
-        // a -> own slab region of bufW (all of this lane's reads of it are done)
-#pragma unroll
-        for (int j = 0; j < N; ++j)
-#pragma unroll
-          for (int i = 0; i < N; ++i) bufW[(s * N + j) * N + i] = a[j][i];
-      }
+        for (int i = 0; i < N; ++i) bufW[(s * N + j) * N + i] = a[j][i];
     }
-    if constexpr (DEFER) {
-      // c = Sy^T Sx^T fz: x3 = Sx^T fz row by row in place (bufX), then Sy^T by columns into
-      // this lane's region of bufZ (whose y2 values the pass above consumed)
-#pragma unroll TUNR
-      for (int q = 0; q < N; ++q) {
-        T fz[N];
-#pragma unroll
-        for (int p = 0; p < N; ++p) fz[p] = bufX[(s * N + q) * N + p];
-        eo_apply<N, T, 1>(tab.eST, fz, [&](int i, T x) { bufX[(s * N + q) * N + i] = x; });
-      }
-#pragma unroll TUNR
-      for (int i = 0; i < N; ++i) {
-        T x3[N];
-#pragma unroll
-        for (int q = 0; q < N; ++q) x3[q] = bufX[(s * N + q) * N + i];
-        eo_apply<N, T, 1>(tab.eST, x3, [&](int j, T x) { bufZ[(s * N + j) * N + i] = x; });
-      }
-    } else {
+    {
       // c = Sy^T Sx^T fz from this lane's fz region, into its own region of bufZ
       T c[N][N];
 #pragma unroll
@@ -882,7 +704,7 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
         T fz[N];
 #pragma unroll
         for (int p = 0; p < N; ++p) fz[p] = bufX[(s * N + q) * N + p];
-        if constexpr (EO2) {
+        if constexpr (EO) {
           T x3v[N]; // x3 = Sx^T fz along this row
           eo_apply<N, T, 1>(tab.eST, fz, [&](int i, T v) { x3v[i] = v; });
 #pragma unroll
@@ -907,10 +729,8 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
     }
     __syncwarp(MASK);
 
-    if (PIPE == 3) load_next_src(g + nwarps); // lands during the scatter
-
     // ---- phase 3: Y-slab y = s, out = Sz^T a + SDz^T c, scatter ----
-#pragma unroll TUNR
+#pragma unroll UNR
     for (int i = 0; i < N; ++i) {
       T A[N], Cc[N];
 #pragma unroll
@@ -936,15 +756,13 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : MinBlocks<N,
       }
 #pragma unroll
       for (int k = 0; k < N; ++k) {
-        const uint32_t id = PIPE == 2 ? ibuf[(slot * N2 + k * N + i) * LANES]
-                                      : ld_stream(ig + (k * N + i) * LANES, pol_first);
+        const uint32_t id = ld_stream(ig + (k * N + i) * LANES, pol_first);
         if (id != kInvalidIdx) red_keep(dst + id, v[k], pol_last);
       }
     }
-    if (PIPE == 2) issue_idx(g + 2 * nwarps, slot); // this group's index slot is free
     __syncwarp(MASK); // buffers are rewritten by the next group
   }
-  if (PIPE == 1 || PIPE == 2) cp_async_wait<0>(); // no copy may land after the warp has left
+  if (PIPE == 1) cp_async_wait<0>(); // no copy may land after the warp has left
 }
 
 // Diagonal of the cell operator summed into diag (atomic), same layout and slab scheme:
@@ -958,7 +776,8 @@ __global__ void __launch_bounds__(128) diag_slab_kernel(const Tab2<N, T> tab,
                                                         const T *__restrict__ coef,
                                                         int64_t n_groups) {
   using Lo = Layout<N>;
-  constexpr int CPW = Lo::CPW, LANES = Lo::LANES, N2 = Lo::N2, N3 = Lo::N3;
+  using CD = CellData<N, line_layout(N, GEOM)>;
+  constexpr int CPW = Lo::CPW, LANES = Lo::LANES, N3 = Lo::N3;
   constexpr unsigned MASK = Lo::MASK;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
@@ -984,16 +803,14 @@ __global__ void __launch_bounds__(128) diag_slab_kernel(const Tab2<N, T> tab,
       for (int p = 0; p < N; ++p) {
         T c[6];
         if (GEOM == 0) {
-          const T *gp = geo + g * (N2 * 6 * LANES) + (p * N + q) * 6 * LANES + lane;
 #pragma unroll
-          for (int m = 0; m < 6; ++m) c[m] = __ldg(gp + m * LANES);
+          for (int m = 0; m < 6; ++m) c[m] = __ldg(geo + CD::template geo<T>(g * CPW + e, p, q, s, m, 6));
         } else if (GEOM == 3) {
           // G = JxW J^{-1} J^{-T} from the inverse-Jacobian layout, in the order of G
-          const T *gp = geo + g * (N2 * 10 * LANES) + (p * N + q) * 10 * LANES + lane;
           T iv[9];
 #pragma unroll
-          for (int m = 0; m < 9; ++m) iv[m] = __ldg(gp + m * LANES);
-          const T jw = __ldg(gp + 9 * LANES);
+          for (int m = 0; m < 9; ++m) iv[m] = __ldg(geo + CD::template geo<T>(g * CPW + e, p, q, s, m, 10));
+          const T jw = __ldg(geo + CD::template geo<T>(g * CPW + e, p, q, s, 9, 10));
           int m = 0;
 #pragma unroll
           for (int d1 = 0; d1 < 3; ++d1)
@@ -1003,7 +820,7 @@ __global__ void __launch_bounds__(128) diag_slab_kernel(const Tab2<N, T> tab,
         } else {
           const T *cg = geo + (g * CPW + e) * 8;
           T w = wr * tab.W[q] * tab.W[p];
-          if (GEOM == 2) w *= __ldg(coef + g * (N2 * LANES) + (q * N + p) * LANES + lane);
+          if (GEOM == 2) w *= __ldg(coef + CD::point(g * CPW + e, p, q, s));
 #pragma unroll
           for (int m = 0; m < 6; ++m) c[m] = w * __ldg(cg + m);
         }
@@ -1051,7 +868,6 @@ __global__ void __launch_bounds__(128) diag_slab_kernel(const Tab2<N, T> tab,
     }
     __syncwarp(MASK);
     // Y-slab (y = s): z contraction and scatter
-    const uint32_t *ig = idx + g * (N2 * LANES) + lane;
 #pragma unroll
     for (int k = 0; k < N; ++k)
 #pragma unroll
@@ -1063,7 +879,7 @@ __global__ void __launch_bounds__(128) diag_slab_kernel(const Tab2<N, T> tab,
           v = fma(SS[k * N + r], b1[(r * N + s) * N + i], v);
           v = fma(D2[k * N + r], b2[(r * N + s) * N + i], v);
         }
-        const uint32_t id = __ldg(ig + (k * N + i) * LANES);
+        const uint32_t id = __ldg(idx + CD::idx(g * CPW + e, i, s, k));
         if (id != kInvalidIdx) atomic_add(diag + id, v);
       }
     __syncwarp(MASK);
@@ -1079,15 +895,15 @@ struct SlabLaunch {
   const uint32_t *idx;
   const void *geo;
   const void *coef;
-  int64_t n_groups;
-  int geom; // 0 full, 1 affine, 2 affine + coefficient
+  int64_t n_groups, n_cells;
+  int geom; // 0 full, 1 affine, 2 affine + coefficient, 3 inverse Jacobian
+  double affine[3]; // diagonal of the affine cell tensor (geom 1 and 2)
   int dtype;
-  int64_t resident_warps;      // warps of the kernel resident on the whole device
-  int64_t resident_warps_ring; // the same for the geometry-ring variant of vmult
+  int64_t resident_warps; // warps of the diagonal kernel resident on the whole device
   unsigned int *err; // device flag set when a bounded wait gives up
   cudaStream_t stream;
   const double *S, *SD, *D, *W; // host tables (double), converted to the kernel type
-  int64_t *launched;            // if set: receives the number of warps the vmult launched
+  int64_t *units, *launched; // if set: receive the vmult's work units and the warps (blocks) sharing them
 };
 void launch_vmult_p1(const SlabLaunch &);
 void launch_vmult_p2(const SlabLaunch &);
@@ -1101,13 +917,7 @@ void launch_diag_p3(const SlabLaunch &);
 void launch_diag_p4(const SlabLaunch &);
 void launch_diag_p5(const SlabLaunch &);
 void launch_diag_p6(const SlabLaunch &);
-// resident warps per SM of the vmult / diagonal kernels
-int occupancy_vmult_p1(int dtype, int geom);
-int occupancy_vmult_p2(int dtype, int geom);
-int occupancy_vmult_p3(int dtype, int geom);
-int occupancy_vmult_p4(int dtype, int geom);
-int occupancy_vmult_p5(int dtype, int geom);
-int occupancy_vmult_p6(int dtype, int geom);
+// resident warps per SM of the diagonal kernels
 int occupancy_diag_p1(int dtype, int geom);
 int occupancy_diag_p2(int dtype, int geom);
 int occupancy_diag_p3(int dtype, int geom);

@@ -1,15 +1,17 @@
-// Launchers of the slab kernels for one polynomial degree.  Included by laplace_p<d>.cu
-// with PMG_DEGREE defined, so each degree compiles as its own translation unit.
+// Launchers of the vmult and diagonal kernels for one polynomial degree.  Included by
+// laplace_p<d>.cu with PMG_DEGREE defined, so each degree compiles as its own translation unit.
 #pragma once
 
 #include <algorithm>
-#include <cstdlib>
 #include <map>
 #include <mutex>
 #include <set>
 #include <utility>
 
+#include "fields.hpp"
 #include "laplace_kernels.cuh"
+#include "line_kernels.cuh"
+#include "line_tables.hpp"
 #include "pmg_internal.hpp"
 
 #ifndef PMG_DEGREE
@@ -33,7 +35,7 @@ template <typename T> kern::Tab<kN, T> make_tab(const SlabLaunch &L) {
     t.D[a] = (T)L.D[a];
   }
   for (int a = 0; a < kN; ++a) t.W[a] = (T)L.W[a];
-  kern::fill_even_odd(t, L.S, L.SD);
+  kern::fill_even_odd<kN>(t, L.S, L.SD);
   return t;
 }
 
@@ -48,15 +50,6 @@ template <typename T> kern::Tab2<kN, T> make_tab2(const SlabLaunch &L) {
   return t;
 }
 
-// warps per block of vmult_slab_kernel: one for the ring variant; for the direct variant four,
-// unless a warp needs more than 24 KB of shared memory (FP64 at N >= 6), where blocks of four
-// would leave most of an SM's shared memory unused (one 132-220 KB block per SM)
-template <typename T, bool SMEM_G, int PIPE> constexpr int vmult_wpb() {
-  return (SMEM_G || kern::SlabSmem<kN, T, SMEM_G, PIPE>::PER_WARP > 24 * 1024) ? 1 : kWarpsPerBlock;
-}
-template <typename T, bool SMEM_G, int PIPE> constexpr size_t vmult_smem() {
-  return size_t(vmult_wpb<T, SMEM_G, PIPE>()) * kern::SlabSmem<kN, T, SMEM_G, PIPE>::PER_WARP;
-}
 template <typename T> constexpr size_t diag_smem() {
   return size_t(kWarpsPerBlock) * 3 * kern::Layout<kN>::CPW * kern::Layout<kN>::N3 * sizeof(T);
 }
@@ -74,66 +67,86 @@ template <typename K> void allow_smem(K kernel, size_t bytes) {
   done.insert(key);
 }
 
-// Full geometry streams through the shared-memory column ring (TMA) where that measured faster
-// on B200 (deformed-cube sweeps at 64^3/128^3): FP64 degrees 1-5 and FP32 degrees 2, 3, 5, 6
-// (FP32 Q5 64^3 621 -> 563 us, Q6 1236 -> 1135 us once the ring no longer prefetched into L2);
-// FP32 degrees 1 and 4 (whose unrolled forms hide the latency at 8 warps/SM: Q4 128^3 2158
-// against 2427 us with the ring) and FP64 degree 6 (2372 against 2488 us) load it directly.
-// PMG_VMULT_STAGE=0 / 1 forces direct loads / the ring (a tuning switch; both are compiled).
-inline int stage_override() {
-  static const int v = [] {
-    const char *e = std::getenv("PMG_VMULT_STAGE");
-    return e ? std::atoi(e) : -1;
-  }();
-  return v;
-}
-template <typename T> bool use_ring() {
-  const int o = stage_override();
-  if (o == 0 || o == 1) return o == 1;
-  return sizeof(T) == 8 ? kN != 7 : (kN != 2 && kN != 5);
-}
-// gather pipeline (PIPE template parameter); PMG_VMULT_PIPE=0/1/2/3 overrides
-inline int pipe_override() {
-  static const int v = [] {
-    const char *e = std::getenv("PMG_VMULT_PIPE");
-    return e ? std::atoi(e) : -1;
-  }();
-  return v;
-}
-// Defaults from B200 sweeps (cell kernel time, 48^3..128^3 meshes), for the FP64 ring variant
-// without the L2 prefetch: the register pipeline (3) at N = 4 (deformed cube 128^3: Q3 1895 ->
-// 1758-1798 us); none at N = 5 (Q4: 3734-3764 us against 3803-3837 us with the register
-// pipeline, which was ahead, 4255 -> 4042 us, while the ring variant still prefetched); the
-// shared-memory index pipeline (1) at N = 3 (Q2 677 -> 657 us) and N >= 6 (Q5 +18 %; the
-// register pipeline there: 1186 -> 1428 us); and the index pipeline for the FP32 Q6 affine
-// kernel (+9 %; register pipeline 356 -> 435 us); none elsewhere (FP32 full geometry Q4 with
-// the register pipeline 2160 -> 2307 us, with the index pipeline 2415 us; Q4/Q5 affine and
-// FP64 Q6 affine lose 15-35 % with the index pipeline).
-template <typename T, int GEOM, bool SG> int use_pipe() {
-  const int o = pipe_override();
-  if (o >= 0 && o <= 3) return o;
-  if (SG) return sizeof(T) == 8 ? ((kN >= 6 || kN == 3) ? 1 : (kN == 4 ? 3 : 0)) : 0;
-  if ((GEOM == 1 || GEOM == 2) && kN == 7 && sizeof(T) == 4) return 1;
-  return 0;
+// ---- line kernels ----
+// Cells per block, cells per warp (0: lines follow one another across the warps of a block) and
+// the blocks per SM that registers are allocated for.  The fastest of the shapes measured on
+// B200 (64^3 cells, Q5 and Q6 32^3, Q6 with a coefficient 48^3; time in us with the shape next
+// in line): one warp per pair of Q3 cells needs no block barrier (FP64 full geometry 163; Q4 has
+// 25 lines, which leave 7 lanes of a warp idle, worth it in FP32: 230 against 236 in blocks of
+// five cells, not in FP64: 381 against 376); Q5 and Q6 fill 3 cells' lines into 4 and 5 warps.
+// MINB trades registers for warps: FP64 Q4 full geometry at 4 / 6 / 7 blocks 423 / 376 / 405,
+// Q6 with a coefficient FP64 at 4 / 6 blocks 339 / 328, FP32 at 7 / 8 blocks 220 / 211.
+template <typename T, int GEOM> constexpr auto line_shape() {
+  constexpr bool d = sizeof(T) == 8;
+  using kern::LineShape;
+  if constexpr (GEOM == 1) { // vmult_box_kernel
+    if constexpr (kN == 2) return LineShape<32, 8, 12>{};
+    else if constexpr (kN == 3) return LineShape<14, 0, 8>{};
+    else if constexpr (kN == 4) return LineShape<4, 2, 16>{};
+    else if constexpr (kN == 5 && d) return LineShape<2, 1, 12>{};
+    else if constexpr (kN == 5) return LineShape<5, 0, 10>{};
+    else if constexpr (kN == 6) return LineShape<3, 0, 9>{};
+    else return LineShape<3, 0, d ? 6 : 8>{};
+  } else if constexpr (GEOM == 2) {
+    if constexpr (kN == 2) return LineShape<16, 8, 20>{};
+    else if constexpr (kN == 4) return LineShape<4, 2, 12>{};
+    else if constexpr (kN == 5 && d) return LineShape<2, 1, 12>{};
+    else if constexpr (kN == 5) return LineShape<5, 0, 6>{};
+    else if constexpr (kN == 6 && d) return LineShape<3, 0, 9>{};
+    else if constexpr (kN == 6) return LineShape<8, 0, 3>{};
+    else return LineShape<3, 0, d ? 6 : 8>{};
+  } else {
+    if constexpr (kN == 4 && d) return LineShape<2, 2, 24>{};
+    else if constexpr (kN == 4) return LineShape<8, 2, 10>{};
+    else if constexpr (kN == 5 && d) return LineShape<5, 0, 6>{};
+    else if constexpr (kN == 5) return LineShape<2, 1, 10>{};
+    else if constexpr (kN == 6) return LineShape<3, 0, d ? 6 : 8>{};
+    else return LineShape<3, 0, d ? 4 : 7>{};
+  }
 }
 
+template <typename T, int GEOM> void line_launch(const SlabLaunch &L) {
+  using SH = decltype(line_shape<T, GEOM>());
+  const int64_t blocks = (L.n_cells + SH::CPB - 1) / SH::CPB;
+  constexpr int threads = kern::line_threads<kN, SH>();
+  const T *src = static_cast<const T *>(L.src);
+  T *dst = static_cast<T *>(L.dst);
+  const T c0 = (T)L.affine[0], c1 = (T)L.affine[1], c2 = (T)L.affine[2];
+  if constexpr (GEOM == 1) {
+    constexpr size_t smem = kern::box_smem<kN, T, SH>();
+    static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
+    kern::vmult_box_kernel<kN, T, SH><<<(unsigned)blocks, threads, smem, L.stream>>>(
+        box_tables<kN, T>(), src, dst, L.idx, c0, c1, c2, L.n_cells);
+  } else {
+    constexpr size_t smem = kern::line_smem<kN, T, SH>();
+    static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
+    kern::vmult_line_kernel<kN, T, GEOM, SH><<<(unsigned)blocks, threads, smem, L.stream>>>(
+        line_tables<kN, T>(), src, dst, L.idx, static_cast<const T *>(L.geo), static_cast<const T *>(L.coef), c0, c1,
+        c2, L.n_cells);
+  }
+  PMG_LAUNCH_CHECK();
+  if (L.units) *L.units = L.n_cells;
+  if (L.launched) *L.launched = blocks;
+}
 
-// Block shape of a vmult variant on the current device: warps per block and resident warps
-// per SM.  The direct variant keeps vmult_wpb(); the ring variant, whose warps share nothing,
-// takes the block size (1..8 warps) that fits the most warps per SM -- the per-block
-// shared-memory reservation can leave room for one more warp in one large block than in
-// one-warp blocks (Q4 FP64: 7 against 6).  PMG_RING_WPB=1..8 fixes it (a tuning switch).
+// ---- slab kernels (degrees 1 and 2) ----
+// Full geometry streams through the shared-memory column ring (TMA), except FP32 degree 1,
+// whose unrolled direct loads hide the latency at 8 warps/SM; the ring variant's index block is
+// copied one group ahead for FP64 degree 2 (677 -> 657 us at 128^3).
+template <typename T, int GEOM> constexpr bool use_ring() { return GEOM == 0 && (sizeof(T) == 8 || kN == 3); }
+template <typename T, int GEOM> constexpr int use_pipe() {
+  return (use_ring<T, GEOM>() && sizeof(T) == 8 && kN == 3) ? 1 : 0;
+}
+
+// Block shape of a slab vmult on the current device: warps per block and resident warps
+// per SM.  The direct variant takes four warps; the ring variant, whose warps share nothing,
+// takes the block size (1..8 warps) that fits the most warps per SM.
 struct VmultShape {
   int wpb = 1, warps_per_sm = 1;
 };
-inline int ring_wpb_override() {
-  static const int v = [] {
-    const char *e = std::getenv("PMG_RING_WPB");
-    return e ? std::atoi(e) : 0;
-  }();
-  return v;
-}
-template <typename T, int GEOM, bool SG, int PIPE> VmultShape vmult_shape() {
+template <typename T, int GEOM> VmultShape slab_shape() {
+  constexpr bool SG = use_ring<T, GEOM>();
+  constexpr int PIPE = use_pipe<T, GEOM>();
   static std::mutex mu;
   static std::map<int, VmultShape> cache; // device -> shape
   int dev = 0;
@@ -144,37 +157,27 @@ template <typename T, int GEOM, bool SG, int PIPE> VmultShape vmult_shape() {
   auto k = kern::vmult_slab_kernel<kN, T, GEOM, SG, PIPE>;
   constexpr size_t per_warp = kern::SlabSmem<kN, T, SG, PIPE>::PER_WARP;
   VmultShape best;
-  if (!SG) {
-    best.wpb = vmult_wpb<T, SG, PIPE>();
-    PMG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(best.wpb * per_warp)));
+  const int lo = SG ? 1 : kWarpsPerBlock, hi = SG ? 8 : kWarpsPerBlock;
+  PMG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(hi * per_warp)));
+  best.warps_per_sm = 0;
+  for (int w = lo; w <= hi; ++w) {
     int nb = 0;
-    PMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 32 * best.wpb, best.wpb * per_warp));
-    best.warps_per_sm = std::max(1, nb * best.wpb);
-  } else {
-    int max_smem = 0;
-    PMG_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const int hi = (int)std::min<size_t>(8, std::max<size_t>(1, (size_t)max_smem / per_warp));
-    PMG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(hi * per_warp)));
-    const int o = ring_wpb_override();
-    best.warps_per_sm = 0;
-    for (int w = 1; w <= hi; ++w) {
-      if (o >= 1 && o <= hi && w != o) continue;
-      int nb = 0;
-      PMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 32 * w, w * per_warp));
-      if (nb * w > best.warps_per_sm) {
-        best.wpb = w;
-        best.warps_per_sm = nb * w;
-      }
+    PMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 32 * w, w * per_warp));
+    if (nb * w > best.warps_per_sm) {
+      best.wpb = w;
+      best.warps_per_sm = nb * w;
     }
-    best.warps_per_sm = std::max(1, best.warps_per_sm);
   }
+  best.warps_per_sm = std::max(1, best.warps_per_sm);
   cache.emplace(dev, best);
   return best;
 }
 
-template <typename T, int GEOM, bool SG, int PIPE> void vmult_launch(const SlabLaunch &L) {
+template <typename T, int GEOM> void slab_launch(const SlabLaunch &L) {
+  constexpr bool SG = use_ring<T, GEOM>();
+  constexpr int PIPE = use_pipe<T, GEOM>();
   auto k = kern::vmult_slab_kernel<kN, T, GEOM, SG, PIPE>;
-  const VmultShape sh = vmult_shape<T, GEOM, SG, PIPE>();
+  const VmultShape sh = slab_shape<T, GEOM>();
   int sms = 0, dev = 0;
   PMG_CUDA(cudaGetDevice(&dev));
   PMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -186,33 +189,13 @@ template <typename T, int GEOM, bool SG, int PIPE> void vmult_launch(const SlabL
       make_tab<T>(L), static_cast<const T *>(L.src), static_cast<T *>(L.dst), L.idx,
       static_cast<const T *>(L.geo), static_cast<const T *>(L.coef), L.n_groups, L.err);
   PMG_LAUNCH_CHECK();
+  if (L.units) *L.units = L.n_groups;
   if (L.launched) *L.launched = (int64_t)grid * sh.wpb;
 }
 
-// The src-staging pipeline (PIPE 2) is built for the direct-load variant only: together with
-// the geometry column ring it raised "an illegal instruction was encountered" on B200
-// (Q1 FP64, deformed 4^3 mesh) for a cause not found, so that combination is not compiled.
-template <typename T, int GEOM, bool SG> void vmult_pipe(const SlabLaunch &L) {
-  const int pp = use_pipe<T, GEOM, SG>();
-  if constexpr (!SG) {
-    if (pp == 2) {
-      vmult_launch<T, GEOM, SG, 2>(L);
-      return;
-    }
-  }
-  if (pp == 3) vmult_launch<T, GEOM, SG, 3>(L);
-  else if (pp >= 1) vmult_launch<T, GEOM, SG, 1>(L);
-  else vmult_launch<T, GEOM, SG, 0>(L);
-}
-
 template <typename T, int GEOM> void vmult_geom(const SlabLaunch &L) {
-  if constexpr (GEOM == 0) {
-    if (use_ring<T>()) {
-      vmult_pipe<T, GEOM, true>(L);
-      return;
-    }
-  }
-  vmult_pipe<T, GEOM, false>(L);
+  if constexpr (kern::line_layout(kN, GEOM)) line_launch<T, GEOM>(L);
+  else slab_launch<T, GEOM>(L);
 }
 
 template <typename T, int GEOM> void diag_geom(const SlabLaunch &L) {
@@ -240,31 +223,12 @@ template <typename T> void diag_type(const SlabLaunch &L) {
   else diag_geom<T, 2>(L);
 }
 
-template <typename T, int GEOM, bool SG, int PIPE> int occ_vmult_variant() {
-  return vmult_shape<T, GEOM, SG, PIPE>().warps_per_sm; // resident warps per SM
-}
-// resident warps per SM of the direct variant (low 16 bits) and of the ring variant (high)
-template <typename T, int GEOM> int occ_vmult() {
-  const int direct = occ_vmult_variant<T, GEOM, false, 0>();
-  int ring = direct;
-  if constexpr (GEOM == 0) ring = occ_vmult_variant<T, GEOM, true, 0>();
-  return direct | (ring << 16);
-}
 template <typename T, int GEOM> int occ_diag() {
   auto k = kern::diag_slab_kernel<kN, T, GEOM>;
   allow_smem(k, diag_smem<T>());
   int nb = 0;
   PMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 32 * kWarpsPerBlock, diag_smem<T>()));
   return nb * kWarpsPerBlock; // resident warps per SM
-}
-
-template <typename T> int occ_vmult_geom(int geom) {
-  switch (geom) {
-  case 0: return occ_vmult<T, 0>();
-  case 1: return occ_vmult<T, 1>();
-  case 3: return occ_vmult<T, 3>();
-  default: return occ_vmult<T, 2>();
-  }
 }
 template <typename T> int occ_diag_geom(int geom) {
   switch (geom) {
@@ -285,10 +249,6 @@ void PMG_CAT(launch_vmult_p, PMG_DEGREE)(const SlabLaunch &L) {
 void PMG_CAT(launch_diag_p, PMG_DEGREE)(const SlabLaunch &L) {
   if (L.dtype == PMG_F64) diag_type<double>(L);
   else diag_type<float>(L);
-}
-
-int PMG_CAT(occupancy_vmult_p, PMG_DEGREE)(int dtype, int geom) {
-  return dtype == PMG_F64 ? occ_vmult_geom<double>(geom) : occ_vmult_geom<float>(geom);
 }
 
 int PMG_CAT(occupancy_diag_p, PMG_DEGREE)(int dtype, int geom) {

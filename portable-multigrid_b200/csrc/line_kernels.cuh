@@ -1,0 +1,391 @@
+// Cell kernels of the continuous Q_p Laplace operator with one thread per line of a cell.
+//
+// What they compute is the BK3 cell operator of the reference
+// (include/kernels/bk3_kokkos_kernel.h:25-746): per cell gather the nodal values (Dirichlet
+// entries read as 0), differentiate at the Gauss points, apply the symmetric geometry tensor,
+// integrate against the gradients and scatter-add.
+//
+// N^2 threads work on a cell, N = p+1.  A thread owns one line of N nodes along the direction
+// being contracted, so a 1D contraction is a register product against tables in the constant
+// bank; changing the direction is one exchange through shared memory.
+// vmult_line_kernel (any geometry) takes the lines z, y, x to the Gauss points and x, y, z back:
+//   z:  t = Sz u, tz = SDz u                                    (E1: 2 arrays)
+//   y:  w = Sy t, wy = SDy t, wz = Sy tz                        (E2: 3 arrays)
+//   x:  dx = SDx w, dy = Sx wy, dz = Sx wz;  f = G grad u;
+//       ax = SDx^T fx, ay = Sx^T fy, az = Sx^T fz               (E2: 3 arrays)
+//   y:  b = Sy^T ax + SDy^T ay, c = Sy^T az                     (E1: 2 arrays)
+//   z:  out = Sz^T b + SDz^T c, scatter
+// vmult_box_kernel (axis-aligned cells, no coefficient) uses that the cell matrix is the sum
+// cx K x M x M + cy M x K x M + cz M x M x K of Kronecker products of the 1D mass matrix M and
+// stiffness matrix K (the Gauss rule is exact for the products of two basis derivatives and
+// the same rule defines M), which takes 7 instead of 16 contractions:
+//   z:  a = Mz u, b = Kz u                                      (E1: 2 arrays)
+//   y:  v = My a, w = cy Ky a + cz My b                         (E2: 2 arrays)
+//   x:  out = cx Kx v + Mx w                                    (E3: 1 array)
+//   z:  scatter
+// Lines along z carry the gather and the scatter because the lanes of a warp then hold
+// neighbouring nodes of an (x, y) plane, which are neighbours in the first-visit numbering too.
+//
+// Against one lane per plane of a cell (laplace_kernels.cuh) a line needs a third of the
+// registers and its exchange buffers hold a third of the cell per thread, so 20 to 45 warps
+// are resident per SM instead of 7 or 8, at twice the shared-memory traffic.
+#pragma once
+
+#include "laplace_kernels.cuh"
+
+namespace pmg {
+namespace kern {
+
+// Layouts of the exchange buffers: node (i, j, k) of cell e is at e*CS + i*I + j*J + k*K.
+// Lanes: z lines r = j*N + i, x lines r = k*N + j, y lines r = k*N + i (YK = 0) or i*N + k
+// (YK = 1).  The strides are those with the fewest bank conflicts for the two access patterns
+// of each exchange (z and y, y and x, x and z), found by exhaustive search over permuted,
+// padded strides: for FP64 Q6, 467 shared-memory wavefronts per cell against 747 with one
+// layout for every exchange (429 without any conflict).
+template <int I_, int J_, int K_> struct XLayout {
+  static constexpr int I = I_, J = J_, K = K_;
+};
+template <int N, typename T> struct LineLayout;
+template <typename T> struct LineLayout<2, T> {
+  using E1 = XLayout<1, 2, 6>;
+  using E2 = XLayout<1, 3, 6>;
+  using E3 = XLayout<1, 2, 5>;
+  static constexpr int YK = 0, CS = 12;
+};
+template <typename T> struct LineLayout<3, T> {
+  using E1 = XLayout<3, 1, 9>;
+  using E2 = XLayout<1, 3, 9>;
+  using E3 = XLayout<1, 3, 9>;
+  static constexpr int YK = 0, CS = 27;
+};
+template <> struct LineLayout<4, float> {
+  using E1 = XLayout<1, 4, 20>;
+  using E2 = XLayout<1, 5, 20>;
+  using E3 = XLayout<1, 4, 17>;
+  static constexpr int YK = 0, CS = 80;
+};
+template <> struct LineLayout<4, double> {
+  using E1 = XLayout<4, 1, 17>;
+  using E2 = XLayout<1, 17, 4>;
+  using E3 = XLayout<1, 4, 17>;
+  static constexpr int YK = 0, CS = 67;
+};
+template <> struct LineLayout<5, float> {
+  using E1 = XLayout<5, 1, 25>;
+  using E2 = XLayout<1, 5, 25>;
+  using E3 = XLayout<1, 5, 25>;
+  static constexpr int YK = 0, CS = 125;
+};
+template <> struct LineLayout<5, double> {
+  using E1 = XLayout<5, 25, 1>;
+  using E2 = XLayout<25, 1, 5>;
+  using E3 = XLayout<1, 5, 25>;
+  static constexpr int YK = 1, CS = 125;
+};
+template <> struct LineLayout<6, float> {
+  using E1 = XLayout<1, 6, 38>;
+  using E2 = XLayout<1, 37, 6>;
+  using E3 = XLayout<1, 6, 37>;
+  static constexpr int YK = 0, CS = 228;
+};
+template <> struct LineLayout<6, double> {
+  using E1 = XLayout<1, 6, 38>;
+  using E2 = XLayout<1, 41, 6>;
+  using E3 = XLayout<1, 6, 37>;
+  static constexpr int YK = 0, CS = 244;
+};
+template <> struct LineLayout<7, float> {
+  using E1 = XLayout<7, 49, 1>;
+  using E2 = XLayout<49, 1, 7>;
+  using E3 = XLayout<1, 7, 49>;
+  static constexpr int YK = 1, CS = 343;
+};
+template <> struct LineLayout<7, double> {
+  using E1 = XLayout<7, 1, 49>;
+  using E2 = XLayout<1, 49, 7>;
+  using E3 = XLayout<1, 7, 49>;
+  static constexpr int YK = 0, CS = 353;
+};
+
+// The tables a line kernel reads
+template <int N, typename T> struct LineTab {
+  EvenOdd<N, T> eS, eSD, eST, eSDT;
+  T W[N];
+};
+// even/odd tables of the 1D mass matrix M and stiffness matrix K on the reference interval
+template <int N, typename T> struct BoxTab {
+  EvenOdd<N, T> eM, eK;
+};
+
+// CPB cells per block.  WC > 0: WC cells per warp, which only warp barriers order; WC = 0: the
+// N^2 threads of the cells follow one another across warps and block barriers order them.
+// MINB: blocks per SM that the registers are allocated for.
+template <int CPB_, int WC_, int MINB_> struct LineShape {
+  static constexpr int CPB = CPB_, WC = WC_, MINB = MINB_;
+};
+template <int N, typename SH> constexpr int line_threads() {
+  return SH::WC ? SH::CPB / (SH::WC ? SH::WC : 1) * 32 : (SH::CPB * N * N + 31) / 32 * 32;
+}
+
+// Position of a thread: its cell in the block and its lines in each direction and layout
+template <int N, typename T, typename SH> struct LinePlace {
+  using L = LineLayout<N, T>;
+  int e, r;      // cell of the block, line of the cell
+  bool active;   // holds a line
+  int z1, y1, y2, x2;
+  __device__ __forceinline__ LinePlace() {
+    constexpr int N2 = N * N;
+    const int t = threadIdx.x, u = SH::WC ? (t & 31) : t, c = u / N2;
+    r = u - c * N2;
+    e = SH::WC ? (t >> 5) * SH::WC + c : c;
+    active = SH::WC ? c < SH::WC : e < SH::CPB;
+    const int ra = r % N, rb = r / N, yi = L::YK ? rb : ra, yk = L::YK ? ra : rb, o = e * L::CS;
+    z1 = o + ra * L::E1::I + rb * L::E1::J;
+    y1 = o + yi * L::E1::I + yk * L::E1::K;
+    y2 = o + yi * L::E2::I + yk * L::E2::K;
+    x2 = o + ra * L::E2::J + rb * L::E2::K;
+  }
+  __device__ __forceinline__ static void sync() {
+    if constexpr (SH::WC != 0 || line_threads<N, SH>() == 32) __syncwarp();
+    else __syncthreads();
+  }
+};
+
+// the N entries of the index map on a z line (the sentinel for a cell past the end)
+template <int N> __device__ __forceinline__ void line_index(const uint32_t *__restrict__ idx, int64_t c, int r,
+                                                            bool in, uint64_t pol, uint32_t (&id)[N]) {
+  const uint32_t *ip = idx + c * (N * N * N) + r;
+#pragma unroll
+  for (int k = 0; k < N; ++k) id[k] = in ? ld_keep_early(ip + k * (N * N), pol) : kInvalidIdx;
+}
+
+template <int N, typename T, typename SH> constexpr size_t line_smem() {
+  return size_t(3) * SH::CPB * LineLayout<N, T>::CS * sizeof(T);
+}
+template <int N, typename T, typename SH> constexpr size_t box_smem() {
+  return size_t(4) * SH::CPB * LineLayout<N, T>::CS * sizeof(T);
+}
+
+// GEOM 0: full geometry [cell][x point][6][z point, y point]; 2: axis-aligned cells (diagonal
+// tensor cd0, cd3, cd5) times a coefficient per point, [cell][x point][z point, y point];
+// 3: inverse-Jacobian layout, as 0 with 10 components.
+// E1 and E2 share the three buffers (A0, A1 and B0, B1, B2), so a y line is read by every
+// thread before any is written; buffers of their own, with two barriers less, cost a fifth of
+// the resident warps and measured slower (FP64 Q4 455 against 419 us at 64^3).
+// The loop over the batches of cells is the grid: a loop in the kernel made the compiler keep
+// the tables in registers (FP64 Q6 207 instead of 88 registers, 652 against 330 us).
+// Full geometry is prefetched into L2 as one bulk request per block, issued before the index
+// map is read, and loaded where it is used: staging it in shared memory takes the room of a
+// block more per SM (FP64 Q4 419 against 376 us, Q3 211 against 163 us at 64^3).
+template <int N, typename T, int GEOM, typename SH>
+__global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
+    vmult_line_kernel(const __grid_constant__ LineTab<N, T> tab, const T *__restrict__ src, T *__restrict__ dst,
+                      const uint32_t *__restrict__ idx, const T *__restrict__ geo, const T *__restrict__ coef,
+                      T cd0, T cd3, T cd5, int64_t n_cells) {
+  using L = LineLayout<N, T>;
+  using E1 = typename L::E1;
+  using E2 = typename L::E2;
+  constexpr int N2 = N * N, N3 = N2 * N, CPB = SH::CPB, NCOMP = GEOM == 3 ? 10 : 6;
+  constexpr int GF = geo_cell_elems<N, T>(NCOMP);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T *A0 = reinterpret_cast<T *>(smem_raw), *A1 = A0 + CPB * L::CS, *A2 = A1 + CPB * L::CS;
+  const LinePlace<N, T, SH> at;
+  const int r = at.r;
+  const int64_t c0 = int64_t(blockIdx.x) * CPB, c = c0 + at.e;
+  const bool in = at.active && c < n_cells;
+  const uint64_t pol_first = policy_evict_first(), pol_last = policy_evict_last();
+  if constexpr (GEOM == 0 || GEOM == 3) {
+    if (threadIdx.x == 0) {
+      const int64_t left = n_cells - c0;
+      prefetch_l2(geo + c0 * GF, (uint32_t)((left < CPB ? (int)left : CPB) * GF * (int)sizeof(T)), pol_first);
+    }
+  }
+  uint32_t id[N];
+  line_index<N>(idx, c, r, in, pol_first, id);
+  T cf[GEOM == 2 ? N : 1]; // the coefficient on the x line, requested before the gather
+  if constexpr (GEOM == 2) {
+    const T *cp = coef + c * N3 + r;
+#pragma unroll
+    for (int p = 0; p < N; ++p) cf[p] = in ? ld_keep_early(cp + p * N2, pol_first) : T(0);
+  }
+  if (at.active) {
+    T u[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) u[k] = id[k] != kInvalidIdx ? ld_keep(src + id[k], pol_last) : T(0);
+    eo_apply<N, T, 1>(tab.eS, u, [&](int q, T v) { A0[at.z1 + q * E1::K] = v; });
+    eo_apply<N, T, -1>(tab.eSD, u, [&](int q, T v) { A1[at.z1 + q * E1::K] = v; });
+  }
+  at.sync();
+  {
+    T a[N], z[N];
+    if (at.active) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        a[j] = A0[at.y1 + j * E1::J];
+        z[j] = A1[at.y1 + j * E1::J];
+      }
+    }
+    at.sync();
+    if (at.active) {
+      eo_apply<N, T, 1>(tab.eS, a, [&](int q, T v) { A0[at.y2 + q * E2::J] = v; });
+      eo_apply<N, T, -1>(tab.eSD, a, [&](int q, T v) { A1[at.y2 + q * E2::J] = v; });
+      eo_apply<N, T, 1>(tab.eS, z, [&](int q, T v) { A2[at.y2 + q * E2::J] = v; });
+    }
+  }
+  at.sync();
+  if (at.active) {
+    if constexpr (GEOM == 2) {
+      // the tensor is diagonal: one direction at a time
+      const T wyz = line_weight<N, T>(tab.W, r % N) * line_weight<N, T>(tab.W, r / N);
+#pragma unroll
+      for (int p = 0; p < N; ++p) cf[p] *= tab.W[p] * wyz;
+      T l[N], d[N];
+#pragma unroll
+      for (int i = 0; i < N; ++i) l[i] = A0[at.x2 + i * E2::I];
+      eo_apply<N, T, -1>(tab.eSD, l, [&](int q, T v) { d[q] = (cf[q] * cd0) * v; });
+      eo_apply<N, T, -1>(tab.eSDT, d, [&](int q, T v) { A0[at.x2 + q * E2::I] = v; });
+#pragma unroll
+      for (int i = 0; i < N; ++i) l[i] = A1[at.x2 + i * E2::I];
+      eo_apply<N, T, 1>(tab.eS, l, [&](int q, T v) { d[q] = (cf[q] * cd3) * v; });
+      eo_apply<N, T, 1>(tab.eST, d, [&](int q, T v) { A1[at.x2 + q * E2::I] = v; });
+#pragma unroll
+      for (int i = 0; i < N; ++i) l[i] = A2[at.x2 + i * E2::I];
+      eo_apply<N, T, 1>(tab.eS, l, [&](int q, T v) { d[q] = (cf[q] * cd5) * v; });
+      eo_apply<N, T, 1>(tab.eST, d, [&](int q, T v) { A2[at.x2 + q * E2::I] = v; });
+    } else {
+      T dx[N], dy[N], dz[N];
+      {
+        T l[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) l[i] = A0[at.x2 + i * E2::I];
+        eo_apply<N, T, -1>(tab.eSD, l, [&](int q, T v) { dx[q] = v; });
+#pragma unroll
+        for (int i = 0; i < N; ++i) l[i] = A1[at.x2 + i * E2::I];
+        eo_apply<N, T, 1>(tab.eS, l, [&](int q, T v) { dy[q] = v; });
+#pragma unroll
+        for (int i = 0; i < N; ++i) l[i] = A2[at.x2 + i * E2::I];
+        eo_apply<N, T, 1>(tab.eS, l, [&](int q, T v) { dz[q] = v; });
+      }
+      const T *gp = geo + c * GF + r;
+#pragma unroll
+      for (int p = 0; p < N; ++p) {
+        T g[NCOMP];
+#pragma unroll
+        for (int m = 0; m < NCOMP; ++m) g[m] = in ? ld_keep(gp + (p * NCOMP + m) * N2, pol_first) : T(0);
+        const T x = dx[p], y = dy[p], z = dz[p];
+        if constexpr (GEOM == 0) {
+          dx[p] = g[0] * x + g[1] * y + g[2] * z;
+          dy[p] = g[1] * x + g[3] * y + g[4] * z;
+          dz[p] = g[2] * x + g[4] * y + g[5] * z;
+        } else { // J^{-1} row by row, then JxW: the physical gradient, times JxW, and back
+          T gx[3];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) gx[k] = g[NCOMP - 1] * (g[k] * x + g[3 + k] * y + g[(6 + k) % NCOMP] * z);
+          dx[p] = g[0] * gx[0] + g[1] * gx[1] + g[2] * gx[2];
+          dy[p] = g[3] * gx[0] + g[4] * gx[1] + g[5] * gx[2];
+          dz[p] = g[6 % NCOMP] * gx[0] + g[7 % NCOMP] * gx[1] + g[8 % NCOMP] * gx[2];
+        }
+      }
+      eo_apply<N, T, -1>(tab.eSDT, dx, [&](int q, T v) { A0[at.x2 + q * E2::I] = v; });
+      eo_apply<N, T, 1>(tab.eST, dy, [&](int q, T v) { A1[at.x2 + q * E2::I] = v; });
+      eo_apply<N, T, 1>(tab.eST, dz, [&](int q, T v) { A2[at.x2 + q * E2::I] = v; });
+    }
+  }
+  at.sync();
+  {
+    T a[N], z[N], o[N];
+    if (at.active) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        a[j] = A0[at.y2 + j * E2::J];
+        z[j] = A1[at.y2 + j * E2::J];
+      }
+      eo_apply<N, T, 1>(tab.eST, a, [&](int q, T v) { o[q] = v; });
+      eo_apply<N, T, -1>(tab.eSDT, z, [&](int q, T v) { o[q] += v; });
+#pragma unroll
+      for (int j = 0; j < N; ++j) a[j] = A2[at.y2 + j * E2::J];
+    }
+    at.sync();
+    if (at.active) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) A0[at.y1 + j * E1::J] = o[j];
+      eo_apply<N, T, 1>(tab.eST, a, [&](int q, T v) { A1[at.y1 + q * E1::J] = v; });
+    }
+  }
+  at.sync();
+  if (at.active) {
+    T a[N], z[N], o[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      a[k] = A0[at.z1 + k * E1::K];
+      z[k] = A1[at.z1 + k * E1::K];
+    }
+    eo_apply<N, T, 1>(tab.eST, a, [&](int q, T v) { o[q] = v; });
+    eo_apply<N, T, -1>(tab.eSDT, z, [&](int q, T v) { o[q] += v; });
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (id[k] != kInvalidIdx) red_keep(dst + id[k], o[k], pol_last);
+  }
+}
+
+// axis-aligned cells without a coefficient: (cx, cy, cz) = vol / h^2 per direction.  E1, E2 and
+// E3 have buffers of their own (E3 over E1's first), so three barriers order a cell.
+template <int N, typename T, typename SH>
+__global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
+    vmult_box_kernel(const __grid_constant__ BoxTab<N, T> tab, const T *__restrict__ src, T *__restrict__ dst,
+                     const uint32_t *__restrict__ idx, T cx, T cy, T cz, int64_t n_cells) {
+  using L = LineLayout<N, T>;
+  using E1 = typename L::E1;
+  using E2 = typename L::E2;
+  using E3 = typename L::E3;
+  constexpr int CPB = SH::CPB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T *A0 = reinterpret_cast<T *>(smem_raw), *A1 = A0 + CPB * L::CS, *B0 = A1 + CPB * L::CS, *B1 = B0 + CPB * L::CS;
+  const LinePlace<N, T, SH> at;
+  const int ra = at.r % N, rb = at.r / N;
+  const int64_t c = int64_t(blockIdx.x) * CPB + at.e;
+  const uint64_t pol_first = policy_evict_first(), pol_last = policy_evict_last();
+  uint32_t id[N];
+  line_index<N>(idx, c, at.r, at.active && c < n_cells, pol_first, id);
+  if (at.active) {
+    T u[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) u[k] = id[k] != kInvalidIdx ? ld_keep(src + id[k], pol_last) : T(0);
+    eo_apply<N, T, 1>(tab.eM, u, [&](int q, T v) { A0[at.z1 + q * E1::K] = v; });
+    eo_apply<N, T, 1>(tab.eK, u, [&](int q, T v) { A1[at.z1 + q * E1::K] = cz * v; });
+  }
+  at.sync();
+  if (at.active) {
+    T a[N], b[N], o[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      a[j] = A0[at.y1 + j * E1::J];
+      b[j] = A1[at.y1 + j * E1::J];
+    }
+    eo_apply<N, T, 1>(tab.eM, a, [&](int q, T v) { B0[at.y2 + q * E2::J] = v; });
+    eo_apply<N, T, 1>(tab.eK, a, [&](int q, T v) { o[q] = cy * v; });
+    eo_apply<N, T, 1>(tab.eM, b, [&](int q, T v) { B1[at.y2 + q * E2::J] = o[q] + v; });
+  }
+  at.sync();
+  if (at.active) {
+    T a[N], b[N], o[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      a[i] = B0[at.x2 + i * E2::I];
+      b[i] = B1[at.x2 + i * E2::I];
+    }
+    T *x3 = A0 + at.e * L::CS + ra * E3::J + rb * E3::K;
+    eo_apply<N, T, 1>(tab.eK, a, [&](int q, T v) { o[q] = cx * v; });
+    eo_apply<N, T, 1>(tab.eM, b, [&](int q, T v) { x3[q * E3::I] = o[q] + v; });
+  }
+  at.sync();
+  if (at.active) {
+    const T *z3 = A0 + at.e * L::CS + ra * E3::I + rb * E3::J;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (id[k] != kInvalidIdx) red_keep(dst + id[k], z3[k * E3::K], pol_last);
+  }
+}
+
+} // namespace kern
+} // namespace pmg

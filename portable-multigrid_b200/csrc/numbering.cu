@@ -186,19 +186,25 @@ __global__ void compact_flags_kernel(const uint8_t *__restrict__ f, const uint32
     }
 }
 
-// the slab layout of the index map: [group][k*N+i][e*N+j], sentinel on constrained DoFs
+// the kernels' index map, sentinel on constrained DoFs: cell by cell as `plain` (line layout), or
+// [group][k*N+i][e*N+j]
 __global__ void slab_index_kernel(const uint32_t *__restrict__ plain, const uint8_t *__restrict__ cons,
-                                  int64_t n_cells, int N, int cpw, int lanes, uint32_t *__restrict__ idx) {
+                                  int64_t n_cells, int N, bool line, int cpw, int lanes, uint32_t *__restrict__ idx) {
   const int N2 = N * N, N3 = N2 * N;
   const int64_t total = n_cells * N3;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t d = plain[t];
+    const uint32_t v = (d == kInvalid || cons[d]) ? kInvalid : d;
+    if (line) {
+      idx[t] = v;
+      continue;
+    }
     const int64_t c = t / N3;
     const int l = (int)(t - c * N3);
     const int i = l % N, j = (l / N) % N, k = l / N2;
-    const uint32_t d = plain[t];
     const int64_t grp = c / cpw;
     const int e = (int)(c - grp * cpw);
-    idx[(grp * N2 + k * N + i) * lanes + e * N + j] = (d == kInvalid || cons[d]) ? kInvalid : d;
+    idx[(grp * N2 + k * N + i) * lanes + e * N + j] = v;
   }
 }
 
@@ -280,14 +286,15 @@ void device_constrained(const uint8_t *cons, int64_t n, int sms, DeviceBuffer &l
   PMG_CUDA(cudaStreamSynchronize(s));
 }
 
-void device_slab_index(const uint32_t *plain, const uint8_t *cons, int64_t n_cells, int N, int cpw, int lanes,
-                       int64_t n_groups, int sms, DeviceBuffer &idx, cudaStream_t s) {
-  const int64_t n_idx = n_groups * N * N * lanes;
+void device_slab_index(const uint32_t *plain, const uint8_t *cons, int64_t n_cells, int N, bool line, int cpw,
+                       int lanes, int64_t n_groups, int sms, DeviceBuffer &idx, cudaStream_t s) {
+  const int64_t n_idx = n_groups * N * N * lanes; // (N^3 entries per cell, whole groups)
   idx.allocate(sizeof(uint32_t) * std::max<int64_t>(1, n_idx));
   PMG_CUDA(cudaMemsetAsync(idx.get(), 0xFF, idx.bytes(), s));
   const int64_t total = n_cells * N * N * N;
   if (total > 0) {
-    slab_index_kernel<<<grid_for(total, sms), 256, 0, s>>>(plain, cons, n_cells, N, cpw, lanes, idx.as<uint32_t>());
+    slab_index_kernel<<<grid_for(total, sms), 256, 0, s>>>(plain, cons, n_cells, N, line, cpw, lanes,
+                                                           idx.as<uint32_t>());
     PMG_LAUNCH_CHECK();
   }
 }

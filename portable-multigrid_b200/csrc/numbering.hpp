@@ -21,8 +21,9 @@ void exclusive_scan_u32(const uint32_t *in, uint32_t *out, int64_t n, cudaStream
 // the DoFs whose flag is set, ascending, and the bitmask of them; synchronises s
 void device_constrained(const uint8_t *cons, int64_t n, int sms, DeviceBuffer &list, DeviceBuffer &bits,
                         int64_t &n_constrained, cudaStream_t s);
-// the slab layout [group][k*N+i][e*N+j] of an index map, sentinel on constrained DoFs
-void device_slab_index(const uint32_t *plain, const uint8_t *cons, int64_t n_cells, int N, int cpw, int lanes,
-                       int64_t n_groups, int sms, DeviceBuffer &idx, cudaStream_t s);
+// the kernels' layout of an index map, sentinel on constrained DoFs: cell by cell (line layout) or
+// [group][k*N+i][e*N+j]
+void device_slab_index(const uint32_t *plain, const uint8_t *cons, int64_t n_cells, int N, bool line, int cpw,
+                       int lanes, int64_t n_groups, int sms, DeviceBuffer &idx, cudaStream_t s);
 
 } // namespace pmg

@@ -23,7 +23,9 @@ struct GeoParams {
   int deform;
   double amp;
   int nm, nq;
-  int N, cpw, lanes; // slab layout of the owning operator (nm == nq == N for G output)
+  int N, cpw, lanes; // layout of the owning operator's cell data (nm == nq == N for G output)
+  bool line;
+  int cell_geo; // line layout: values of a cell's full or inverse-Jacobian geometry
   double xl[kMaxNm];
   double S[kMaxNm * kMaxNq], SD[kMaxNm * kMaxNq], W[kMaxNq];
 };
@@ -40,6 +42,23 @@ __device__ __forceinline__ void map_point(const GeoParams &g, const double xr[3]
   }
 }
 
+// places of the cell data (kern::CellData with the sizes at run time)
+__device__ __forceinline__ int64_t at_geo(const GeoParams &g, int64_t c, int p, int q, int r, int m, int ncomp) {
+  if (g.line) return c * g.cell_geo + (p * ncomp + m) * (g.N * g.N) + r * g.N + q;
+  const int64_t grp = c / g.cpw;
+  return ((grp * (g.N * g.N) + p * g.N + q) * ncomp + m) * g.lanes + int(c - grp * g.cpw) * g.N + r;
+}
+__device__ __forceinline__ int64_t at_point(const GeoParams &g, int64_t c, int p, int q, int r) {
+  if (g.line) return (c * g.N + p) * (g.N * g.N) + r * g.N + q;
+  const int64_t grp = c / g.cpw;
+  return (grp * (g.N * g.N) + q * g.N + p) * g.lanes + int(c - grp * g.cpw) * g.N + r;
+}
+__device__ __forceinline__ int64_t at_index(const GeoParams &g, int64_t c, int i, int j, int k) {
+  if (g.line) return ((c * g.N + k) * g.N + j) * g.N + i;
+  const int64_t grp = c / g.cpw;
+  return (grp * (g.N * g.N) + k * g.N + i) * g.lanes + int(c - grp * g.cpw) * g.N + j;
+}
+
 __device__ __forceinline__ double coefficient(int kind, const double x[3]) {
   if (kind == PMG_COEFF_KAPPA)
     return 1.0 + 0.9 * sin(2 * M_PI * x[0]) * sin(2 * M_PI * x[1]) * sin(2 * M_PI * x[2]);
@@ -48,15 +67,15 @@ __device__ __forceinline__ double coefficient(int kind, const double x[3]) {
 
 // One block per cell (grid-stride): mapping nodes in shared memory, then per quadrature
 // point the Jacobian of the isoparametric Q_p map, its inverse and determinant.
-// mode 0: write G = coef * |det J| w_q J^{-1} J^{-T} into the slab layout (full geometry);
-// mode 1: write coef * (per-point factor) into the affine coefficient layout;
+// mode 0: write G = coef * |det J| w_q J^{-1} J^{-T} into the layout of full geometry;
+// mode 1: write coef * (per-point factor) into the layout of a value per point;
 // mode 2: right-hand side, b_i += sum_q phi_i(x_q) f(x_q) |det J| w_q (atomic);
 // mode 3: the quadrature points, out[cell][q][3];
-// mode 4: coef * |det J| w_q into the affine coefficient layout (mass-matrix weights);
+// mode 4: coef * |det J| w_q into the layout of a value per point (mass-matrix weights);
 // mode 5: out[cell] = (sum_q (u_h(x_q) - u(x_q))^2 |det J| w_q)^(1/2) for the exact solution
 //         u of f_kind 1 (sin(pi x) sin(pi y) sin(pi z)) or 2 (exp(x) sin(pi y) cos(pi z));
-// mode 6: write J^{-1} (9 entries, row d = d xi_d / dx) and coef * |det J| w_q into the slab
-//         layout of the inverse-Jacobian formulation, [group][x point][y point][10][lane];
+// mode 6: write J^{-1} (9 entries, row d = d xi_d / dx) and coef * |det J| w_q into the
+//         layout of full geometry with 10 components;
 // mode 7: out[dof][3] = the mapped position of every node (DoFs shared by cells receive the
 //         same value from each of them).
 template <typename T>
@@ -133,11 +152,6 @@ __global__ void cell_geometry_kernel(const GeoParams g, const int32_t *__restric
       const double wq = g.W[q0] * g.W[q1] * g.W[q2];
       double kap = coefficient(coeff_kind, xq);
       if (coef_values) kap *= coef_values[c * nq3 + q];
-      const int64_t grp = c / g.cpw;
-      const int e = (int)(c % g.cpw);
-      // full geometry is column-major per group (x point outer) so that each x column of a
-      // group is one contiguous chunk; the per-point coefficient stays row-major
-      const int m = q0 * g.N + q1, m_row = q1 * g.N + q0, lane = e * g.N + q2;
       if (mode == 0) {
         const double f = fabs(det) * wq * kap;
         int comp = 0;
@@ -145,19 +159,18 @@ __global__ void cell_geometry_kernel(const GeoParams g, const int32_t *__restric
           for (int d2 = d1; d2 < 3; ++d2) {
             const double s = inv[3 * d1] * inv[3 * d2] + inv[3 * d1 + 1] * inv[3 * d2 + 1] +
                              inv[3 * d1 + 2] * inv[3 * d2 + 2];
-            out[((grp * (g.N * g.N) + m) * 6 + comp) * g.lanes + lane] = (T)(f * s);
+            out[at_geo(g, c, q0, q1, q2, comp, 6)] = (T)(f * s);
             ++comp;
           }
       } else if (mode == 6) {
-        for (int comp = 0; comp < 9; ++comp)
-          out[((grp * (g.N * g.N) + m) * 10 + comp) * g.lanes + lane] = (T)inv[comp];
-        out[((grp * (g.N * g.N) + m) * 10 + 9) * g.lanes + lane] = (T)(fabs(det) * wq * kap);
+        for (int comp = 0; comp < 9; ++comp) out[at_geo(g, c, q0, q1, q2, comp, 10)] = (T)inv[comp];
+        out[at_geo(g, c, q0, q1, q2, 9, 10)] = (T)(fabs(det) * wq * kap);
       } else if (mode == 1) {
-        out[(grp * (g.N * g.N) + m_row) * g.lanes + lane] = (T)kap;
+        out[at_point(g, c, q0, q1, q2)] = (T)kap;
       } else if (mode == 3) {
         for (int d = 0; d < 3; ++d) out[(c * nq3 + q) * 3 + d] = (T)xq[d];
       } else if (mode == 4) {
-        out[(grp * (g.N * g.N) + m_row) * g.lanes + lane] = (T)(fabs(det) * wq * kap);
+        out[at_point(g, c, q0, q1, q2)] = (T)(fabs(det) * wq * kap);
       } else if (mode == 5) {
         double ex = 0.0;
         if (f_kind == 1) ex = sin(M_PI * xq[0]) * sin(M_PI * xq[1]) * sin(M_PI * xq[2]);
@@ -186,10 +199,7 @@ __global__ void cell_geometry_kernel(const GeoParams g, const int32_t *__restric
             for (int q0 = 0; q0 < nq; ++q0)
               s += g.S[i * nq + q0] * sjk * fq[(q2 * nq + q1) * nq + q0];
           }
-        const int64_t grp = c / g.cpw;
-        const int e = (int)(c % g.cpw);
-        // Y-slab layout of the index map: [group][k*N + i][lane = e*N + j]
-        const uint32_t id = idx_perm[(grp * (g.N * g.N) + k * g.N + i) * g.lanes + e * g.N + j];
+        const uint32_t id = idx_perm[at_index(g, c, i, j, k)];
         if (id != kInvalid) atomicAdd(out + id, (T)s);
       }
       __syncthreads();
@@ -222,6 +232,17 @@ __global__ void set_constrained_kernel(T *__restrict__ dst, const T *__restrict_
     dst[list[i]] = src ? src[list[i]] : value;
 }
 
+// line layout: values of a cell's geometry with ncomp values per point (kern::geo_cell_elems)
+int64_t geo_cell_elems(const pmg_operator &op, int ncomp) {
+  const int64_t s = (int64_t)dtype_size(op.dtype), n = (int64_t)ncomp * op.nm * op.nm * op.nm;
+  return (n * s + 15) / 16 * 16 / s;
+}
+// values of the whole geometry array
+int64_t geo_elems(const pmg_operator &op, int ncomp) {
+  const int64_t cells = std::max<int64_t>(1, op.n_groups) * op.cpw;
+  return op.line ? cells * geo_cell_elems(op, ncomp) : cells * ncomp * op.nm * op.nm * op.nm;
+}
+
 GeoParams make_geo_params(const pmg_operator &op, int nq) {
   GeoParams g{};
   const auto &b = op.mesh.box;
@@ -236,6 +257,8 @@ GeoParams make_geo_params(const pmg_operator &op, int nq) {
   g.N = op.nm;
   g.cpw = op.cpw;
   g.lanes = op.lanes;
+  g.line = op.line;
+  g.cell_geo = (int)geo_cell_elems(op, op.geometry == PMG_GEOMETRY_INVJAC ? 10 : 6);
   const Tables1D t = make_tables(op.degree, nq);
   for (int i = 0; i < op.nm; ++i) g.xl[i] = t.xl[i];
   for (size_t a = 0; a < t.S.size(); ++a) {
@@ -263,15 +286,12 @@ slab_fn diag_fn(int degree) {
                               launch_diag_p4, launch_diag_p5, launch_diag_p6};
   return f[degree];
 }
-int occupancy(bool diag, int degree, int dtype, int geom) {
+int occupancy_diag(int degree, int dtype, int geom) {
   typedef int (*occ_fn)(int, int);
-  static const occ_fn fv[] = {nullptr,           occupancy_vmult_p1, occupancy_vmult_p2,
-                              occupancy_vmult_p3, occupancy_vmult_p4, occupancy_vmult_p5,
-                              occupancy_vmult_p6};
   static const occ_fn fd[] = {nullptr,          occupancy_diag_p1, occupancy_diag_p2,
                               occupancy_diag_p3, occupancy_diag_p4, occupancy_diag_p5,
                               occupancy_diag_p6};
-  return (diag ? fd : fv)[degree](dtype, geom);
+  return fd[degree](dtype, geom);
 }
 
 int geom_code(const pmg_operator &op) {
@@ -286,7 +306,9 @@ SlabLaunch slab_launch(const pmg_operator &op, const Tables1D &t, cudaStream_t s
   L.geo = op.geo.get();
   L.coef = op.coef.get();
   L.n_groups = op.n_groups;
+  L.n_cells = op.n_cells;
   L.geom = geom_code(op);
+  for (int d = 0; d < 3; ++d) L.affine[d] = op.affine[d];
   L.dtype = op.dtype;
   L.stream = s;
   L.S = t.S.data();
@@ -296,11 +318,12 @@ SlabLaunch slab_launch(const pmg_operator &op, const Tables1D &t, cudaStream_t s
   return L;
 }
 
-// The index map with the sentinel, permuted into the Y-slab layout [group][k*N+i][e*N+j]
+// The index map with the sentinel in the kernels' layout
 // (setup_dof_indices_per_color, bk3.h:360-437) from the device numbering: entries that are
 // constrained DoFs, or the sentinel already, become the sentinel.
 void build_slab_index(pmg_operator &op) {
-  device_slab_index(op.dplain.as<uint32_t>(), op.dcons.as<uint8_t>(), op.n_cells, op.nm, op.cpw, op.lanes,
+  op.line = op.kind == PMG_OP_MASS ? kern::mass_line_layout(op.nm) : kern::line_layout(op.nm, geom_code(op));
+  device_slab_index(op.dplain.as<uint32_t>(), op.dcons.as<uint8_t>(), op.n_cells, op.nm, op.line, op.cpw, op.lanes,
                     op.n_groups, op.sms, op.idx, nullptr);
 }
 
@@ -310,29 +333,25 @@ void build_constrained(pmg_operator &op) {
                      op.n_constrained, nullptr);
 }
 
-// persistent grids (as many warps as can be resident on this device) and the error flag
+// the diagonal kernel's grid (as many warps as can be resident on this device) and the error flag
 void finish_setup(pmg_operator &op) {
   PMG_CUDA(cudaDeviceSynchronize());
   const int sms = num_sms(op.device);
-  const int gc = geom_code(op);
-  const int occ = occupancy(false, op.degree, op.dtype, gc);
-  op.warps_vmult = (int64_t)std::max(1, occ & 0xffff) * sms;
-  op.warps_vmult_ring = (int64_t)std::max(1, occ >> 16) * sms;
-  op.warps_diag = (int64_t)std::max(1, occupancy(true, op.degree, op.dtype, gc)) * sms;
+  op.warps_diag = (int64_t)std::max(1, occupancy_diag(op.degree, op.dtype, geom_code(op))) * sms;
   op.err_flag.allocate(sizeof(unsigned int));
   PMG_CUDA(cudaMemset(op.err_flag.get(), 0, sizeof(unsigned int)));
 }
 
-// Caller geometry (cell order of the caller, points lexicographic x fastest) into the slab
-// layout [group][x point p][y point q][ncomp][lane = e*N + z point r]:
+// Caller geometry (cell order of the caller, points lexicographic x fastest) into the kernels'
+// layout:
 //   mode 0: in = G[C][6][nq^3] (rr, rs, rt, ss, st, tt);
 //   mode 1: in = inv_jacobian[C][nq^3][3][3] (components 0..8), in2 = JxW[C][nq^3] (component 9).
 // One thread per input value: reads are coalesced, writes land in lane-contiguous runs.
 template <typename T>
 __global__ void geometry_from_caller_kernel(const double *__restrict__ in, const double *__restrict__ in2,
-                                            int mode, int64_t n_cells, int N, int cpw, int lanes,
+                                            int mode, int64_t n_cells, const GeoParams g,
                                             T *__restrict__ out) {
-  const int N2 = N * N, N3 = N2 * N, ncomp = mode == 0 ? 6 : 10, nin = mode == 0 ? 6 : 9;
+  const int N = g.N, N2 = N * N, N3 = N2 * N, ncomp = mode == 0 ? 6 : 10, nin = mode == 0 ? 6 : 9;
   const int64_t total = n_cells * N3 * (mode == 0 ? 6 : 10);
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     int64_t c;
@@ -358,9 +377,7 @@ __global__ void geometry_from_caller_kernel(const double *__restrict__ in, const
       v = in2[u];
     }
     const int p = pt % N, q = (pt / N) % N, r = pt / N2;
-    const int64_t grp = c / cpw;
-    const int e = (int)(c - grp * cpw);
-    out[((grp * N2 + p * N + q) * ncomp + comp) * lanes + e * N + r] = (T)v;
+    out[at_geo(g, c, p, q, r, comp, ncomp)] = (T)v;
   }
 }
 
@@ -432,11 +449,11 @@ void operator_setup_from_maps(pmg_operator &op, const pmg_operator_maps &m, cons
   op.dcons = upload(op.num.constrained);
   build_slab_index(op);
   build_constrained(op);
-  // geometry: the caller's arrays, permuted into the slab layout on the device
+  // geometry: the caller's arrays, permuted into the kernels' layout on the device
   const size_t s = dtype_size(op.dtype);
   const bool ij = m.geometry == PMG_MAPS_INVJAC;
   const int ncomp = ij ? 10 : 6;
-  op.geo.allocate(s * std::max<int64_t>(1, op.n_groups) * N2 * ncomp * op.lanes);
+  op.geo.allocate(s * geo_elems(op, ncomp));
   PMG_CUDA(cudaMemset(op.geo.get(), 0, op.geo.bytes()));
   if (op.n_cells > 0) {
     const int64_t n_in = op.n_cells * N3 * (ij ? 9 : 6);
@@ -446,13 +463,14 @@ void operator_setup_from_maps(pmg_operator &op, const pmg_operator_maps &m, cons
       in2.allocate(sizeof(double) * op.n_cells * N3);
       PMG_CUDA(cudaMemcpy(in2.get(), m.JxW, sizeof(double) * op.n_cells * N3, cudaMemcpyHostToDevice));
     }
+    const GeoParams gp = make_geo_params(op, op.nq);
     const int grid = (int)std::min<int64_t>((op.n_cells * N3 * ncomp + 255) / 256, (int64_t)op.sms * 32);
     if (op.dtype == PMG_F64)
       geometry_from_caller_kernel<double><<<grid, 256>>>(in.as<double>(), in2.as<double>(), ij ? 1 : 0, op.n_cells,
-                                                         N, op.cpw, op.lanes, op.geo.as<double>());
+                                                         gp, op.geo.as<double>());
     else
       geometry_from_caller_kernel<float><<<grid, 256>>>(in.as<double>(), in2.as<double>(), ij ? 1 : 0, op.n_cells,
-                                                        N, op.cpw, op.lanes, op.geo.as<float>());
+                                                        gp, op.geo.as<float>());
     PMG_LAUNCH_CHECK();
     PMG_CUDA(cudaDeviceSynchronize()); // the input buffers are freed on return
   }
@@ -577,7 +595,7 @@ void operator_setup(pmg_operator &op, const pmg_mesh &mesh, const pmg_operator_p
     }
   } else if (geometry == PMG_GEOMETRY_FULL || geometry == PMG_GEOMETRY_INVJAC) {
     const bool ij = geometry == PMG_GEOMETRY_INVJAC;
-    op.geo.allocate(s * op.n_groups * N2 * (ij ? 10 : 6) * op.lanes);
+    op.geo.allocate(s * geo_elems(op, ij ? 10 : 6));
     PMG_CUDA(cudaMemset(op.geo.get(), 0, op.geo.bytes()));
     if (op.dtype == PMG_F64)
       cell_geometry_kernel<double><<<grid, 128>>>(gp, xyz.as<int32_t>(), op.n_cells, ij ? 6 : 0, prm.coeff_kind,
@@ -597,6 +615,9 @@ void operator_setup(pmg_operator &op, const pmg_mesh &mesh, const pmg_operator_p
     c8[3] = vol / (h[1] * h[1]);
     c8[5] = vol / (h[2] * h[2]);
     c8[6] = vol;
+    op.affine[0] = c8[0];
+    op.affine[1] = c8[3];
+    op.affine[2] = c8[5];
     const int64_t n_slots = op.n_groups * op.cpw;
     if (op.dtype == PMG_F64) {
       std::vector<double> v(n_slots * 8, 0.0);
@@ -684,11 +705,9 @@ void operator_vmult(const pmg_operator &op, void *dst, const void *src, cudaStre
     SlabLaunch L = slab_launch(op, cached_tables(op.degree), s);
     L.src = src;
     L.dst = dst;
-    L.resident_warps = op.warps_vmult;
-    L.resident_warps_ring = op.warps_vmult_ring;
     L.err = op.err_flag.as<unsigned int>();
+    L.units = &op.launch_units[PMG_KERNEL_VMULT_CELL];
     L.launched = &op.launch_par[PMG_KERNEL_VMULT_CELL];
-    op.launch_units[PMG_KERNEL_VMULT_CELL] = op.n_groups;
     {
       prof::Scope scope("vmult_cell", s);
       if (op.tensor_cores) vmult_cells_tensor_cores(op, src, dst, s);
@@ -703,8 +722,8 @@ void operator_vmult(const pmg_operator &op, void *dst, const void *src, cudaStre
 }
 
 // The cells [cell_begin, cell_end) of the operator's cell order added into dst (after
-// vmult_init when init is set): the cell kernel on the warp groups that hold them, with the
-// index map, geometry and coefficient pointers advanced to the first of those groups.
+// vmult_init when init is set): the cell kernel with the index map, geometry and coefficient
+// pointers advanced to the first of them.
 void operator_vmult_cells(const pmg_operator &op, void *dst, const void *src, int64_t cell_begin,
                           int64_t cell_end, bool init, cudaStream_t s) {
   PMG_REQUIRE(dst && src, "null vector");
@@ -715,26 +734,25 @@ void operator_vmult_cells(const pmg_operator &op, void *dst, const void *src, in
   PMG_REQUIRE(cell_begin % op.cpw == 0 && (cell_end % op.cpw == 0 || cell_end == op.n_cells),
               "cell range bounds must be multiples of the cells per warp group (or the cell count)");
   if (init) vmult_init(op, dst, src, s);
-  const int64_t g0 = cell_begin / op.cpw, g1 = (cell_end + op.cpw - 1) / op.cpw;
-  if (g1 <= g0) return;
-  const int N2 = op.nm * op.nm;
-  const size_t sz = dtype_size(op.dtype);
+  if (cell_end <= cell_begin) return;
+  const int64_t N2 = (int64_t)op.nm * op.nm, N3 = N2 * op.nm, sz = (int64_t)dtype_size(op.dtype);
+  // entries per cell of the index map and of a value per point: whole groups, cpw cells each
+  // (cell_begin is a multiple of cpw, so both layouts start at cell_begin * N^3)
   SlabLaunch L = slab_launch(op, cached_tables(op.degree), s);
-  const int gc = geom_code(op);
-  L.idx = op.idx.as<uint32_t>() + g0 * N2 * op.lanes;
+  const int gc = geom_code(op), ncomp = gc == 3 ? 10 : 6;
+  L.idx = op.idx.as<uint32_t>() + cell_begin * N3;
   if (gc == 0 || gc == 3)
-    L.geo = static_cast<const char *>(op.geo.get()) + sz * g0 * N2 * (gc == 3 ? 10 : 6) * op.lanes;
+    L.geo = static_cast<const char *>(op.geo.get()) + sz * cell_begin * (op.line ? geo_cell_elems(op, ncomp) : ncomp * N3);
   else
-    L.geo = static_cast<const char *>(op.geo.get()) + sz * g0 * op.cpw * 8;
-  if (op.coef.get()) L.coef = static_cast<const char *>(op.coef.get()) + sz * g0 * N2 * op.lanes;
-  L.n_groups = g1 - g0;
+    L.geo = static_cast<const char *>(op.geo.get()) + sz * cell_begin * 8;
+  if (op.coef.get()) L.coef = static_cast<const char *>(op.coef.get()) + sz * cell_begin * N3;
+  L.n_cells = cell_end - cell_begin;
+  L.n_groups = (L.n_cells + op.cpw - 1) / op.cpw;
   L.src = src;
   L.dst = dst;
-  L.resident_warps = op.warps_vmult;
-  L.resident_warps_ring = op.warps_vmult_ring;
   L.err = op.err_flag.as<unsigned int>();
+  L.units = &op.launch_units[PMG_KERNEL_VMULT_CELL];
   L.launched = &op.launch_par[PMG_KERNEL_VMULT_CELL];
-  op.launch_units[PMG_KERNEL_VMULT_CELL] = L.n_groups;
   prof::Scope scope("vmult_cell", s);
   vmult_fn(op.degree)(L);
 }
@@ -795,7 +813,7 @@ void operator_assemble_rhs(const pmg_operator &op, int f_kind, int nq, void *b, 
 void operator_copy_geometry(const pmg_operator &op, double *host) {
   PMG_REQUIRE(op.geometry == PMG_GEOMETRY_FULL, "geometry copy needs the full geometry layout");
   const int N = op.nm, N2 = N * N, N3 = N2 * N;
-  const size_t n = (size_t)op.n_groups * N2 * 6 * op.lanes;
+  const size_t n = (size_t)geo_elems(op, 6);
   std::vector<double> g(n);
   if (op.dtype == PMG_F64) {
     PMG_CUDA(cudaMemcpy(g.data(), op.geo.get(), n * 8, cudaMemcpyDeviceToHost));
@@ -804,6 +822,7 @@ void operator_copy_geometry(const pmg_operator &op, double *host) {
     PMG_CUDA(cudaMemcpy(f.data(), op.geo.get(), n * 4, cudaMemcpyDeviceToHost));
     std::copy(f.begin(), f.end(), g.begin());
   }
+  const int64_t per_cell = geo_cell_elems(op, 6);
   for (int64_t c = 0; c < op.n_cells; ++c) {
     const int64_t grp = c / op.cpw, e = c % op.cpw;
     for (int r = 0; r < N; ++r)
@@ -811,7 +830,8 @@ void operator_copy_geometry(const pmg_operator &op, double *host) {
         for (int p = 0; p < N; ++p)
           for (int comp = 0; comp < 6; ++comp)
             host[(c * 6 + comp) * N3 + (r * N + q) * N + p] =
-                g[((grp * N2 + p * N + q) * 6 + comp) * op.lanes + e * N + r];
+                op.line ? g[c * per_cell + (p * 6 + comp) * N2 + r * N + q]
+                        : g[((grp * N2 + p * N + q) * 6 + comp) * op.lanes + e * N + r];
   }
 }
 

@@ -188,15 +188,17 @@ struct pmg_operator {
   int64_t n_cells = 0, n_dofs = 0;
   int cpw = 1, lanes = 1;           // cells per warp group, active lanes per group
   int64_t n_groups = 0;
+  bool line = false;                // cell data in the line layout (kern::CellData)
+  double affine[3] = {0, 0, 0};     // AFFINE: diagonal of the cell tensor (vol / h^2 per direction)
   // numbering on the device: plain [C][nm^3] (no sentinel; caller maps: the sentinel kept),
   // constrained flags [N], node lattice -> DoF (continuous box operators)
   pmg::DeviceBuffer dplain, dcons, dlattice;
   // host copy of the numbering, filled on first use (pmg::host_numbering); L and n_dofs always set
   mutable pmg::Numbering num;
   mutable bool host_num_valid = false;
-  pmg::DeviceBuffer idx;            // permuted [group][nm^2][lanes] uint32
-  pmg::DeviceBuffer geo;            // FULL: [group][nq^2][6][lanes]; AFFINE: [C][8]
-  pmg::DeviceBuffer coef;           // AFFINE with coefficient: [group][nq^2][lanes];
+  pmg::DeviceBuffer idx;            // uint32, n_groups * cpw cells of nm^3 entries
+  pmg::DeviceBuffer geo;            // FULL: 6 (INVJAC: 10) values per point; AFFINE: [C][8]
+  pmg::DeviceBuffer coef;           // AFFINE with coefficient: a value per point;
                                     // MASS with mass_geom 0: |det J| w_q (times coefficient)
   int mass_geom = 0;                // MASS: 1 = affine volume in geo[cell][6], 0 = coef
   pmg::DeviceBuffer coef_qp;        // PMG_COEFF_VALUES: the values [C][nq^3] FP64
@@ -207,8 +209,7 @@ struct pmg_operator {
   int64_t n_constrained = 0;
   pmg::DeviceBuffer inv_diag;       // [N] dtype
   bool has_diag = false;
-  int64_t warps_vmult = 0, warps_diag = 0; // resident warps of the cell kernels
-  int64_t warps_vmult_ring = 0;             // ... of the geometry-ring vmult variant
+  int64_t warps_diag = 0;                   // resident warps of the diagonal kernel
   int sms = 0;                              // SM count of the device
   std::vector<pmg::DeviceBuffer> cg_work;   // CG work vectors kept between solves
   std::vector<pmg::DeviceBuffer> adj_work;  // adjoint-gradient work vectors

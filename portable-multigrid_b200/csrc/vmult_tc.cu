@@ -17,6 +17,7 @@
 #include <map>
 #include <mutex>
 
+#include "laplace_kernels.cuh"
 #include "pmg_internal.hpp"
 #include "fields.hpp"
 #include "vmult_tc.hpp"
@@ -137,7 +138,8 @@ __global__ void __launch_bounds__(32 * kTcWarps) vmult_tc_kernel(const __grid_co
                                                                  const uint32_t *__restrict__ idx,
                                                                  const float *__restrict__ geo,
                                                                  const float *__restrict__ coef, int64_t n_cells) {
-  constexpr int CPW = 32 / N, LANES = CPW * N, N2 = N * N, N3 = N2 * N;
+  using CD = kern::CellData<N, kern::line_layout(N, GEOM)>;
+  constexpr int N2 = N * N, N3 = N2 * N;
   extern __shared__ __align__(16) float tc_smem[];
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   float *const A0 = tc_smem + (threadIdx.x >> 5) * kArrays * kArr;
@@ -149,12 +151,10 @@ __global__ void __launch_bounds__(32 * kTcWarps) vmult_tc_kernel(const __grid_co
   const int64_t warp0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   for (int64_t c = warp0; c < n_cells; c += nwarps) {
-    const int64_t grp = c / CPW;
-    const int e = (int)(c - grp * CPW);
-    // gather U[k][j][i] (sentinel -> 0) from the slab index map [group][k*N+i][e*N+j]
+    // gather U[k][j][i] (sentinel -> 0)
     for (int l = lane; l < N3; l += 32) {
       const int i = l % N, j = (l / N) % N, k = l / N2;
-      const uint32_t id = __ldg(idx + (grp * N2 + k * N + i) * LANES + e * N + j);
+      const uint32_t id = __ldg(idx + CD::idx(c, i, j, k));
       A0[off3(k, j, i)] = id != 0xFFFFFFFFu ? __ldg(src + id) : 0.f;
     }
     __syncwarp();
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(32 * kTcWarps) vmult_tc_kernel(const __grid_co
         float w = 0.f;
         if (qx < N && qy < N && qz < N) {
           w = tab.W[qx] * tab.W[qy] * tab.W[qz];
-          if (GEOM == 2) w *= __ldg(coef + (grp * N2 + qy * N + qx) * LANES + e * N + qz);
+          if (GEOM == 2) w *= __ldg(coef + CD::point(c, qx, qy, qz));
         }
         dx[m] *= c0 * w;
         dy[m] *= c3 * w;
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(32 * kTcWarps) vmult_tc_kernel(const __grid_co
         const int r = 16 * mt + g + (m >= 2 ? 8 : 0), i = 2 * t + (m & 1);
         const int k = r >> 3, j = r & 7;
         if (i < N && j < N && k < N) {
-          const uint32_t id = __ldg(idx + (grp * N2 + k * N + i) * LANES + e * N + j);
+          const uint32_t id = __ldg(idx + CD::idx(c, i, j, k));
           if (id != 0xFFFFFFFFu) atomicAdd(dst + id, o[m]);
         }
       }
