@@ -677,7 +677,8 @@ pmg_status pmg_vector_chebyshev_step(void *out, const void *cur, const void *pre
     NEED(inv_diag);
     PMG_REQUIRE(dtype == PMG_F64 || dtype == PMG_F32, "bad dtype");
     PMG_REQUIRE(n >= 0, "n must be >= 0");
-    if (n > 0) pmg::vec::cheb_update_into(out, cur, prev, src, Ax, inv_diag, f1, f2, dtype, n, as_stream(stream));
+    if (n > 0) pmg::vec::cheb_update(out, cur, prev, src, pmg::vec::Product{const_cast<void *>(Ax)}, inv_diag, f1, f2, dtype,
+                                    n, as_stream(stream));
   });
 }
 

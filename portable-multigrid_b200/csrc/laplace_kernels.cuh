@@ -35,6 +35,8 @@
 
 #include <cstdint>
 
+#include "pdl.cuh"
+
 namespace pmg {
 namespace kern {
 
@@ -396,6 +398,8 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : (sizeof(T) =
   constexpr int UNR = (SMEM_G || sizeof(T) == 4 || EO) ? N : 1;
   using SM = SlabSmem<N, T, SMEM_G, PIPE>;
   constexpr int NCOMP = GEOM == 3 ? 10 : 6; // geometry values per quadrature point
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   if (lane >= LANES) return;

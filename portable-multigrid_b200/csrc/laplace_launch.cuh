@@ -12,6 +12,7 @@
 #include "laplace_kernels.cuh"
 #include "line_kernels.cuh"
 #include "line_tables.hpp"
+#include "pdl.cuh"
 #include "pmg_internal.hpp"
 
 #ifndef PMG_DEGREE
@@ -115,16 +116,15 @@ template <typename T, int GEOM> void line_launch(const SlabLaunch &L) {
   if constexpr (GEOM == 1) {
     constexpr size_t smem = kern::box_smem<kN, T, SH>();
     static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
-    kern::vmult_box_kernel<kN, T, SH><<<(unsigned)blocks, threads, smem, L.stream>>>(
-        box_tables<kN, T>(), src, dst, L.idx, c0, c1, c2, L.n_cells);
+    launch_dependent(kern::vmult_box_kernel<kN, T, SH>, (unsigned)blocks, threads, smem, L.stream, box_tables<kN, T>(), src,
+                     dst, L.idx, c0, c1, c2, L.n_cells);
   } else {
     constexpr size_t smem = kern::line_smem<kN, T, SH>();
     static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
-    kern::vmult_line_kernel<kN, T, GEOM, SH><<<(unsigned)blocks, threads, smem, L.stream>>>(
-        line_tables<kN, T>(), src, dst, L.idx, static_cast<const T *>(L.geo), static_cast<const T *>(L.coef), c0, c1,
-        c2, L.n_cells);
+    launch_dependent(kern::vmult_line_kernel<kN, T, GEOM, SH>, (unsigned)blocks, threads, smem, L.stream,
+                     line_tables<kN, T>(), src, dst, L.idx, static_cast<const T *>(L.geo),
+                     static_cast<const T *>(L.coef), c0, c1, c2, L.n_cells);
   }
-  PMG_LAUNCH_CHECK();
   if (L.units) *L.units = L.n_cells;
   if (L.launched) *L.launched = blocks;
 }
@@ -185,10 +185,9 @@ template <typename T, int GEOM> void slab_launch(const SlabLaunch &L) {
   const int64_t resident_blocks = (int64_t)sh.warps_per_sm * sms / sh.wpb;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, resident_blocks));
   const size_t smem = (size_t)sh.wpb * kern::SlabSmem<kN, T, SG, PIPE>::PER_WARP;
-  k<<<grid, 32 * sh.wpb, smem, L.stream>>>(
-      make_tab<T>(L), static_cast<const T *>(L.src), static_cast<T *>(L.dst), L.idx,
-      static_cast<const T *>(L.geo), static_cast<const T *>(L.coef), L.n_groups, L.err);
-  PMG_LAUNCH_CHECK();
+  launch_dependent(k, grid, 32 * sh.wpb, smem, L.stream, make_tab<T>(L), static_cast<const T *>(L.src),
+                   static_cast<T *>(L.dst), L.idx, static_cast<const T *>(L.geo), static_cast<const T *>(L.coef),
+                   L.n_groups, L.err);
   if (L.units) *L.units = L.n_groups;
   if (L.launched) *L.launched = (int64_t)grid * sh.wpb;
 }

@@ -32,6 +32,7 @@
 #pragma once
 
 #include "laplace_kernels.cuh"
+#include "pdl.cuh"
 
 namespace pmg {
 namespace kern {
@@ -187,6 +188,7 @@ __global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
   using E2 = typename L::E2;
   constexpr int N2 = N * N, N3 = N2 * N, CPB = SH::CPB, NCOMP = GEOM == 3 ? 10 : 6;
   constexpr int GF = geo_cell_elems<N, T>(NCOMP);
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *A0 = reinterpret_cast<T *>(smem_raw), *A1 = A0 + CPB * L::CS, *A2 = A1 + CPB * L::CS;
   const LinePlace<N, T, SH> at;
@@ -201,7 +203,8 @@ __global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
     }
   }
   uint32_t id[N];
-  line_index<N>(idx, c, r, in, pol_first, id);
+  line_index<N>(idx, c, r, in, pol_first, id); // (fixed at setup: read before the wait)
+  pdl_wait();
   T cf[GEOM == 2 ? N : 1]; // the coefficient on the x line, requested before the gather
   if constexpr (GEOM == 2) {
     const T *cp = coef + c * N3 + r;
@@ -339,6 +342,7 @@ __global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
   using E2 = typename L::E2;
   using E3 = typename L::E3;
   constexpr int CPB = SH::CPB;
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *A0 = reinterpret_cast<T *>(smem_raw), *A1 = A0 + CPB * L::CS, *B0 = A1 + CPB * L::CS, *B1 = B0 + CPB * L::CS;
   const LinePlace<N, T, SH> at;
@@ -346,7 +350,8 @@ __global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
   const int64_t c = int64_t(blockIdx.x) * CPB + at.e;
   const uint64_t pol_first = policy_evict_first(), pol_last = policy_evict_last();
   uint32_t id[N];
-  line_index<N>(idx, c, at.r, at.active && c < n_cells, pol_first, id);
+  line_index<N>(idx, c, at.r, at.active && c < n_cells, pol_first, id); // (fixed at setup: read before the wait)
+  pdl_wait();
   if (at.active) {
     T u[N];
 #pragma unroll

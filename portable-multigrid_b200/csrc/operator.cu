@@ -214,16 +214,6 @@ __global__ void invert_diagonal_kernel(T *__restrict__ d, int64_t n) {
     d[i] = (d[i] != T(0)) ? T(1) / d[i] : T(1);
 }
 
-// dst_i = src_i on constrained DoFs (bit i of `bits`), 0 elsewhere
-template <typename T>
-__global__ void init_dst_kernel(T *__restrict__ dst, const T *__restrict__ src, const uint32_t *__restrict__ bits,
-                                int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t w = __ldg(bits + (i >> 5));
-    dst[i] = ((w >> (i & 31)) & 1u) ? src[i] : T(0);
-  }
-}
-
 template <typename T>
 __global__ void set_constrained_kernel(T *__restrict__ dst, const T *__restrict__ src,
                                        const uint32_t *__restrict__ list, int64_t n, T value) {
@@ -649,20 +639,10 @@ namespace {
 // dst = 0 (bk3.h:134) with the identity rows of copy_constrained_values (bk3.h:230) written
 // in the same pass: the cell kernels never touch constrained entries (index sentinel)
 void vmult_init(const pmg_operator &op, void *dst, const void *src, cudaStream_t s) {
-  const size_t bytes = dtype_size(op.dtype) * op.n_dofs;
-  if (op.n_constrained > 0) {
-    prof::Scope scope("vmult_init", s);
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((op.n_dofs + 255) / 256, (int64_t)op.sms * 16));
-    if (op.dtype == PMG_F64)
-      init_dst_kernel<double><<<grid, 256, 0, s>>>(static_cast<double *>(dst), static_cast<const double *>(src),
-                                                   op.constrained_bits.as<uint32_t>(), op.n_dofs);
-    else
-      init_dst_kernel<float><<<grid, 256, 0, s>>>(static_cast<float *>(dst), static_cast<const float *>(src),
-                                                  op.constrained_bits.as<uint32_t>(), op.n_dofs);
-    PMG_LAUNCH_CHECK();
-  } else {
-    PMG_CUDA(cudaMemsetAsync(dst, 0, bytes, s));
-  }
+  if (op.n_constrained > 0)
+    vec::init_product(dst, src, op.constrained_bits.as<uint32_t>(), op.dtype, op.n_dofs, s);
+  else
+    PMG_CUDA(cudaMemsetAsync(dst, 0, dtype_size(op.dtype) * op.n_dofs, s));
 }
 } // namespace
 
@@ -683,42 +663,62 @@ bool operator_vmult_chebyshev(const pmg_operator &op, void *out, const void *cur
   return ran;
 }
 
+namespace {
+// DG on 4x4x4 tiles: cell and face terms in one kernel that writes dst once; both launch records
+// describe it.  False, with nothing launched, elsewhere.
+bool vmult_fused(const pmg_operator &op, void *dst, const void *src, cudaStream_t s) {
+  if (!op.dg || op.n_cells == 0 || op.n_constrained > 0 || op.tensor_cores) return false;
+  prof::Scope scope("vmult_dg_tile", s);
+  if (!dg_apply_fused(*op.dg, op.degree, op.dtype, src, dst, op.n_cells, op.sms, s,
+                      &op.launch_units[PMG_KERNEL_DG_FACES], &op.launch_par[PMG_KERNEL_DG_FACES]))
+    return false;
+  op.launch_units[PMG_KERNEL_VMULT_CELL] = op.launch_units[PMG_KERNEL_DG_FACES];
+  op.launch_par[PMG_KERNEL_VMULT_CELL] = op.launch_par[PMG_KERNEL_DG_FACES];
+  return true;
+}
+
+// dst += the cells' (and faces') part of A src
+void add_product(const pmg_operator &op, void *dst, const void *src, cudaStream_t s) {
+  if (op.n_cells == 0) return;
+  if (op.kind == PMG_OP_MASS) {
+    prof::Scope scope("vmult_mass", s);
+    mass_vmult_cells(op, src, dst, s);
+    return;
+  }
+  SlabLaunch L = slab_launch(op, cached_tables(op.degree), s);
+  L.src = src;
+  L.dst = dst;
+  L.err = op.err_flag.as<unsigned int>();
+  L.units = &op.launch_units[PMG_KERNEL_VMULT_CELL];
+  L.launched = &op.launch_par[PMG_KERNEL_VMULT_CELL];
+  {
+    prof::Scope scope("vmult_cell", s);
+    if (op.tensor_cores) {
+      op.launch_units[PMG_KERNEL_VMULT_CELL] = op.n_groups;
+      vmult_cells_tensor_cores(op, src, dst, s);
+    } else {
+      vmult_fn(op.degree)(L);
+    }
+  }
+  if (op.dg) {
+    prof::Scope scope("vmult_dg_faces", s);
+    dg_apply_faces(*op.dg, op.degree, op.dtype, src, dst, op.n_cells, op.sms, s,
+                   &op.launch_units[PMG_KERNEL_DG_FACES], &op.launch_par[PMG_KERNEL_DG_FACES]);
+  }
+}
+} // namespace
+
 void operator_vmult(const pmg_operator &op, void *dst, const void *src, cudaStream_t s, bool compute) {
   PMG_REQUIRE(dst && src, "null vector");
   PMG_REQUIRE(dst != src, "vmult needs distinct src and dst");
-  if (compute && op.dg && op.n_cells > 0 && op.n_constrained == 0 && !op.tensor_cores) {
-    // DG on 4x4x4 tiles: cell and face terms in one kernel that writes dst once; both launch
-    // records describe it
-    prof::Scope scope("vmult_dg_tile", s);
-    if (dg_apply_fused(*op.dg, op.degree, op.dtype, src, dst, op.n_cells, op.sms, s,
-                       &op.launch_units[PMG_KERNEL_DG_FACES], &op.launch_par[PMG_KERNEL_DG_FACES])) {
-      op.launch_units[PMG_KERNEL_VMULT_CELL] = op.launch_units[PMG_KERNEL_DG_FACES];
-      op.launch_par[PMG_KERNEL_VMULT_CELL] = op.launch_par[PMG_KERNEL_DG_FACES];
-      return;
-    }
-  }
+  if (compute && vmult_fused(op, dst, src, s)) return;
   vmult_init(op, dst, src, s);
-  if (compute && op.n_cells > 0 && op.kind == PMG_OP_MASS) {
-    prof::Scope scope("vmult_mass", s);
-    mass_vmult_cells(op, src, dst, s);
-  } else if (compute && op.n_cells > 0) {
-    SlabLaunch L = slab_launch(op, cached_tables(op.degree), s);
-    L.src = src;
-    L.dst = dst;
-    L.err = op.err_flag.as<unsigned int>();
-    L.units = &op.launch_units[PMG_KERNEL_VMULT_CELL];
-    L.launched = &op.launch_par[PMG_KERNEL_VMULT_CELL];
-    {
-      prof::Scope scope("vmult_cell", s);
-      if (op.tensor_cores) vmult_cells_tensor_cores(op, src, dst, s);
-      else vmult_fn(op.degree)(L);
-    }
-    if (op.dg) {
-      prof::Scope scope("vmult_dg_faces", s);
-      dg_apply_faces(*op.dg, op.degree, op.dtype, src, dst, op.n_cells, op.sms, s,
-                     &op.launch_units[PMG_KERNEL_DG_FACES], &op.launch_par[PMG_KERNEL_DG_FACES]);
-    }
-  }
+  if (compute) add_product(op, dst, src, s);
+}
+
+vec::Product operator_product(const pmg_operator &op, void *Ax, const void *x, cudaStream_t s) {
+  if (!vmult_fused(op, Ax, x, s)) add_product(op, Ax, x, s);
+  return vec::Product{Ax, op.n_constrained > 0 ? op.constrained_bits.as<uint32_t>() : nullptr, true};
 }
 
 // The cells [cell_begin, cell_end) of the operator's cell order added into dst (after

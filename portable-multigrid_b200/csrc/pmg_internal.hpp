@@ -234,6 +234,12 @@ inline void require_mesh(const pmg_operator &op, const char *what) {
 }
 void operator_vmult(const pmg_operator &op, void *dst, const void *src, cudaStream_t s,
                     bool compute = true);
+namespace vec {
+struct Product;
+}
+// A x for an update that consumes it: Ax is zero before (but for the last update's clearing, see
+// vec::Product) and holds the sum over cells after; the fused DG kernel overwrites it
+vec::Product operator_product(const pmg_operator &op, void *Ax, const void *x, cudaStream_t s);
 void operator_vmult_cells(const pmg_operator &op, void *dst, const void *src, int64_t cell_begin,
                           int64_t cell_end, bool init, cudaStream_t s);
 bool operator_vmult_chebyshev(const pmg_operator &op, void *out, const void *cur, const void *prev, const void *b,

@@ -3,6 +3,7 @@
 // as the reference configures them (tests/poisson_cube_bk3/program.cc:474-515) and the
 // reference's multigrid driver (tests/common/portable_multigrid_solver.h:147-271,
 // include/multigrid/portable_v_cycle_multigrid.h:163-206).
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <vector>
@@ -63,6 +64,7 @@ void chebyshev_setup(pmg_chebyshev &c, pmg_operator &op, const pmg_chebyshev_par
   PMG_CUDA(cudaSetDevice(op.device));
   c.xo.allocate(bytes);
   c.Ax.allocate(bytes);
+  PMG_CUDA(cudaMemset(c.Ax.get(), 0, bytes)); // every product is consumed and cleared by its update
   if (!op.has_diag) {
     operator_compute_inverse_diagonal(op, nullptr);
     PMG_CUDA(cudaDeviceSynchronize());
@@ -91,33 +93,44 @@ void chebyshev_estimate(pmg_chebyshev &c, cudaStream_t s) {
   PMG_CUDA(cudaMemsetAsync(x.get(), 0, bytes, s));
   vec::fill_mod11(r.get(), dt, N, s);
   std::vector<double> diag, offd;
-  double res = std::sqrt(vec::dot(r.get(), r.get(), dt, N, s));
+  // The step lengths stay on the device and the host looks at the scalars once every kChunk
+  // iterations; iterations past the one at which CG stops are not looked at.
+  constexpr int kChunk = 16, kRho = 0, kRhoRing = kChunk + 2, kPv = kRhoRing, kRes = kPv + kChunk;
+  static_assert(kRes + kChunk + 1 <= vec::Scalars::kSlots, "scalar slots");
+  vec::Scalars sc(s);
+  const int kRes0 = kRes + kChunk;
+  sc.dot(kRes0, r.get(), r.get(), dt, N);
+  auto rho_slot = [&](int k) { return kRho + k % kRhoRing; }; // r.z before iteration k + 1
   int it = 0;
-  if (!(res <= 1e-10) && c.eig_its > 0) {
-    double rho = vec::jacobi_dot(z.get(), op.inv_diag.get(), r.get(), dt, N, s);
-    double rho_old = rho, alpha = 0, prev_alpha = 0, beta = 0, eig_beta_alpha = 0;
-    while (true) {
-      ++it;
-      if (it > 1) {
-        beta = rho / rho_old;
-        vec::xpay(p.get(), z.get(), beta, dt, N, s);
-      } else {
-        PMG_CUDA(cudaMemcpyAsync(p.get(), z.get(), bytes, cudaMemcpyDeviceToDevice, s));
+  if (c.eig_its > 0) {
+    double alpha = 0, prev_alpha = 0, beta = 0, eig_beta_alpha = 0;
+    sc.jacobi_dot(rho_slot(0), z.get(), op.inv_diag.get(), r.get(), dt, N);
+    for (bool done = false; !done;) {
+      const int chunk = std::min(kChunk, c.eig_its - it);
+      for (int k = 0; k < chunk; ++k) {
+        const int at = it + k + 1; // iteration
+        if (at > 1) sc.xpay(p.get(), z.get(), rho_slot(at - 1), rho_slot(at - 2), dt, N);
+        else PMG_CUDA(cudaMemcpyAsync(p.get(), z.get(), bytes, cudaMemcpyDeviceToDevice, s));
+        operator_vmult(op, v.get(), p.get(), s);
+        sc.dot(kPv + k, p.get(), v.get(), dt, N);
+        sc.cg_update(kRes + k, x.get(), r.get(), p.get(), v.get(), rho_slot(at - 1), kPv + k, dt, N);
+        sc.jacobi_dot(rho_slot(at), z.get(), op.inv_diag.get(), r.get(), dt, N);
       }
-      operator_vmult(op, v.get(), p.get(), s);
-      prev_alpha = alpha;
-      const double pv = vec::dot(p.get(), v.get(), dt, N, s);
-      check_finite(pv, "Chebyshev eigenvalue estimate");
-      alpha = rho / pv;
-      res = std::sqrt(vec::cg_update(x.get(), r.get(), p.get(), v.get(), alpha, dt, N, s));
-      rho_old = rho;
-      rho = vec::jacobi_dot(z.get(), op.inv_diag.get(), r.get(), dt, N, s);
-      if (it > 1) {
-        diag.push_back(1.0 / prev_alpha + eig_beta_alpha);
-        eig_beta_alpha = beta / prev_alpha;
-        offd.push_back(std::sqrt(beta) / prev_alpha);
+      sc.sync();
+      if (it == 0 && std::sqrt(sc[kRes0]) <= 1e-10) break;
+      for (int k = 0; k < chunk && !done; ++k) {
+        ++it;
+        if (it > 1) beta = sc[rho_slot(it - 1)] / sc[rho_slot(it - 2)];
+        prev_alpha = alpha;
+        check_finite(sc[kPv + k], "Chebyshev eigenvalue estimate");
+        alpha = sc[rho_slot(it - 1)] / sc[kPv + k];
+        if (it > 1) {
+          diag.push_back(1.0 / prev_alpha + eig_beta_alpha);
+          eig_beta_alpha = beta / prev_alpha;
+          offd.push_back(std::sqrt(beta) / prev_alpha);
+        }
+        done = it >= c.eig_its || std::sqrt(sc[kRes + k]) <= 1e-10;
       }
-      if (it >= c.eig_its || res <= 1e-10) break;
     }
   }
   c.cg_its = it;
@@ -138,7 +151,7 @@ void chebyshev_estimate(pmg_chebyshev &c, cudaStream_t s) {
   c.theta = (c.max_ev + alpha_ev) * 0.5;
   c.estimated = true;
   ++c.generation;
-  PMG_CUDA(cudaStreamSynchronize(s)); // the work vectors are freed on return
+  sc.sync(); // the work vectors are freed on return
 }
 
 // Chebyshev iteration of the first kind: vmult from x = 0 (degree-1 products), step from dst
@@ -158,15 +171,15 @@ void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zer
   void *cur = nullptr, *prev = nullptr; // x_k and x_{k-1} (null: x_{k-1} = 0)
   if (from_zero) {
     cur = ((d - 1) % 2 == 0) ? A : B;
-    vec::cheb_init(cur, nullptr, src, op.inv_diag.get(), 1.0 / c.theta, dt, N, s);
+    vec::cheb_init(cur, src, op.inv_diag.get(), 1.0 / c.theta, dt, N, s);
   } else {
-    operator_vmult(op, c.Ax.get(), dst, s);
+    const vec::Product Ax = operator_product(op, c.Ax.get(), dst, s);
     if (d % 2 == 0) { // x_1 into xo, x_0 stays in dst as the previous iterate
-      vec::cheb_first_step_into(B, A, src, c.Ax.get(), op.inv_diag.get(), 1.0 / c.theta, dt, N, s);
+      vec::cheb_first_step(B, nullptr, A, src, Ax, op.inv_diag.get(), 1.0 / c.theta, dt, N, s);
       cur = B;
       prev = A;
     } else { // x_0 moved to xo, x_1 in dst
-      vec::cheb_first_step(A, B, src, c.Ax.get(), op.inv_diag.get(), 1.0 / c.theta, dt, N, s);
+      vec::cheb_first_step(A, more ? B : nullptr, A, src, Ax, op.inv_diag.get(), 1.0 / c.theta, dt, N, s);
       cur = A;
       prev = B;
     }
@@ -181,8 +194,8 @@ void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zer
     void *out = prev ? prev : (cur == A ? B : A);
     // DG operators on cell tiles apply the step inside their vmult kernel (A cur never stored)
     if (!operator_vmult_chebyshev(op, out, cur, prev, src, op.inv_diag.get(), f1, f2, s)) {
-      operator_vmult(op, c.Ax.get(), cur, s);
-      vec::cheb_update_into(out, cur, prev, src, c.Ax.get(), op.inv_diag.get(), f1, f2, dt, N, s);
+      const vec::Product Ax = operator_product(op, c.Ax.get(), cur, s);
+      vec::cheb_update(out, cur, prev, src, Ax, op.inv_diag.get(), f1, f2, dt, N, s);
     }
     prev = cur;
     cur = out;
@@ -229,9 +242,9 @@ void mg_vcycle(pmg_mg &mg, int l, cudaStream_t s) {
   }
   pmg_operator &opc = *mg.levels[l - 1];
   chebyshev_apply(*mg.smoothers[l], mg.sol[l].get(), mg.def[l].get(), true, s);
-  operator_vmult(op, mg.t[l].get(), mg.sol[l].get(), s);
-  vec::residual(mg.t[l].get(), mg.def[l].get(), dt, N, s);
-  PMG_CUDA(cudaMemsetAsync(mg.def[l - 1].get(), 0, dtype_size(opc.dtype) * opc.n_dofs, s));
+  // t = def - A sol, and def[l - 1] = 0 for the restriction (portable_multigrid_solver.h:180-183)
+  const vec::Product Ax = operator_product(op, mg.smoothers[l]->Ax.get(), mg.sol[l].get(), s);
+  vec::residual(mg.t[l].get(), mg.def[l].get(), mg.sol[l].get(), Ax, mg.def[l - 1].get(), opc.n_dofs, dt, N, s);
   transfer_apply(*mg.transfers[l], 1, mg.def[l - 1].get(), mg.t[l].get(), s);
   mg_vcycle(mg, l - 1, s);
   transfer_apply(*mg.transfers[l], 0, mg.sol[l].get(), mg.sol[l - 1].get(), s);
@@ -239,14 +252,6 @@ void mg_vcycle(pmg_mg &mg, int l, cudaStream_t s) {
 }
 
 namespace {
-
-// defect[level] = 0 below the top (portable_multigrid_solver.h:180-183), then the cycle
-void mg_cycle_body(pmg_mg &mg, cudaStream_t s) {
-  const int L = (int)mg.levels.size() - 1;
-  for (int l = 0; l < L; ++l)
-    PMG_CUDA(cudaMemsetAsync(mg.def[l].get(), 0, dtype_size(mg.levels[l]->dtype) * mg.levels[l]->n_dofs, s));
-  mg_vcycle(mg, L, s);
-}
 
 bool graphs_allowed() {
   static const bool on = [] {
@@ -272,7 +277,7 @@ void mg_capture(pmg_mg &mg) {
   bool ok = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
   if (ok) {
     try {
-      mg_cycle_body(mg, cs);
+      mg_vcycle(mg, (int)mg.levels.size() - 1, cs);
     } catch (const Error &) {
       ok = false;
     }
@@ -311,7 +316,7 @@ void mg_vmult(pmg_mg &mg, void *dst, const void *src, int vec_dtype, cudaStream_
   vec::convert(mg.def[L].get(), top.dtype, src, vec_dtype, top.n_dofs, s);
   if (mg.graph_enabled && graphs_allowed() && !prof::enabled() && !mg.graph) mg_capture(mg);
   if (mg.graph && !prof::enabled()) PMG_CUDA(cudaGraphLaunch(mg.graph, s));
-  else mg_cycle_body(mg, s);
+  else mg_vcycle(mg, L, s);
   vec::convert(dst, vec_dtype, mg.sol[L].get(), top.dtype, top.n_dofs, s);
 }
 
@@ -333,32 +338,38 @@ void cg_solve(pmg_operator &A, pmg_mg *mg, void *x, const void *b, double reduce
     for (int i = 0; i < 4; ++i) A.cg_work.emplace_back(bytes);
   }
   DeviceBuffer &r = A.cg_work[0], &z = A.cg_work[1], &p = A.cg_work[2], &v = A.cg_work[3];
-  // r = b - A x and ||r|| in one pass
+  // r = b - A x and ||r|| in one pass; the step lengths stay on the device, and the host waits once
+  // per iteration, for the residual norm (with the scalars it checks)
+  enum { kRho = 0, kPv = 2, kRes = 3 }; // kRho, kRho + 1 in turn
+  vec::Scalars sc(s);
   operator_vmult(A, v.get(), x, s);
-  double res = std::sqrt(vec::residual_dot(r.get(), b, v.get(), dt, N, s));
+  sc.residual_dot(kRes, r.get(), b, v.get(), dt, N);
+  sc.sync();
+  double res = std::sqrt(sc[kRes]);
   check_finite(res, "CG residual");
   info = pmg_cg_info{};
   info.initial_residual = res;
   const double tol = std::max(abs_tol, reduce * res);
   int it = 0;
-  double rho = 0, rho_old = 0;
   while (res > tol && it < max_it) {
+    const int rho = kRho + (it & 1), rho_old = kRho + ((it + 1) & 1);
     if (mg) {
       mg_vmult(*mg, z.get(), r.get(), dt, s);
-      rho = vec::dot(r.get(), z.get(), dt, N, s);
+      sc.dot(rho, r.get(), z.get(), dt, N);
     } else {
-      rho = vec::jacobi_dot(z.get(), A.inv_diag.get(), r.get(), dt, N, s);
+      sc.jacobi_dot(rho, z.get(), A.inv_diag.get(), r.get(), dt, N);
     }
-    check_finite(rho, "CG preconditioned residual");
     if (it == 0) PMG_CUDA(cudaMemcpyAsync(p.get(), z.get(), bytes, cudaMemcpyDeviceToDevice, s));
-    else vec::xpay(p.get(), z.get(), rho / rho_old, dt, N, s);
-    rho_old = rho;
+    else sc.xpay(p.get(), z.get(), rho, rho_old, dt, N);
     ++it;
     operator_vmult(A, v.get(), p.get(), s);
-    const double pv = vec::dot(p.get(), v.get(), dt, N, s);
-    check_finite(pv, "CG curvature");
-    if (pv <= 0) fail(PMG_ENOCONV, "CG breakdown: p.Ap <= 0");
-    res = std::sqrt(vec::cg_update(x, r.get(), p.get(), v.get(), rho / pv, dt, N, s));
+    sc.dot(kPv, p.get(), v.get(), dt, N);
+    sc.cg_update(kRes, x, r.get(), p.get(), v.get(), rho, kPv, dt, N);
+    sc.sync();
+    check_finite(sc[rho], "CG preconditioned residual");
+    check_finite(sc[kPv], "CG curvature");
+    if (sc[kPv] <= 0) fail(PMG_ENOCONV, "CG breakdown: p.Ap <= 0");
+    res = std::sqrt(sc[kRes]);
     check_finite(res, "CG residual");
   }
   info.iterations = it;

@@ -10,6 +10,7 @@
 #include <map>
 #include <mutex>
 
+#include "pdl.cuh"
 #include "pmg_internal.hpp"
 #include "transfer.hpp"
 
@@ -112,8 +113,10 @@ __global__ void __launch_bounds__(32 * kPatchWarps)
   constexpr int A = Sh::A, B = Sh::B, NC3 = NC * NC * NC, NF3 = NF * NF * NF;
   __shared__ T sM[NC * NF];
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_trigger();
   for (int i = threadIdx.x; i < NC * NF; i += blockDim.x) sM[i] = P.m[i];
   __syncthreads();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   T *in = reinterpret_cast<T *>(smem_raw) + (threadIdx.x >> 5) * Sh::PER_WARP;
   T *t1 = in + Sh::A3;
@@ -207,10 +210,8 @@ void patch_launch(const pmg_transfer &t, void *dst, const void *src, cudaStream_
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)blocks * t.sms));
   t.launch_units = t.n_patches;
   t.launch_par = (int64_t)grid * kPatchWarps;
-  k<<<grid, 32 * kPatchWarps, smem, s>>>(P, static_cast<const T *>(src), static_cast<T *>(dst),
-                                         t.coarse_idx.as<uint32_t>(), t.fine_idx.as<uint32_t>(),
-                                         t.weights.as<T>(), t.n_patches);
-  PMG_LAUNCH_CHECK();
+  launch_dependent(k, grid, 32 * kPatchWarps, smem, s, P, static_cast<const T *>(src), static_cast<T *>(dst),
+                   t.coarse_idx.as<uint32_t>(), t.fine_idx.as<uint32_t>(), t.weights.as<T>(), t.n_patches);
 }
 
 // runtime (nc, nf) -> compiled pair; false if the pair has no compiled form

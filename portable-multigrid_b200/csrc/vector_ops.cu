@@ -1,8 +1,14 @@
 // Vector kernels of the Chebyshev smoother, the V-cycle and CG: fused updates (one pass
 // over HBM per update instead of deal.II's chain of sadd/add/DiagonalMatrix::vmult calls)
 // and deterministic dot products accumulated in FP64 whatever the vector type.
+//
+// All are bound by memory: every thread moves 16 bytes per vector and step where the vectors allow
+// it (all 16-byte aligned), else one entry.
+#include <cmath>
 #include <mutex>
+#include <vector>
 
+#include "pdl.cuh"
 #include "pmg_internal.hpp"
 #include "vector_ops.hpp"
 
@@ -25,180 +31,432 @@ int current_sms() {
   return n;
 }
 
-// grid of an elementwise grid-stride kernel: eight 256-thread blocks per SM at most
-inline int grid_for(int64_t n) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>((n + kBlock - 1) / kBlock, 8 * (int64_t)current_sms()));
+// grid of a grid-stride kernel over `items`: eight 256-thread blocks per SM at most
+inline int grid_for(int64_t items) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>((items + kBlock - 1) / kBlock, 8 * (int64_t)current_sms()));
+}
+inline int reduce_grid(int64_t items) {
+  return (int)std::min<int64_t>(kMaxPartials, std::max<int64_t>(1, (items + kBlock - 1) / kBlock));
 }
 
-#define GRID_STRIDE(i, n)                                                                     \
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n);                  \
-       i += (int64_t)gridDim.x * blockDim.x)
-
-template <typename T> __global__ void fill_mod11_k(T *x, int64_t n, double mean) {
-  GRID_STRIDE(i, n) x[i] = (T)((double)(i % 11) - mean);
+inline bool aligned16() { return true; }
+template <typename... P> bool aligned16(const void *p, P... rest) {
+  return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && aligned16(rest...);
 }
 
-template <typename TD, typename TS> __global__ void convert_k(TD *d, const TS *s, int64_t n) {
-  GRID_STRIDE(i, n) d[i] = (TD)s[i];
+// W consecutive entries of a vector
+template <typename T, int W> struct Pack {
+  T v[W];
+};
+template <int W, typename T> __device__ __forceinline__ Pack<T, W> load(const T *p) {
+  Pack<T, W> r;
+  constexpr int bytes = W * (int)sizeof(T);
+  if constexpr (bytes % 16 == 0) {
+#pragma unroll
+    for (int b = 0; b < bytes / 16; ++b) {
+      const uint4 q = reinterpret_cast<const uint4 *>(p)[b];
+      memcpy(reinterpret_cast<char *>(r.v) + 16 * b, &q, 16);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < W; ++k) r.v[k] = p[k];
+  }
+  return r;
 }
-
-template <typename T>
-__global__ void cheb_init_k(T *dst, T *xo, const T *src, const T *invd, T scale, int64_t n) {
-  GRID_STRIDE(i, n) {
-    dst[i] = scale * invd[i] * src[i];
-    if (xo) xo[i] = T(0);
+template <int W, typename T> __device__ __forceinline__ void store(T *p, const Pack<T, W> &r) {
+  constexpr int bytes = W * (int)sizeof(T);
+  if constexpr (bytes % 16 == 0) {
+#pragma unroll
+    for (int b = 0; b < bytes / 16; ++b) {
+      uint4 q;
+      memcpy(&q, reinterpret_cast<const char *>(r.v) + 16 * b, 16);
+      reinterpret_cast<uint4 *>(p)[b] = q;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < W; ++k) p[k] = r.v[k];
   }
 }
 
-template <typename T>
-__global__ void cheb_first_step_k(T *dst, T *xo, const T *src, const T *Ax, const T *invd, T scale,
-                                  int64_t n) {
-  GRID_STRIDE(i, n) {
-    const T x = dst[i];
-    xo[i] = x;
-    dst[i] = x + scale * invd[i] * (src[i] - Ax[i]);
+// f.template run<W>(i) for the entries i .. i+W-1 of every pack, run<1> for the tail
+template <int W, typename F> __device__ __forceinline__ void for_packs(int64_t n, F &f) {
+  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t m = n / W;
+  for (int64_t i = id; i < m; i += step) f.template run<W>(i * W);
+  if (W > 1 && id < n - m * W) f.template run<1>(m * W + id);
+}
+template <int W, typename F> __global__ void __launch_bounds__(kBlock) map_k(F f, int64_t n) {
+  pdl_trigger();
+  pdl_wait();
+  for_packs<W>(n, f);
+}
+// W: entries of a 16-byte pack of the widest type, if `wide`
+template <int W, typename F> void map(const F &f, int64_t n, bool wide, cudaStream_t s) {
+  if (wide) launch_dependent(map_k<W, F>, grid_for((n + W - 1) / W), kBlock, 0, s, f, n);
+  else launch_dependent(map_k<1, F>, grid_for(n), kBlock, 0, s, f, n);
+}
+template <typename T> constexpr int kW = 16 / (int)sizeof(T);
+
+template <typename T> struct FillMod11 {
+  T *x;
+  double mean;
+  template <int W> __device__ void run(int64_t i) {
+    Pack<T, W> r;
+#pragma unroll
+    for (int k = 0; k < W; ++k) r.v[k] = (T)((double)((i + k) % 11) - mean);
+    store<W>(x + i, r);
   }
-}
+};
 
-// the same first step into another vector: x0 is kept as the previous iterate
-template <typename T>
-__global__ void cheb_first_step_into_k(T *out, const T *x0, const T *src, const T *Ax, const T *invd,
-                                       T scale, int64_t n) {
-  GRID_STRIDE(i, n) {
-    const T x = x0[i];
-    out[i] = x + scale * invd[i] * (src[i] - Ax[i]);
+template <typename TD, typename TS> struct Convert {
+  TD *d;
+  const TS *s;
+  template <int W> __device__ void run(int64_t i) {
+    const auto a = load<W>(s + i);
+    Pack<TD, W> r;
+#pragma unroll
+    for (int k = 0; k < W; ++k) r.v[k] = (TD)a.v[k];
+    store<W>(d + i, r);
   }
-}
+};
 
-// the update written over the previous iterate (out == prev allowed; prev == nullptr: zero)
-template <typename T>
-__global__ void cheb_update_into_k(T *out, const T *cur, const T *prev, const T *src, const T *Ax,
-                                   const T *invd, T f1, T f2, int64_t n) {
-  GRID_STRIDE(i, n) {
-    const T x = cur[i];
-    const T xo = prev ? prev[i] : T(0);
-    out[i] = x + f1 * (x - xo) + f2 * invd[i] * (src[i] - Ax[i]);
+template <typename T> struct ChebInit {
+  T *dst;
+  const T *src, *invd;
+  T scale;
+  template <int W> __device__ void run(int64_t i) {
+    const auto b = load<W>(src + i), di = load<W>(invd + i);
+    Pack<T, W> r;
+#pragma unroll
+    for (int k = 0; k < W; ++k) r.v[k] = scale * di.v[k] * b.v[k];
+    store<W>(dst + i, r);
   }
+};
+
+// entries i .. of the product with the identity rows of x; zero afterwards if `clear`
+template <typename T> struct Consumed {
+  T *Ax;
+  const uint32_t *bits;
+  bool clear;
+  template <int W> __device__ Pack<T, W> take(int64_t i, const Pack<T, W> &x) const {
+    Pack<T, W> a = load<W>(Ax + i);
+    if (bits) { // (W divides 32: one word)
+      const uint32_t w = __ldg(bits + (i >> 5)) >> (i & 31);
+#pragma unroll
+      for (int k = 0; k < W; ++k)
+        if ((w >> k) & 1u) a.v[k] = x.v[k];
+    }
+    return a;
+  }
+  // called once the entries have been used: a store to a line whose load is still in flight stalls the
+  // load pipe (8.5M FP32 entries: an update that cleared first took 138 us, 37 without clearing)
+  template <int W> __device__ void done(int64_t i) const {
+    if (clear) store<W>(Ax + i, Pack<T, W>{});
+  }
+};
+
+template <typename T> struct InitProduct {
+  T *dst;
+  const T *src;
+  const uint32_t *bits;
+  template <int W> __device__ void run(int64_t i) {
+    Pack<T, W> r{};
+    const uint32_t w = __ldg(bits + (i >> 5)) >> (i & 31);
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+      if ((w >> k) & 1u) r.v[k] = src[i + k];
+    store<W>(dst + i, r);
+  }
+};
+
+template <typename T, bool KEEP> struct ChebFirst {
+  T *out, *keep;
+  const T *x0, *src;
+  Consumed<T> p;
+  const T *invd;
+  T scale;
+  template <int W> __device__ void run(int64_t i) {
+    const auto x = load<W>(x0 + i), b = load<W>(src + i), di = load<W>(invd + i), a = p.template take<W>(i, x);
+    Pack<T, W> r;
+#pragma unroll
+    for (int k = 0; k < W; ++k) r.v[k] = x.v[k] + scale * di.v[k] * (b.v[k] - a.v[k]);
+    if (KEEP) store<W>(keep + i, x);
+    store<W>(out + i, r);
+    p.template done<W>(i);
+  }
+};
+
+template <typename T, bool PREV> struct ChebUpdate {
+  T *out;
+  const T *cur, *prev, *src;
+  Consumed<T> p;
+  const T *invd;
+  T f1, f2;
+  template <int W> __device__ void run(int64_t i) {
+    const auto x = load<W>(cur + i), b = load<W>(src + i), di = load<W>(invd + i), a = p.template take<W>(i, x);
+    Pack<T, W> xo{}, r;
+    if (PREV) xo = load<W>(prev + i);
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+      r.v[k] = x.v[k] + f1 * (x.v[k] - xo.v[k]) + f2 * di.v[k] * (b.v[k] - a.v[k]);
+    store<W>(out + i, r);
+    p.template done<W>(i);
+  }
+};
+
+template <typename T> struct Residual {
+  T *t;
+  const T *def, *x;
+  Consumed<T> p;
+  template <int W> __device__ void run(int64_t i) {
+    Pack<T, W> xv{};
+    if (p.bits) xv = load<W>(x + i);
+    const auto b = load<W>(def + i), a = p.template take<W>(i, xv);
+    Pack<T, W> r;
+#pragma unroll
+    for (int k = 0; k < W; ++k) r.v[k] = b.v[k] - a.v[k];
+    store<W>(t + i, r);
+    p.template done<W>(i);
+  }
+};
+template <typename T> struct Zero {
+  T *p;
+  template <int W> __device__ void run(int64_t i) { store<W>(p + i, Pack<T, W>{}); }
+};
+template <int W, typename T>
+__global__ void __launch_bounds__(kBlock) residual_k(Residual<T> f, int64_t n, Zero<T> z, int64_t n_zero) {
+  pdl_trigger();
+  pdl_wait();
+  for_packs<W>(n, f);
+  for_packs<W>(n_zero, z);
 }
 
-template <typename T> __global__ void residual_k(T *t, const T *def, int64_t n) {
-  GRID_STRIDE(i, n) t[i] = def[i] - t[i];
+template <typename T> struct Jacobi {
+  T *z;
+  const T *invd, *r;
+  template <int W> __device__ void run(int64_t i) {
+    const auto d = load<W>(invd + i), a = load<W>(r + i);
+    Pack<T, W> v;
+#pragma unroll
+    for (int k = 0; k < W; ++k) v.v[k] = d.v[k] * a.v[k];
+    store<W>(z + i, v);
+  }
+};
+template <typename T> struct Xpay {
+  T *p;
+  const T *z;
+  T beta;
+  const double *rho, *rho_old; // beta = rho / rho_old where given
+  template <int W> __device__ void run(int64_t i) {
+    const auto a = load<W>(z + i), b = load<W>(p + i);
+    Pack<T, W> v;
+#pragma unroll
+    for (int k = 0; k < W; ++k) v.v[k] = a.v[k] + beta * b.v[k];
+    store<W>(p + i, v);
+  }
+};
+template <int W, typename T> __global__ void __launch_bounds__(kBlock) xpay_k(Xpay<T> f, int64_t n) {
+  pdl_trigger();
+  pdl_wait();
+  if (f.rho) f.beta = (T)(*f.rho / *f.rho_old);
+  for_packs<W>(n, f);
 }
+template <typename T> struct Axpy {
+  T *y;
+  const T *x;
+  T alpha;
+  template <int W> __device__ void run(int64_t i) {
+    const auto a = load<W>(x + i), b = load<W>(y + i);
+    Pack<T, W> v;
+#pragma unroll
+    for (int k = 0; k < W; ++k) v.v[k] = b.v[k] + alpha * a.v[k];
+    store<W>(y + i, v);
+  }
+};
 
-template <typename T> __global__ void jacobi_k(T *z, const T *invd, const T *r, int64_t n) {
-  GRID_STRIDE(i, n) z[i] = invd[i] * r[i];
-}
+// ---- reductions: every block stores a partial sum and the last block to arrive adds the
+// partials in a fixed order (deterministic), into device memory and into host-visible memory ----
+struct Sum {
+  double *partials;
+  unsigned int *arrived; // 0 between kernels
+  double *device, *host; // the result's places
+};
 
-template <typename T> __global__ void xpay_k(T *p, const T *z, T beta, int64_t n) {
-  GRID_STRIDE(i, n) p[i] = z[i] + beta * p[i];
-}
-
-template <typename T> __global__ void axpy_k(T *y, const T *x, T alpha, int64_t n) {
-  GRID_STRIDE(i, n) y[i] += alpha * x[i];
-}
-
-// block partial sums of a*b (or of the CG update's new r*r), FP64 accumulation
-template <typename T>
-__device__ __forceinline__ void block_reduce_store(double v, double *partials) {
+__device__ __forceinline__ double block_sum(double v) { // valid in thread 0
   __shared__ double red[kBlock / 32];
+  __syncthreads();
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    double w = (threadIdx.x < kBlock / 32) ? red[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) w += __shfl_down_sync(0xffffffffu, w, o);
-    if (threadIdx.x == 0) partials[blockIdx.x] = w;
+  v = threadIdx.x < kBlock / 32 ? red[threadIdx.x] : 0.0;
+  for (int o = kBlock / 64; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ void finish_sum(double v, const Sum &sum) {
+  __shared__ bool last;
+  v = block_sum(v);
+  if (threadIdx.x == 0) {
+    __stcg(sum.partials + blockIdx.x, v);
+    __threadfence();
+    last = atomicInc(sum.arrived, gridDim.x - 1) == gridDim.x - 1;
   }
-}
-
-template <typename T>
-__global__ void dot_partial_k(const T *a, const T *b, int64_t n, double *partials) {
-  double v = 0.0;
-  GRID_STRIDE(i, n) v += (double)a[i] * (double)b[i];
-  block_reduce_store<T>(v, partials);
-}
-
-template <typename T>
-__global__ void cg_update_k(T *x, T *r, const T *p, const T *v, T alpha, int64_t n, double *partials) {
-  double acc = 0.0;
-  GRID_STRIDE(i, n) {
-    x[i] += alpha * p[i];
-    const T ri = r[i] - alpha * v[i];
-    r[i] = ri;
-    acc += (double)ri * (double)ri;
-  }
-  block_reduce_store<T>(acc, partials);
-}
-
-// r = b - Ax and partial sums of r*r
-template <typename T>
-__global__ void residual_dot_k(T *r, const T *b, const T *Ax, int64_t n, double *partials) {
-  double acc = 0.0;
-  GRID_STRIDE(i, n) {
-    const T ri = b[i] - Ax[i];
-    r[i] = ri;
-    acc += (double)ri * (double)ri;
-  }
-  block_reduce_store<T>(acc, partials);
-}
-
-// z = invd * r and partial sums of r*z
-template <typename T>
-__global__ void jacobi_dot_k(T *z, const T *invd, const T *r, int64_t n, double *partials) {
-  double acc = 0.0;
-  GRID_STRIDE(i, n) {
-    const T zi = invd[i] * r[i];
-    z[i] = zi;
-    acc += (double)r[i] * (double)zi;
-  }
-  block_reduce_store<T>(acc, partials);
-}
-
-__global__ void finalize_k(const double *partials, int n_partials, double *out) {
-  // fixed-order tree over at most kMaxPartials values: deterministic
-  __shared__ double s[kMaxPartials];
-  for (int i = threadIdx.x; i < kMaxPartials; i += blockDim.x) s[i] = (i < n_partials) ? partials[i] : 0.0;
   __syncthreads();
-  for (int w = kMaxPartials / 2; w > 0; w >>= 1) {
-    for (int i = threadIdx.x; i < w; i += blockDim.x) s[i] += s[i + w];
-    __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double w = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kBlock) w += __ldcg(sum.partials + i);
+  w = block_sum(w);
+  if (threadIdx.x == 0) {
+    *sum.device = w;
+    *sum.host = w;
   }
-  if (threadIdx.x == 0) *out = s[0];
+}
+template <int W, typename F> __global__ void __launch_bounds__(kBlock) reduce_k(F f, int64_t n, Sum sum) {
+  pdl_trigger();
+  pdl_wait();
+  f.begin();
+  for_packs<W>(n, f);
+  finish_sum(f.acc, sum);
+}
+template <int W, typename F> void reduce(const F &f, int64_t n, bool wide, const Sum &sum, cudaStream_t s) {
+  if (wide) launch_dependent(reduce_k<W, F>, reduce_grid((n + W - 1) / W), kBlock, 0, s, f, n, sum);
+  else launch_dependent(reduce_k<1, F>, reduce_grid(n), kBlock, 0, s, f, n, sum);
 }
 
-struct Workspace {
-  DeviceBuffer partials;
-  DeviceBuffer results; // 64 doubles
-  double *host = nullptr; // pinned, 64 doubles
+template <typename T> struct Dot {
+  const T *a, *b;
+  double acc;
+  __device__ void begin() {}
+  template <int W> __device__ void run(int64_t i) {
+    const auto x = load<W>(a + i), y = load<W>(b + i);
+#pragma unroll
+    for (int k = 0; k < W; ++k) acc += (double)x.v[k] * (double)y.v[k];
+  }
+};
+template <typename T> struct CgUpdate {
+  T *x, *r;
+  const T *p, *v;
+  const double *rho, *pv;
+  double acc;
+  T alpha;
+  bool step;
+  __device__ void begin() {
+    const double a = *rho, b = *pv;
+    step = isfinite(a) && isfinite(b) && b > 0.0;
+    alpha = (T)(a / b);
+  }
+  template <int W> __device__ void run(int64_t i) {
+    Pack<T, W> rv = load<W>(r + i);
+    if (step) {
+      const auto pp = load<W>(p + i), vv = load<W>(v + i);
+      auto xv = load<W>(x + i);
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+        xv.v[k] += alpha * pp.v[k];
+        rv.v[k] = rv.v[k] - alpha * vv.v[k];
+      }
+      store<W>(x + i, xv);
+      store<W>(r + i, rv);
+    }
+#pragma unroll
+    for (int k = 0; k < W; ++k) acc += (double)rv.v[k] * (double)rv.v[k];
+  }
+};
+// r = b - Ax and r.r
+template <typename T> struct ResidualDot {
+  T *r;
+  const T *b, *Ax;
+  double acc;
+  __device__ void begin() {}
+  template <int W> __device__ void run(int64_t i) {
+    const auto x = load<W>(b + i), y = load<W>(Ax + i);
+    Pack<T, W> v;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      v.v[k] = x.v[k] - y.v[k];
+      acc += (double)v.v[k] * (double)v.v[k];
+    }
+    store<W>(r + i, v);
+  }
+};
+// z = invd * r and r.z
+template <typename T> struct JacobiDot {
+  T *z;
+  const T *invd, *r;
+  double acc;
+  __device__ void begin() {}
+  template <int W> __device__ void run(int64_t i) {
+    const auto d = load<W>(invd + i), a = load<W>(r + i);
+    Pack<T, W> v;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      v.v[k] = d.v[k] * a.v[k];
+      acc += (double)a.v[k] * (double)v.v[k];
+    }
+    store<W>(z + i, v);
+  }
 };
 
-Workspace &workspace() {
-  static std::mutex mu;
-  static Workspace ws[64];
+} // namespace
+
+// device and host-visible memory of one user of reductions; kept in a pool per device between
+// uses (at most kPool idle ones), so that concurrent users have memory of their own
+struct ScalarSpace {
+  int device = 0;
+  DeviceBuffer partials; // kMaxPartials partial sums, kSlots results, the arrival counter
+  double *host = nullptr;
+  ScalarSpace() = default;
+  ~ScalarSpace() {
+    if (host) cudaFreeHost(host);
+  }
+  Sum sum(int slot) {
+    double *p = partials.as<double>();
+    return Sum{p, reinterpret_cast<unsigned int *>(p + kMaxPartials + Scalars::kSlots), p + kMaxPartials + slot, host + slot};
+  }
+  const double *value(int slot) { return partials.as<double>() + kMaxPartials + slot; }
+};
+namespace {
+constexpr size_t kPool = 4;
+struct Pool {
+  std::mutex mu;
+  std::vector<std::unique_ptr<ScalarSpace>> idle;
+};
+Pool &pool() {
+  static Pool *p = new Pool; // never destroyed: the CUDA context may be gone by then
+  return *p;
+}
+} // namespace
+
+Scalars::Scalars(cudaStream_t s) : s_(s) {
   int dev = 0;
   PMG_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lock(mu);
-  Workspace &w = ws[dev & 63];
-  if (!w.partials.get()) {
-    w.partials.allocate(sizeof(double) * kMaxPartials * 4);
-    w.results.allocate(sizeof(double) * 64);
-    PMG_CUDA(cudaMallocHost(&w.host, sizeof(double) * 64));
+  {
+    Pool &p = pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    for (auto &w : p.idle)
+      if (w->device == dev) {
+        w_ = std::move(w);
+        std::swap(w, p.idle.back());
+        p.idle.pop_back();
+        return;
+      }
   }
-  return w;
+  w_ = std::make_unique<ScalarSpace>();
+  w_->device = dev;
+  w_->partials.allocate(sizeof(double) * (kMaxPartials + kSlots + 1));
+  PMG_CUDA(cudaMemset(w_->partials.get(), 0, w_->partials.bytes()));
+  PMG_CUDA(cudaDeviceSynchronize());
+  PMG_CUDA(cudaMallocHost(&w_->host, sizeof(double) * kSlots));
 }
-
-inline int reduce_grid(int64_t n) { return (int)std::min<int64_t>(kMaxPartials, std::max<int64_t>(1, (n + kBlock - 1) / kBlock)); }
-
-double finish(Workspace &w, int grid, int slot, cudaStream_t s) {
-  finalize_k<<<1, 1024, 0, s>>>(w.partials.as<double>(), grid, w.results.as<double>() + slot);
-  PMG_LAUNCH_CHECK();
-  PMG_CUDA(cudaMemcpyAsync(w.host + slot, w.results.as<double>() + slot, sizeof(double),
-                           cudaMemcpyDeviceToHost, s));
-  PMG_CUDA(cudaStreamSynchronize(s));
-  return w.host[slot];
+// the memory goes back to the pool only once no kernel uses it
+Scalars::~Scalars() {
+  const bool ok = cudaStreamSynchronize(s_) == cudaSuccess;
+  Pool &p = pool();
+  std::lock_guard<std::mutex> lock(p.mu);
+  if (ok && p.idle.size() < kPool) p.idle.push_back(std::move(w_));
 }
-
-} // namespace
+void Scalars::sync() { PMG_CUDA(cudaStreamSynchronize(s_)); }
+double Scalars::operator[](int slot) const { return w_->host[slot]; }
 
 #define DISPATCH(dtype, ...)                                                                  \
   do {                                                                                        \
@@ -211,14 +469,19 @@ double finish(Workspace &w, int grid, int slot, cudaStream_t s) {
     }                                                                                         \
   } while (0)
 
+namespace {
+template <typename T> const T *in(const void *p) { return static_cast<const T *>(p); }
+template <typename T> T *io(void *p) { return static_cast<T *>(p); }
+template <typename T> Consumed<T> consumed(const Product &p) { return Consumed<T>{io<T>(p.Ax), p.bits, p.clear}; }
+} // namespace
+
 void fill_mod11(void *x, int dtype, int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
   // mean of (i mod 11) over i < n, exactly
   const int64_t full = n / 11, rem = n % 11;
   const double sum = double(full) * 55.0 + double(rem * (rem - 1) / 2);
   const double mean = n > 0 ? sum / double(n) : 0.0;
-  DISPATCH(dtype, fill_mod11_k<T><<<grid_for(n), kBlock, 0, s>>>(static_cast<T *>(x), n, mean));
-  PMG_LAUNCH_CHECK();
+  DISPATCH(dtype, map<kW<T>>(FillMod11<T>{io<T>(x), mean}, n, aligned16(x), s));
 }
 
 void convert(void *dst, int dt_dst, const void *src, int dt_src, int64_t n, cudaStream_t s) {
@@ -227,114 +490,114 @@ void convert(void *dst, int dt_dst, const void *src, int dt_src, int64_t n, cuda
     PMG_CUDA(cudaMemcpyAsync(dst, src, dtype_size(dt_dst) * n, cudaMemcpyDeviceToDevice, s));
     return;
   }
-  if (dt_dst == PMG_F32)
-    convert_k<float, double><<<grid_for(n), kBlock, 0, s>>>(static_cast<float *>(dst), static_cast<const double *>(src), n);
-  else
-    convert_k<double, float><<<grid_for(n), kBlock, 0, s>>>(static_cast<double *>(dst), static_cast<const float *>(src), n);
-  PMG_LAUNCH_CHECK();
+  const bool wide = aligned16(dst, src);
+  if (dt_dst == PMG_F32) map<4>(Convert<float, double>{io<float>(dst), in<double>(src)}, n, wide, s);
+  else map<4>(Convert<double, float>{io<double>(dst), in<float>(src)}, n, wide, s);
 }
 
-void cheb_init(void *dst, void *xo, const void *src, const void *invd, double scale, int dtype,
-               int64_t n, cudaStream_t s) {
+void init_product(void *dst, const void *src, const uint32_t *bits, int dtype, int64_t n, cudaStream_t s) {
+  prof::Scope scope_("vmult_init", s);
+  DISPATCH(dtype, map<kW<T>>(InitProduct<T>{io<T>(dst), in<T>(src), bits}, n, aligned16(dst), s));
+}
+
+void cheb_init(void *dst, const void *src, const void *invd, double scale, int dtype, int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
-  DISPATCH(dtype, cheb_init_k<T><<<grid_for(n), kBlock, 0, s>>>(static_cast<T *>(dst), static_cast<T *>(xo),
-                                                                 static_cast<const T *>(src), static_cast<const T *>(invd), (T)scale, n));
-  PMG_LAUNCH_CHECK();
+  DISPATCH(dtype, map<kW<T>>(ChebInit<T>{io<T>(dst), in<T>(src), in<T>(invd), (T)scale}, n, aligned16(dst, src, invd), s));
 }
 
-void cheb_first_step(void *dst, void *xo, const void *src, const void *Ax, const void *invd,
+void cheb_first_step(void *out, void *keep, const void *x0, const void *src, const Product &p, const void *invd,
                      double scale, int dtype, int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
-  DISPATCH(dtype, cheb_first_step_k<T><<<grid_for(n), kBlock, 0, s>>>(
-                      static_cast<T *>(dst), static_cast<T *>(xo), static_cast<const T *>(src),
-                      static_cast<const T *>(Ax), static_cast<const T *>(invd), (T)scale, n));
-  PMG_LAUNCH_CHECK();
+  const bool wide = aligned16(out, keep, x0, src, p.Ax, invd);
+  if (keep)
+    DISPATCH(dtype, map<kW<T>>(ChebFirst<T, true>{io<T>(out), io<T>(keep), in<T>(x0), in<T>(src), consumed<T>(p),
+                                                  in<T>(invd), (T)scale}, n, wide, s));
+  else
+    DISPATCH(dtype, map<kW<T>>(ChebFirst<T, false>{io<T>(out), nullptr, in<T>(x0), in<T>(src), consumed<T>(p),
+                                                   in<T>(invd), (T)scale}, n, wide, s));
 }
 
-void cheb_first_step_into(void *out, const void *x0, const void *src, const void *Ax, const void *invd,
-                          double scale, int dtype, int64_t n, cudaStream_t s) {
+void cheb_update(void *out, const void *cur, const void *prev, const void *src, const Product &p, const void *invd,
+                 double f1, double f2, int dtype, int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
-  DISPATCH(dtype, cheb_first_step_into_k<T><<<grid_for(n), kBlock, 0, s>>>(
-                      static_cast<T *>(out), static_cast<const T *>(x0), static_cast<const T *>(src),
-                      static_cast<const T *>(Ax), static_cast<const T *>(invd), (T)scale, n));
-  PMG_LAUNCH_CHECK();
+  const bool wide = aligned16(out, cur, prev, src, p.Ax, invd);
+  if (prev)
+    DISPATCH(dtype, map<kW<T>>(ChebUpdate<T, true>{io<T>(out), in<T>(cur), in<T>(prev), in<T>(src), consumed<T>(p),
+                                                   in<T>(invd), (T)f1, (T)f2}, n, wide, s));
+  else
+    DISPATCH(dtype, map<kW<T>>(ChebUpdate<T, false>{io<T>(out), in<T>(cur), nullptr, in<T>(src), consumed<T>(p),
+                                                    in<T>(invd), (T)f1, (T)f2}, n, wide, s));
 }
 
-void cheb_update_into(void *out, const void *cur, const void *prev, const void *src, const void *Ax,
-                      const void *invd, double f1, double f2, int dtype, int64_t n, cudaStream_t s) {
+void residual(void *t, const void *def, const void *x, const Product &p, void *zero, int64_t n_zero, int dtype,
+              int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
-  DISPATCH(dtype, cheb_update_into_k<T><<<grid_for(n), kBlock, 0, s>>>(
-                      static_cast<T *>(out), static_cast<const T *>(cur), static_cast<const T *>(prev),
-                      static_cast<const T *>(src), static_cast<const T *>(Ax), static_cast<const T *>(invd),
-                      (T)f1, (T)f2, n));
-  PMG_LAUNCH_CHECK();
-}
-
-void residual(void *t, const void *def, int dtype, int64_t n, cudaStream_t s) {
-  prof::Scope scope_("vector_update", s);
-  DISPATCH(dtype, residual_k<T><<<grid_for(n), kBlock, 0, s>>>(static_cast<T *>(t), static_cast<const T *>(def), n));
-  PMG_LAUNCH_CHECK();
+  if (!zero) n_zero = 0;
+  const bool wide = aligned16(t, def, x, p.Ax, zero);
+  DISPATCH(dtype, {
+    const Residual<T> f{io<T>(t), in<T>(def), in<T>(x), consumed<T>(p)};
+    const Zero<T> z{io<T>(zero)};
+    if (wide)
+      launch_dependent(residual_k<kW<T>, T>, grid_for((std::max(n, n_zero) + kW<T> - 1) / kW<T>), kBlock, 0, s, f, n, z, n_zero);
+    else
+      launch_dependent(residual_k<1, T>, grid_for(std::max(n, n_zero)), kBlock, 0, s, f, n, z, n_zero);
+  });
 }
 
 void jacobi(void *z, const void *invd, const void *r, int dtype, int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
-  DISPATCH(dtype, jacobi_k<T><<<grid_for(n), kBlock, 0, s>>>(static_cast<T *>(z), static_cast<const T *>(invd),
-                                                              static_cast<const T *>(r), n));
-  PMG_LAUNCH_CHECK();
+  DISPATCH(dtype, map<kW<T>>(Jacobi<T>{io<T>(z), in<T>(invd), in<T>(r)}, n, aligned16(z, invd, r), s));
 }
+
+namespace {
+template <typename T> void xpay_launch(const Xpay<T> &f, int64_t n, cudaStream_t s) {
+  constexpr int W = kW<T>;
+  if (aligned16(f.p, f.z)) launch_dependent(xpay_k<W, T>, grid_for((n + W - 1) / W), kBlock, 0, s, f, n);
+  else launch_dependent(xpay_k<1, T>, grid_for(n), kBlock, 0, s, f, n);
+}
+} // namespace
 
 void xpay(void *p, const void *z, double beta, int dtype, int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
-  DISPATCH(dtype, xpay_k<T><<<grid_for(n), kBlock, 0, s>>>(static_cast<T *>(p), static_cast<const T *>(z), (T)beta, n));
-  PMG_LAUNCH_CHECK();
+  DISPATCH(dtype, xpay_launch<T>(Xpay<T>{io<T>(p), in<T>(z), (T)beta, nullptr, nullptr}, n, s));
 }
 
 void axpy(void *y, const void *x, double alpha, int dtype, int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
-  DISPATCH(dtype, axpy_k<T><<<grid_for(n), kBlock, 0, s>>>(static_cast<T *>(y), static_cast<const T *>(x), (T)alpha, n));
-  PMG_LAUNCH_CHECK();
+  DISPATCH(dtype, map<kW<T>>(Axpy<T>{io<T>(y), in<T>(x), (T)alpha}, n, aligned16(y, x), s));
 }
 
 double dot(const void *a, const void *b, int dtype, int64_t n, cudaStream_t s) {
-  prof::Scope scope_("vector_reduce", s);
-  Workspace &w = workspace();
-  const int grid = reduce_grid(n);
-  DISPATCH(dtype, dot_partial_k<T><<<grid, kBlock, 0, s>>>(static_cast<const T *>(a), static_cast<const T *>(b), n,
-                                                            w.partials.as<double>()));
-  PMG_LAUNCH_CHECK();
-  return finish(w, grid, 0, s);
+  Scalars v(s);
+  v.dot(0, a, b, dtype, n);
+  v.sync();
+  return v[0];
 }
 
-double cg_update(void *x, void *r, const void *p, const void *v, double alpha, int dtype, int64_t n,
-                 cudaStream_t s) {
-  prof::Scope scope_("vector_reduce", s);
-  Workspace &w = workspace();
-  const int grid = reduce_grid(n);
-  DISPATCH(dtype, cg_update_k<T><<<grid, kBlock, 0, s>>>(static_cast<T *>(x), static_cast<T *>(r),
-                                                          static_cast<const T *>(p), static_cast<const T *>(v),
-                                                          (T)alpha, n, w.partials.as<double>()));
-  PMG_LAUNCH_CHECK();
-  return finish(w, grid, 1, s);
+void Scalars::dot(int slot, const void *a, const void *b, int dtype, int64_t n) {
+  prof::Scope scope_("vector_reduce", s_);
+  DISPATCH(dtype, reduce<kW<T>>(Dot<T>{in<T>(a), in<T>(b), 0.0}, n, aligned16(a, b), w_->sum(slot), s_));
 }
 
-double residual_dot(void *r, const void *b, const void *Ax, int dtype, int64_t n, cudaStream_t s) {
-  prof::Scope scope_("vector_reduce", s);
-  Workspace &w = workspace();
-  const int grid = reduce_grid(n);
-  DISPATCH(dtype, residual_dot_k<T><<<grid, kBlock, 0, s>>>(static_cast<T *>(r), static_cast<const T *>(b),
-                                                             static_cast<const T *>(Ax), n, w.partials.as<double>()));
-  PMG_LAUNCH_CHECK();
-  return finish(w, grid, 3, s);
+void Scalars::cg_update(int slot, void *x, void *r, const void *p, const void *v, int rho, int pv, int dtype, int64_t n) {
+  prof::Scope scope_("vector_reduce", s_);
+  DISPATCH(dtype, reduce<kW<T>>(CgUpdate<T>{io<T>(x), io<T>(r), in<T>(p), in<T>(v), w_->value(rho), w_->value(pv), 0.0, T(0),
+                                            false}, n, aligned16(x, r, p, v), w_->sum(slot), s_));
 }
 
-double jacobi_dot(void *z, const void *invd, const void *r, int dtype, int64_t n, cudaStream_t s) {
-  prof::Scope scope_("vector_reduce", s);
-  Workspace &w = workspace();
-  const int grid = reduce_grid(n);
-  DISPATCH(dtype, jacobi_dot_k<T><<<grid, kBlock, 0, s>>>(static_cast<T *>(z), static_cast<const T *>(invd),
-                                                           static_cast<const T *>(r), n, w.partials.as<double>()));
-  PMG_LAUNCH_CHECK();
-  return finish(w, grid, 2, s);
+void Scalars::residual_dot(int slot, void *r, const void *b, const void *Ax, int dtype, int64_t n) {
+  prof::Scope scope_("vector_reduce", s_);
+  DISPATCH(dtype, reduce<kW<T>>(ResidualDot<T>{io<T>(r), in<T>(b), in<T>(Ax), 0.0}, n, aligned16(r, b, Ax), w_->sum(slot), s_));
+}
+
+void Scalars::jacobi_dot(int slot, void *z, const void *invd, const void *r, int dtype, int64_t n) {
+  prof::Scope scope_("vector_reduce", s_);
+  DISPATCH(dtype, reduce<kW<T>>(JacobiDot<T>{io<T>(z), in<T>(invd), in<T>(r), 0.0}, n, aligned16(z, invd, r), w_->sum(slot), s_));
+}
+
+void Scalars::xpay(void *p, const void *z, int rho, int rho_old, int dtype, int64_t n) {
+  prof::Scope scope_("vector_update", s_);
+  DISPATCH(dtype, xpay_launch<T>(Xpay<T>{io<T>(p), in<T>(z), T(0), w_->value(rho), w_->value(rho_old)}, n, s_));
 }
 
 } // namespace vec

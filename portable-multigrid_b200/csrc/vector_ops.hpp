@@ -5,34 +5,66 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <memory>
 
 namespace pmg {
 namespace vec {
 
 void fill_mod11(void *x, int dtype, int64_t n, cudaStream_t s);
 void convert(void *dst, int dt_dst, const void *src, int dt_src, int64_t n, cudaStream_t s);
+
+// A product A x that an update consumes: the cells' sum, to which the identity rows of the
+// constrained DoFs (bit i of `bits`; null: none) are added as it is read, and which is left zero
+// for the next product (clear) -- so no launch zeroes it.
+struct Product {
+  void *Ax;
+  const uint32_t *bits = nullptr;
+  bool clear = false;
+};
+// dst = 0 with the identity rows dst_i = src_i of the constrained DoFs
+void init_product(void *dst, const void *src, const uint32_t *bits, int dtype, int64_t n, cudaStream_t s);
 // Chebyshev vector steps (x_{k+1} = x_k + f1 (x_k - x_{k-1}) + f2 D^{-1} (b - A x_k)):
-// cheb_init: dst = scale D^{-1} src, xo = 0 unless xo is null; cheb_first_step: xo = dst,
-// dst += scale D^{-1} (src - Ax); cheb_first_step_into: out = x0 + scale D^{-1} (src - Ax);
-// cheb_update_into: out = the update from cur and prev (null: zero), out == prev allowed
-void cheb_init(void *dst, void *xo, const void *src, const void *invd, double scale, int dtype,
-               int64_t n, cudaStream_t s);
-void cheb_first_step(void *dst, void *xo, const void *src, const void *Ax, const void *invd,
+// cheb_init: dst = scale D^{-1} src
+void cheb_init(void *dst, const void *src, const void *invd, double scale, int dtype, int64_t n, cudaStream_t s);
+// cheb_first_step: out = x0 + scale D^{-1} (src - A x0), and keep = x0 unless null (keep != x0;
+// out == x0 allowed)
+void cheb_first_step(void *out, void *keep, const void *x0, const void *src, const Product &p, const void *invd,
                      double scale, int dtype, int64_t n, cudaStream_t s);
-void cheb_first_step_into(void *out, const void *x0, const void *src, const void *Ax, const void *invd,
-                          double scale, int dtype, int64_t n, cudaStream_t s);
-void cheb_update_into(void *out, const void *cur, const void *prev, const void *src, const void *Ax,
-                      const void *invd, double f1, double f2, int dtype, int64_t n, cudaStream_t s);
-void residual(void *t, const void *def, int dtype, int64_t n, cudaStream_t s);
+// cheb_update: out = the update from cur and prev (null: zero), out == prev allowed
+void cheb_update(void *out, const void *cur, const void *prev, const void *src, const Product &p, const void *invd,
+                 double f1, double f2, int dtype, int64_t n, cudaStream_t s);
+// t = def - A x; zero (null: none) [n_zero] is set to zero in the same launch
+void residual(void *t, const void *def, const void *x, const Product &p, void *zero, int64_t n_zero, int dtype,
+              int64_t n, cudaStream_t s);
 void jacobi(void *z, const void *invd, const void *r, int dtype, int64_t n, cudaStream_t s);
 void xpay(void *p, const void *z, double beta, int dtype, int64_t n, cudaStream_t s);
 void axpy(void *y, const void *x, double alpha, int dtype, int64_t n, cudaStream_t s); // y += alpha x
 double dot(const void *a, const void *b, int dtype, int64_t n, cudaStream_t s);
-double cg_update(void *x, void *r, const void *p, const void *v, double alpha, int dtype, int64_t n,
-                 cudaStream_t s);
-double jacobi_dot(void *z, const void *invd, const void *r, int dtype, int64_t n, cudaStream_t s);
-// r = b - Ax; returns r.r
-double residual_dot(void *r, const void *b, const void *Ax, int dtype, int64_t n, cudaStream_t s);
+
+// Reductions whose results stay on the device, where later kernels of the same stream take the CG
+// step lengths from them; the host reads them after sync().  Slots 0 .. kSlots-1.
+struct ScalarSpace;
+class Scalars {
+public:
+  static constexpr int kSlots = 64;
+  explicit Scalars(cudaStream_t s);
+  ~Scalars();
+  Scalars(const Scalars &) = delete;
+  Scalars &operator=(const Scalars &) = delete;
+  void dot(int slot, const void *a, const void *b, int dtype, int64_t n);
+  void jacobi_dot(int slot, void *z, const void *invd, const void *r, int dtype, int64_t n); // z = invd r; r.z
+  void residual_dot(int slot, void *r, const void *b, const void *Ax, int dtype, int64_t n); // r = b - Ax; r.r
+  // alpha = rho / pv: x += alpha p, r -= alpha v; r.r.  Where rho or pv is not finite or pv <= 0, x
+  // and r stay as they are.
+  void cg_update(int slot, void *x, void *r, const void *p, const void *v, int rho, int pv, int dtype, int64_t n);
+  void xpay(void *p, const void *z, int rho, int rho_old, int dtype, int64_t n); // p = z + (rho / rho_old) p
+  void sync();                  // waits for the stream
+  double operator[](int slot) const; // valid after sync()
+
+private:
+  cudaStream_t s_;
+  std::unique_ptr<ScalarSpace> w_;
+};
 
 } // namespace vec
 } // namespace pmg
