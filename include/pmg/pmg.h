@@ -337,8 +337,7 @@ pmg_status pmg_transfer_prolongate_and_add(const pmg_transfer *transfer, void *d
 pmg_status pmg_transfer_restrict_and_add(const pmg_transfer *transfer, void *dst_coarse,
                                          const void *src_fine, void *stream);
 /* Shape of the last launch (inspection, no reference counterpart): *units = patches (the
- * DG <-> CG transfer: entries; the runtime-size kernel: patch batches) and *parallel = the
- * warps (threads; blocks) of the grid that shared them.  Zero before the first launch. */
+ * DG <-> CG transfer: entries) and *parallel = the blocks (threads) of the grid that shared them.  Zero before the first launch. */
 pmg_status pmg_transfer_last_launch(const pmg_transfer *transfer, int64_t *units, int64_t *parallel);
 
 /* ---------------------------------------------------------------------------------- */

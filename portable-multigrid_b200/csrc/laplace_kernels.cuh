@@ -191,15 +191,15 @@ __device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes, uint6
                : "memory");
 }
 
-// read-only loads with an L2 policy, not allocated in L1
+// loads with an L2 policy, not allocated in L1 (index maps through the read-only path)
 __device__ __forceinline__ double ld_stream(const double *p, uint64_t pol) {
   double v;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+  asm("ld.global.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ float ld_stream(const float *p, uint64_t pol) {
   float v;
-  asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+  asm("ld.global.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t *p, uint64_t pol) {
@@ -211,12 +211,12 @@ __device__ __forceinline__ uint32_t ld_stream(const uint32_t *p, uint64_t pol) {
 // towards their first use
 __device__ __forceinline__ double ld_keep_early(const double *p, uint64_t pol) {
   double v;
-  asm volatile("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ float ld_keep_early(const float *p, uint64_t pol) {
   float v;
-  asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ uint32_t ld_keep_early(const uint32_t *p, uint64_t pol) {
@@ -235,12 +235,12 @@ template <int N, typename T> __device__ __forceinline__ T line_weight(const T (&
 // gathered loads that are reused by neighbouring cells
 __device__ __forceinline__ double ld_keep(const double *p, uint64_t pol) {
   double v;
-  asm("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+  asm("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ float ld_keep(const float *p, uint64_t pol) {
   float v;
-  asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+  asm("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
   return v;
 }
 
@@ -400,6 +400,9 @@ __global__ void __launch_bounds__(SMEM_G ? 256 : 128, (SMEM_G ? 1 : (sizeof(T) =
   constexpr int NCOMP = GEOM == 3 ? 10 : 6; // geometry values per quadrature point
   pdl_trigger();
   pdl_wait();
+  src = pdl_after(src);
+  geo = pdl_after(geo);
+  coef = pdl_after(coef);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   if (lane >= LANES) return;

@@ -205,6 +205,9 @@ __global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
   uint32_t id[N];
   line_index<N>(idx, c, r, in, pol_first, id); // (fixed at setup: read before the wait)
   pdl_wait();
+  src = pdl_after(src);
+  geo = pdl_after(geo);
+  coef = pdl_after(coef);
   T cf[GEOM == 2 ? N : 1]; // the coefficient on the x line, requested before the gather
   if constexpr (GEOM == 2) {
     const T *cp = coef + c * N3 + r;
@@ -352,6 +355,7 @@ __global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
   uint32_t id[N];
   line_index<N>(idx, c, at.r, at.active && c < n_cells, pol_first, id); // (fixed at setup: read before the wait)
   pdl_wait();
+  src = pdl_after(src);
   if (at.active) {
     T u[N];
 #pragma unroll

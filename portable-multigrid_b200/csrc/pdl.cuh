@@ -18,6 +18,14 @@ namespace pmg {
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// p as a value that exists only after the wait, for loads the compiler may otherwise move before it
+// (inline PTX, const __restrict__ pointers).  What the chain writes is read with plain loads, not
+// through the non-coherent path: it changes while the waiting kernel is resident.
+template <typename T> __device__ __forceinline__ T *pdl_after(T *p) {
+  asm volatile("" : "+l"(p));
+  return p;
+}
+
 template <typename... P, typename... A>
 void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A &&...args) {
   cudaLaunchConfig_t cfg = {};

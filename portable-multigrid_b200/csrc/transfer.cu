@@ -4,11 +4,12 @@
 // refinement; include/multigrid/portable_geometric_transfer.h).  Both are "patch"
 // transfers: every patch (fine cell for p, coarse cell for h) maps its coarse DoFs
 // (Dirichlet entries dropped) through the tensor product of a 1D matrix onto its fine
-// DoFs, each fine entry scaled by 1/(number of patches holding it), 0 when constrained.
+// DoFs.  On the caller's maps each fine entry is scaled by its weight, 1/(number of patches
+// holding it) by default and 0 when constrained.  On box meshes the patches that hold a fine DoF
+// interpolate the same value there (the coarse function is continuous), so the first of them
+// alone stands for the DoF and the others skip it: no weights, and about half of the fine entries
+// of a patch are neither read nor added to.
 #include <algorithm>
-#include <cstdlib>
-#include <map>
-#include <mutex>
 
 #include "pdl.cuh"
 #include "pmg_internal.hpp"
@@ -17,162 +18,144 @@
 namespace pmg {
 namespace {
 
-template <typename T>
-__global__ void transfer_kernel(int dir, int nc, int nf, int ppb, const T *__restrict__ P,
-                                const T *__restrict__ src, T *__restrict__ dst,
-                                const uint32_t *__restrict__ cidx,
-                                const uint32_t *__restrict__ fidx, const T *__restrict__ w,
-                                int64_t n_patches) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *sP = reinterpret_cast<T *>(smem_raw);
-  const int nf3 = nf * nf * nf, nc3 = nc * nc * nc;
-  T *buf = sP + ((nc * nf + 3) & ~3);
-  for (int i = threadIdx.x; i < nc * nf; i += blockDim.x) sP[i] = P[i];
-  __syncthreads();
-  const int a = dir == 0 ? nc : nf, b = dir == 0 ? nf : nc;
-  const int a3 = a * a * a, b3 = b * b * b;
-  const int bs = blockDim.x;
-#define MAT(i, o) (dir == 0 ? sP[(i) * nf + (o)] : sP[(o) * nf + (i)])
-  for (int64_t base = blockIdx.x * (int64_t)ppb; base < n_patches; base += (int64_t)gridDim.x * ppb) {
-    const int np = (int)min((int64_t)ppb, n_patches - base);
-    for (int t = threadIdx.x; t < np * a3; t += bs) {
-      const int pi = t / a3, l = t - pi * a3;
-      const int64_t patch = base + pi;
-      T *in = buf + pi * 3 * nf3;
-      if (dir == 0) {
-        const uint32_t id = cidx[patch * nc3 + l];
-        in[l] = (id != kInvalid) ? src[id] : T(0);
-      } else {
-        in[l] = w[patch * nf3 + l] * src[fidx[patch * nf3 + l]];
-      }
-    }
-    __syncthreads();
-    // x: t1[k][j][x] = sum_i M(i,x) in[k][j][i]
-    for (int t = threadIdx.x; t < np * a * a * b; t += bs) {
-      const int pi = t / (a * a * b), r = t - pi * (a * a * b);
-      const int x = r % b, kj = r / b;
-      const T *in = buf + pi * 3 * nf3 + kj * a;
-      T s = 0;
-      for (int i = 0; i < a; ++i) s += MAT(i, x) * in[i];
-      buf[pi * 3 * nf3 + nf3 + kj * b + x] = s;
-    }
-    __syncthreads();
-    // y: t2[k][y][x] = sum_j M(j,y) t1[k][j][x]
-    for (int t = threadIdx.x; t < np * a * b * b; t += bs) {
-      const int pi = t / (a * b * b), r = t - pi * (a * b * b);
-      const int x = r % b, y = (r / b) % b, k = r / (b * b);
-      const T *t1 = buf + pi * 3 * nf3 + nf3 + k * a * b;
-      T s = 0;
-      for (int j = 0; j < a; ++j) s += MAT(j, y) * t1[j * b + x];
-      buf[pi * 3 * nf3 + 2 * nf3 + (k * b + y) * b + x] = s;
-    }
-    __syncthreads();
-    // z and scatter
-    for (int t = threadIdx.x; t < np * b3; t += bs) {
-      const int pi = t / b3, l = t - pi * b3;
-      const int yx = l % (b * b), z = l / (b * b);
-      const T *t2 = buf + pi * 3 * nf3 + 2 * nf3 + yx;
-      T s = 0;
-      for (int k = 0; k < a; ++k) s += MAT(k, z) * t2[k * b * b];
-      const int64_t patch = base + pi;
-      if (dir == 0) {
-        atomicAdd(dst + fidx[patch * nf3 + l], w[patch * nf3 + l] * s);
-      } else {
-        const uint32_t id = cidx[patch * nc3 + l];
-        if (id != kInvalid) atomicAdd(dst + id, s);
-      }
-    }
-    __syncthreads();
-  }
-#undef MAT
-}
-
-// Warp-per-patch form of transfer_kernel for NC, NF <= 7 (every p-transfer up to degree 6
-// and the h-transfers up to degree 3): sizes known at compile time, the patch's three
-// tensor sweeps run through per-warp shared-memory buffers with warp barriers only, the 1D
-// matrix sits in shared memory (lanes read different entries).  Same index conventions
-// and results as transfer_kernel.
+// One thread per line of a patch's fine nodes, NF^2 threads per patch; coarse -> fine takes the
+// lines x, y, z, fine -> coarse z, y, x, so that lines along z gather or scatter the fine nodes:
+// neighbouring lanes hold neighbouring fine DoFs.  fidx: the sentinel for an entry that another
+// patch stands for; w: weights, or null.
 template <int NC, int NF, typename T> struct TMat {
   T m[NC * NF]; // m[i_c * NF + j_f]
 };
 
-template <typename T, int NC, int NF, int DIR> struct PatchShape {
-  static constexpr int A = DIR == 0 ? NC : NF, B = DIR == 0 ? NF : NC;
-  static constexpr int A3 = A * A * A, B3 = B * B * B, T1 = A * A * B, T2 = A * B * B;
-  static constexpr int PER_WARP = A3 + T1 + T2; // elements of T
+template <int NC, int NF> struct PatchShape {
+  static constexpr int NF2 = NF * NF;
+  // patches per block: lines of several patches fill its warps (at least 90 % of the lanes but for
+  // the patches of 11^2 and 13^2 lines)
+  static constexpr int PPB = NF == 3 ? 14 : NF == 4 ? 8 : NF == 5 ? 5 : NF == 6 ? 7 : NF == 7 ? 5 : NF == 9 ? 3 : NF == 11 ? 2 : 1;
+  static constexpr int THREADS = (PPB * NF2 + 31) / 32 * 32;
+  static constexpr int ROW = NF | 1;                 // x lines of the first exchange, odd stride
+  static constexpr int A = NC * NC * ROW, B = NC * NF2; // the exchanges between x and y, y and z
+  static constexpr int ELEMS = (A + B) | 1;
 };
 
-constexpr int kPatchWarps = 8;
-
 template <typename T, int NC, int NF, int DIR>
-__global__ void __launch_bounds__(32 * kPatchWarps)
-    transfer_patch_kernel(const __grid_constant__ TMat<NC, NF, T> P, const T *__restrict__ src,
-                          T *__restrict__ dst, const uint32_t *__restrict__ cidx,
-                          const uint32_t *__restrict__ fidx, const T *__restrict__ w, int64_t n_patches) {
-  using Sh = PatchShape<T, NC, NF, DIR>;
-  constexpr int A = Sh::A, B = Sh::B, NC3 = NC * NC * NC, NF3 = NF * NF * NF;
-  __shared__ T sM[NC * NF];
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+__global__ void __launch_bounds__(PatchShape<NC, NF>::THREADS)
+    transfer_line_kernel(const __grid_constant__ TMat<NC, NF, T> P, const T *src, T *dst,
+                         const uint32_t *__restrict__ cidx, const uint32_t *__restrict__ fidx,
+                         const T *__restrict__ w, int64_t n_patches) {
+  using Sh = PatchShape<NC, NF>;
+  constexpr int NF2 = NF * NF, NF3 = NF2 * NF, NC2 = NC * NC, NC3 = NC2 * NC, ROW = Sh::ROW;
   pdl_trigger();
-  for (int i = threadIdx.x; i < NC * NF; i += blockDim.x) sM[i] = P.m[i];
-  __syncthreads();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int e = threadIdx.x / NF2, r = threadIdx.x - e * NF2;
+  T *A = reinterpret_cast<T *>(smem_raw) + e * Sh::ELEMS, *B = A + Sh::A;
+  const int64_t patch = int64_t(blockIdx.x) * Sh::PPB + e;
+  const bool in = e < Sh::PPB && patch < n_patches;
+  // the maps are fixed at setup: read before the wait
+  uint32_t f[NF], c[NC];
+#pragma unroll
+  for (int k = 0; k < NF; ++k) f[k] = in ? __ldg(fidx + patch * NF3 + k * NF2 + r) : kInvalid;
+  const bool xline = in && r < NC2;      // x line (j, k): r = k*NC + j
+  const bool yline = in && r < NC * NF;  // y line (i, k): r = k*NF + i
+  const int yk = r / NF, yi = r - yk * NF;
+#pragma unroll
+  for (int i = 0; i < NC; ++i) c[i] = xline ? __ldg(cidx + patch * NC3 + r * NC + i) : kInvalid;
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  T *in = reinterpret_cast<T *>(smem_raw) + (threadIdx.x >> 5) * Sh::PER_WARP;
-  T *t1 = in + Sh::A3;
-  T *t2 = t1 + Sh::T1;
-  const int64_t warp0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  // M(i, o): input index i, output index o
-  auto M = [&](int i, int o) -> T { return DIR == 0 ? sM[i * NF + o] : sM[o * NF + i]; };
-  for (int64_t patch = warp0; patch < n_patches; patch += nwarps) {
-    for (int l = lane; l < Sh::A3; l += 32) {
-      if (DIR == 0) {
-        const uint32_t id = __ldg(cidx + patch * NC3 + l);
-        in[l] = (id != kInvalid) ? src[id] : T(0);
-      } else {
-        in[l] = __ldg(w + patch * NF3 + l) * src[__ldg(fidx + patch * NF3 + l)];
+  src = pdl_after(src);
+  if (DIR == 0) {
+    if (xline) {
+      T u[NC];
+#pragma unroll
+      for (int i = 0; i < NC; ++i) u[i] = c[i] != kInvalid ? src[c[i]] : T(0);
+#pragma unroll
+      for (int x = 0; x < NF; ++x) {
+        T v = T(0);
+#pragma unroll
+        for (int i = 0; i < NC; ++i) v = fma(P.m[i * NF + x], u[i], v);
+        A[r * ROW + x] = v;
       }
     }
-    __syncwarp();
-    for (int t = lane; t < Sh::T1; t += 32) { // t1[k][j][x] = sum_i M(i, x) in[k][j][i]
-      const int x = t % B, kj = t / B;
-      T s = T(0);
+    __syncthreads();
+    if (yline) {
+      T u[NC];
 #pragma unroll
-      for (int i = 0; i < A; ++i) s = fma(M(i, x), in[kj * A + i], s);
-      t1[kj * B + x] = s;
-    }
-    __syncwarp();
-    for (int t = lane; t < Sh::T2; t += 32) { // t2[k][y][x] = sum_j M(j, y) t1[k][j][x]
-      const int x = t % B, y = (t / B) % B, k = t / (B * B);
-      T s = T(0);
+      for (int j = 0; j < NC; ++j) u[j] = A[(yk * NC + j) * ROW + yi];
 #pragma unroll
-      for (int j = 0; j < A; ++j) s = fma(M(j, y), t1[(k * A + j) * B + x], s);
-      t2[(k * B + y) * B + x] = s;
-    }
-    __syncwarp();
-    for (int t = lane; t < Sh::B3; t += 32) { // z sweep and scatter
-      const int yx = t % (B * B), z = t / (B * B);
-      T s = T(0);
+      for (int y = 0; y < NF; ++y) {
+        T v = T(0);
 #pragma unroll
-      for (int k = 0; k < A; ++k) s = fma(M(k, z), t2[k * B * B + yx], s);
-      if (DIR == 0) {
-        atomicAdd(dst + __ldg(fidx + patch * NF3 + t), __ldg(w + patch * NF3 + t) * s);
-      } else {
-        const uint32_t id = __ldg(cidx + patch * NC3 + t);
-        if (id != kInvalid) atomicAdd(dst + id, s);
+        for (int j = 0; j < NC; ++j) v = fma(P.m[j * NF + y], u[j], v);
+        B[yk * NF2 + y * NF + yi] = v;
       }
     }
-    __syncwarp();
+    __syncthreads();
+    if (in) {
+      T u[NC];
+#pragma unroll
+      for (int k = 0; k < NC; ++k) u[k] = B[k * NF2 + r];
+#pragma unroll
+      for (int z = 0; z < NF; ++z) {
+        T v = T(0);
+#pragma unroll
+        for (int k = 0; k < NC; ++k) v = fma(P.m[k * NF + z], u[k], v);
+        if (w) v *= __ldg(w + patch * NF3 + z * NF2 + r);
+        if (f[z] != kInvalid) atomicAdd(dst + f[z], v);
+      }
+    }
+  } else {
+    if (in) {
+      T u[NF];
+#pragma unroll
+      for (int z = 0; z < NF; ++z) u[z] = f[z] != kInvalid ? src[f[z]] : T(0);
+      if (w) {
+#pragma unroll
+        for (int z = 0; z < NF; ++z) u[z] *= __ldg(w + patch * NF3 + z * NF2 + r);
+      }
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        T v = T(0);
+#pragma unroll
+        for (int z = 0; z < NF; ++z) v = fma(P.m[k * NF + z], u[z], v);
+        B[k * NF2 + r] = v;
+      }
+    }
+    __syncthreads();
+    if (yline) {
+      T u[NF];
+#pragma unroll
+      for (int y = 0; y < NF; ++y) u[y] = B[yk * NF2 + y * NF + yi];
+#pragma unroll
+      for (int j = 0; j < NC; ++j) {
+        T v = T(0);
+#pragma unroll
+        for (int y = 0; y < NF; ++y) v = fma(P.m[j * NF + y], u[y], v);
+        A[(yk * NC + j) * ROW + yi] = v;
+      }
+    }
+    __syncthreads();
+    if (xline) {
+      T u[NF];
+#pragma unroll
+      for (int x = 0; x < NF; ++x) u[x] = A[r * ROW + x];
+#pragma unroll
+      for (int i = 0; i < NC; ++i) {
+        T v = T(0);
+#pragma unroll
+        for (int x = 0; x < NF; ++x) v = fma(P.m[i * NF + x], u[x], v);
+        if (c[i] != kInvalid) atomicAdd(dst + c[i], v);
+      }
+    }
   }
 }
 
 // DG <-> CG at equal degree: the 1D matrix is the identity and every fine (DG) entry is
 // listed once, so the transfer is an entry-wise gather / scatter-add.
 template <typename T, int DIR>
-__global__ void transfer_identity_kernel(const T *__restrict__ src, T *__restrict__ dst,
+__global__ void transfer_identity_kernel(const T *src, T *dst,
                                          const uint32_t *__restrict__ cidx, const uint32_t *__restrict__ fidx,
                                          const T *__restrict__ w, int64_t n_entries) {
+  pdl_trigger();
+  pdl_wait();
+  src = pdl_after(src);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n_entries;
        e += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t id = __ldg(cidx + e);
@@ -187,31 +170,17 @@ __global__ void transfer_identity_kernel(const T *__restrict__ src, T *__restric
 
 template <typename T, int NC, int NF, int DIR>
 void patch_launch(const pmg_transfer &t, void *dst, const void *src, cudaStream_t s) {
-  using Sh = PatchShape<T, NC, NF, DIR>;
-  auto k = transfer_patch_kernel<T, NC, NF, DIR>;
-  const size_t smem = size_t(kPatchWarps) * Sh::PER_WARP * sizeof(T);
+  using Sh = PatchShape<NC, NF>;
+  constexpr size_t smem = size_t(Sh::PPB) * Sh::ELEMS * sizeof(T);
+  static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
   TMat<NC, NF, T> P;
   for (int i = 0; i < NC * NF; ++i) P.m[i] = (T)t.P_host[i];
-  static std::mutex mu;
-  static std::map<int, int> per_sm; // device -> resident blocks per SM
-  int blocks = 0;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = per_sm.find(t.device);
-    if (it == per_sm.end()) {
-      PMG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      int nb = 0;
-      PMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 32 * kPatchWarps, smem));
-      it = per_sm.emplace(t.device, std::max(1, nb)).first;
-    }
-    blocks = it->second;
-  }
-  const int64_t want = (t.n_patches + kPatchWarps - 1) / kPatchWarps;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)blocks * t.sms));
+  const int64_t blocks = (t.n_patches + Sh::PPB - 1) / Sh::PPB;
   t.launch_units = t.n_patches;
-  t.launch_par = (int64_t)grid * kPatchWarps;
-  launch_dependent(k, grid, 32 * kPatchWarps, smem, s, P, static_cast<const T *>(src), static_cast<T *>(dst),
-                   t.coarse_idx.as<uint32_t>(), t.fine_idx.as<uint32_t>(), t.weights.as<T>(), t.n_patches);
+  t.launch_par = blocks;
+  launch_dependent(transfer_line_kernel<T, NC, NF, DIR>, (unsigned)blocks, Sh::THREADS, smem, s, P,
+                   static_cast<const T *>(src), static_cast<T *>(dst), t.coarse_idx.as<uint32_t>(),
+                   t.fine_idx.as<uint32_t>(), t.weights.as<T>(), t.n_patches);
 }
 
 // runtime (nc, nf) -> compiled pair; false if the pair has no compiled form
@@ -229,20 +198,12 @@ template <typename T, int DIR> bool patch_dispatch(const pmg_transfer &t, void *
          try_pair<T, DIR, 3, 7>(t, dst, src, s) || try_pair<T, DIR, 4, 5>(t, dst, src, s) ||
          try_pair<T, DIR, 4, 6>(t, dst, src, s) || try_pair<T, DIR, 4, 7>(t, dst, src, s) ||
          try_pair<T, DIR, 5, 6>(t, dst, src, s) || try_pair<T, DIR, 5, 7>(t, dst, src, s) ||
-         try_pair<T, DIR, 6, 7>(t, dst, src, s);
+         try_pair<T, DIR, 6, 7>(t, dst, src, s) || try_pair<T, DIR, 5, 9>(t, dst, src, s) ||
+         try_pair<T, DIR, 6, 11>(t, dst, src, s) || try_pair<T, DIR, 7, 13>(t, dst, src, s);
 }
 
 template <typename T> std::vector<T> cast(const std::vector<double> &v) {
   return std::vector<T>(v.begin(), v.end());
-}
-
-// PMG_TRANSFER_GENERIC=1 keeps every transfer on transfer_kernel (a comparison switch)
-bool patch_kernels_enabled() {
-  static const bool on = [] {
-    const char *e = std::getenv("PMG_TRANSFER_GENERIC");
-    return !(e && e[0] == '1');
-  }();
-  return on;
 }
 
 bool same_box_geometry(const pmg_box &a, const pmg_box &b) {
@@ -293,22 +254,46 @@ __global__ void weights_kernel(const uint32_t *__restrict__ fidx, int64_t n, con
   }
 }
 
+// the first patch that holds each fine DoF (owner: all ones before), and the map without the entries
+// of other patches and of constrained DoFs
+__global__ void first_patch_kernel(const uint32_t *__restrict__ fidx, int64_t n, int nf3, uint32_t *__restrict__ owner) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
+    atomicMin(owner + fidx[e], (uint32_t)(e / nf3));
+}
+__global__ void keep_first_kernel(uint32_t *__restrict__ fidx, int64_t n, int nf3, const uint32_t *__restrict__ owner,
+                                  const uint8_t *__restrict__ cons) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t d = fidx[e];
+    if (cons[d] || owner[d] != (uint32_t)(e / nf3)) fidx[e] = kInvalid;
+  }
+}
+
 int setup_grid(int64_t n, int sms) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sms * 32));
 }
 
-// the 1D matrix, the weights (1 / multiplicity of the fine DoF over all patches, 0 when
-// constrained, unless given), launch parameters; t.coarse_idx and t.fine_idx are set
+// the 1D matrix and, on box meshes (`nested`), the fine map without repeated entries; else the
+// weights (1 / multiplicity of the fine DoF over all patches, 0 when constrained, unless given).
+// t.coarse_idx and t.fine_idx are set
 void transfer_finish(pmg_transfer &t, const pmg_operator &fine, const std::vector<double> &P,
-                     const double *given_weights) {
+                     const double *given_weights, bool nested) {
   int sms = 0;
   PMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, t.device));
   t.sms = sms;
   const int64_t nf3 = (int64_t)t.nf * t.nf * t.nf, n_w = t.n_patches * nf3;
   t.P_host = P;
-  if (t.dtype == PMG_F64) t.P1d = upload(P);
-  else t.P1d = upload(cast<float>(P));
-  if (given_weights) {
+  if (nested) {
+    if (n_w > 0) {
+      DeviceBuffer owner(sizeof(uint32_t) * std::max<int64_t>(1, t.n_fine));
+      PMG_CUDA(cudaMemset(owner.get(), 0xFF, owner.bytes()));
+      first_patch_kernel<<<setup_grid(n_w, sms), 256>>>(t.fine_idx.as<uint32_t>(), n_w, (int)nf3, owner.as<uint32_t>());
+      PMG_LAUNCH_CHECK();
+      keep_first_kernel<<<setup_grid(n_w, sms), 256>>>(t.fine_idx.as<uint32_t>(), n_w, (int)nf3, owner.as<uint32_t>(),
+                                                       fine.dcons.as<uint8_t>());
+      PMG_LAUNCH_CHECK();
+      PMG_CUDA(cudaDeviceSynchronize()); // owner is freed on return
+    }
+  } else if (given_weights) {
     std::vector<double> w(given_weights, given_weights + n_w);
     if (t.dtype == PMG_F64) t.weights = upload(w);
     else t.weights = upload(cast<float>(w));
@@ -329,15 +314,6 @@ void transfer_finish(pmg_transfer &t, const pmg_operator &fine, const std::vecto
       PMG_CUDA(cudaDeviceSynchronize()); // cnt is freed on return
     }
   }
-  const size_t s = dtype_size(t.dtype);
-  t.ppb = (int)std::max<size_t>(1, (32 * 1024) / (3 * nf3 * s));
-  t.smem = s * (((t.nc * t.nf + 3) & ~3) + (size_t)t.ppb * 3 * nf3);
-  t.patch_kernels = patch_kernels_enabled();
-  t.grid = (int)std::max<int64_t>(1, std::min<int64_t>((t.n_patches + t.ppb - 1) / t.ppb, (int64_t)sms * 8));
-  if (t.dtype == PMG_F64)
-    PMG_CUDA(cudaFuncSetAttribute(transfer_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-  else
-    PMG_CUDA(cudaFuncSetAttribute(transfer_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
 }
 
 // coarse map with the sentinel from the coarse operator's device numbering
@@ -404,7 +380,7 @@ void transfer_setup_from_maps(pmg_transfer &t, const pmg_operator &coarse, const
   coarse_map_from(t, coarse, craw.as<uint32_t>(), (int64_t)n_c);
   t.fine_idx = upload(std::vector<uint32_t>(m.fine_indices, m.fine_indices + n_f));
   PMG_CUDA(cudaDeviceSynchronize()); // craw is freed on return
-  transfer_finish(t, fine, P, m.weights);
+  transfer_finish(t, fine, P, m.weights, false);
 }
 
 void transfer_setup(pmg_transfer &t, const pmg_operator &coarse, const pmg_operator &fine) {
@@ -468,7 +444,7 @@ void transfer_setup(pmg_transfer &t, const pmg_operator &coarse, const pmg_opera
       PMG_LAUNCH_CHECK();
     }
   }
-  transfer_finish(t, fine, P, nullptr);
+  transfer_finish(t, fine, P, nullptr, t.kind != 2);
 }
 
 void transfer_apply(const pmg_transfer &t, int dir, void *dst, const void *src, cudaStream_t s) {
@@ -480,47 +456,19 @@ void transfer_apply(const pmg_transfer &t, int dir, void *dst, const void *src, 
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)t.sms * 16));
     t.launch_units = n;
     t.launch_par = (int64_t)grid * 256;
-    if (t.dtype == PMG_F64) {
-      if (dir == 0)
-        transfer_identity_kernel<double, 0><<<grid, 256, 0, s>>>(static_cast<const double *>(src), static_cast<double *>(dst),
-                                                                 t.coarse_idx.as<uint32_t>(), t.fine_idx.as<uint32_t>(),
-                                                                 t.weights.as<double>(), n);
-      else
-        transfer_identity_kernel<double, 1><<<grid, 256, 0, s>>>(static_cast<const double *>(src), static_cast<double *>(dst),
-                                                                 t.coarse_idx.as<uint32_t>(), t.fine_idx.as<uint32_t>(),
-                                                                 t.weights.as<double>(), n);
-    } else {
-      if (dir == 0)
-        transfer_identity_kernel<float, 0><<<grid, 256, 0, s>>>(static_cast<const float *>(src), static_cast<float *>(dst),
-                                                                t.coarse_idx.as<uint32_t>(), t.fine_idx.as<uint32_t>(),
-                                                                t.weights.as<float>(), n);
-      else
-        transfer_identity_kernel<float, 1><<<grid, 256, 0, s>>>(static_cast<const float *>(src), static_cast<float *>(dst),
-                                                                t.coarse_idx.as<uint32_t>(), t.fine_idx.as<uint32_t>(),
-                                                                t.weights.as<float>(), n);
-    }
-    PMG_LAUNCH_CHECK();
+    auto go = [&](auto kernel, auto zero) {
+      using T = decltype(zero);
+      launch_dependent(kernel, grid, 256, 0, s, static_cast<const T *>(src), static_cast<T *>(dst),
+                       t.coarse_idx.as<uint32_t>(), t.fine_idx.as<uint32_t>(), t.weights.as<T>(), n);
+    };
+    if (t.dtype == PMG_F64) dir == 0 ? go(transfer_identity_kernel<double, 0>, 0.0) : go(transfer_identity_kernel<double, 1>, 0.0);
+    else dir == 0 ? go(transfer_identity_kernel<float, 0>, 0.0f) : go(transfer_identity_kernel<float, 1>, 0.0f);
     return;
   }
-  if (t.patch_kernels) {
-    bool done = false;
-    if (t.dtype == PMG_F64) done = dir == 0 ? patch_dispatch<double, 0>(t, dst, src, s) : patch_dispatch<double, 1>(t, dst, src, s);
-    else done = dir == 0 ? patch_dispatch<float, 0>(t, dst, src, s) : patch_dispatch<float, 1>(t, dst, src, s);
-    if (done) return;
-  }
-  t.launch_units = (t.n_patches + t.ppb - 1) / t.ppb;
-  t.launch_par = t.grid;
-  if (t.dtype == PMG_F64)
-    transfer_kernel<double><<<t.grid, 128, t.smem, s>>>(dir, t.nc, t.nf, t.ppb, t.P1d.as<double>(),
-                                                        static_cast<const double *>(src), static_cast<double *>(dst),
-                                                        t.coarse_idx.as<uint32_t>(), t.fine_idx.as<uint32_t>(),
-                                                        t.weights.as<double>(), t.n_patches);
-  else
-    transfer_kernel<float><<<t.grid, 128, t.smem, s>>>(dir, t.nc, t.nf, t.ppb, t.P1d.as<float>(),
-                                                       static_cast<const float *>(src), static_cast<float *>(dst),
-                                                       t.coarse_idx.as<uint32_t>(), t.fine_idx.as<uint32_t>(),
-                                                       t.weights.as<float>(), t.n_patches);
-  PMG_LAUNCH_CHECK();
+  bool done = false;
+  if (t.dtype == PMG_F64) done = dir == 0 ? patch_dispatch<double, 0>(t, dst, src, s) : patch_dispatch<double, 1>(t, dst, src, s);
+  else done = dir == 0 ? patch_dispatch<float, 0>(t, dst, src, s) : patch_dispatch<float, 1>(t, dst, src, s);
+  PMG_REQUIRE(done, "no transfer kernel for these degrees");
 }
 
 } // namespace pmg

@@ -11,13 +11,11 @@ struct pmg_transfer {
   int kind = 0; // 0 polynomial, 1 geometric, 2 DG <-> CG
   int nc = 0, nf = 0;
   int64_t n_patches = 0, n_coarse = 0, n_fine = 0;
-  pmg::DeviceBuffer P1d, coarse_idx, fine_idx, weights;
+  // fine_idx: on box meshes the sentinel on entries that another patch stands for, and no weights
+  pmg::DeviceBuffer coarse_idx, fine_idx, weights;
   std::vector<double> P_host; // the 1D matrix [nc][nf], passed to the kernels by value
-  int ppb = 1, grid = 1;
-  size_t smem = 0;
-  int sms = 0;               // SM count of the device
-  bool patch_kernels = true; // warp-per-patch kernels for the compiled (nc, nf) pairs
-  // last launch (pmg_transfer_last_launch): patches (or entries) and the warps (or threads)
+  int sms = 0; // SM count of the device
+  // last launch (pmg_transfer_last_launch): patches (or entries) and the blocks (or threads)
   // of the grid that shared them
   mutable int64_t launch_units = 0, launch_par = 0;
 };
