@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "dg.hpp"
+#include "dg_line.cuh"
 #include "pmg_internal.hpp"
 
 namespace pmg {
@@ -1151,9 +1152,83 @@ bool fused_launch(const DGHost &h, const void *src, void *dst, int64_t n_cells, 
   }
 }
 
+// cells per block of the line kernel (kern::LineShape): warps of whole cells at N^2 = 4 and 16, else
+// the lines of 7, 5 or 3 cells in 2, 4 or 5 warps
+template <int N> constexpr auto dg_line_shape() {
+  using kern::LineShape;
+  if constexpr (N == 2) return LineShape<32, 8, 4>{};
+  else if constexpr (N == 3) return LineShape<14, 0, 4>{};
+  else if constexpr (N == 4) return LineShape<8, 2, 4>{};
+  else if constexpr (N == 5) return LineShape<5, 0, 4>{};
+  else return LineShape<3, 0, 3>{};
+}
+
+template <int N, typename T>
+void line_launch(const DGHost &h, const void *src, void *dst, int64_t n_cells, cudaStream_t s, int64_t *units,
+                 int64_t *blocks, const DGChebStep *cheb) {
+  using SH = decltype(dg_line_shape<N>());
+  kern::DGLineTab<N, T> tab;
+  kern::fill_even_odd(tab.eM, [&](int i, int q) { return h.M1[i * N + q]; });
+  kern::fill_even_odd(tab.eK, [&](int i, int q) { return h.K1[i * N + q]; });
+  for (int i = 0; i < N; ++i) {
+    tab.dphi0[i] = (T)h.dphi0[i];
+    tab.dphi1[i] = (T)h.dphi1[i];
+  }
+  kern::DGLineGeo g;
+  for (int d = 0; d < 3; ++d) {
+    g.area[d] = h.h[(d + 1) % 3] * h.h[(d + 2) % 3];
+    g.rh[d] = 1.0 / h.h[d];
+    g.area_h[d] = g.area[d] / h.h[d];
+    g.sigma[d] = h.c_pen / h.h[d];
+  }
+  g.dirichlet = h.dirichlet;
+  constexpr size_t smem = kern::dg_line_smem<N, T, SH>();
+  static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
+  constexpr int threads = kern::line_threads<N, SH>(), line = N * (int)sizeof(T);
+  constexpr int wide = line % 16 == 0 ? 16 : (line % 8 == 0 && sizeof(T) == 4 ? 8 : 0); // bytes of the x lines' loads
+  const unsigned grid = (unsigned)((n_cells + SH::CPB - 1) / SH::CPB);
+  const T *sp = static_cast<const T *>(src);
+  T *dp = static_cast<T *>(dst);
+  const int32_t *nb = h.nbr.as<int32_t>();
+  kern::DGLineStep<T> st{};
+  if (cheb)
+    st = kern::DGLineStep<T>{static_cast<const T *>(cheb->prev), static_cast<const T *>(cheb->b),
+                             static_cast<const T *>(cheb->invd), (T)cheb->f1, (T)cheb->f2};
+  auto go = [&](auto kernel) { launch_dependent(kernel, grid, threads, smem, s, tab, g, sp, dp, nb, n_cells, st); };
+  bool done = false;
+  if constexpr (wide > 0) {
+    if (reinterpret_cast<uintptr_t>(src) % wide == 0) {
+      if (cheb) go(kern::dg_line_kernel<N, T, SH, true, true>);
+      else go(kern::dg_line_kernel<N, T, SH, true, false>);
+      done = true;
+    }
+  }
+  if (!done) {
+    if (cheb) go(kern::dg_line_kernel<N, T, SH, false, true>);
+    else go(kern::dg_line_kernel<N, T, SH, false, false>);
+  }
+  if (units) *units = n_cells;
+  if (blocks) *blocks = grid;
+}
+
+// the line kernel, unless a comparison form is asked for (PMG_DG_FACE, PMG_DG_FUSE)
+bool line_form() { return face_form() < 0 && fuse_allowed(); }
+
 template <typename T>
 bool fused_dispatch(int degree, const DGHost &h, const void *src, void *dst, int64_t n_cells, int sms, cudaStream_t s,
                     int64_t *units, int64_t *blocks, const DGChebStep *cheb, bool launch = true) {
+  if (line_form()) {
+    if (!launch) return true;
+    switch (degree) {
+    case 1: line_launch<2, T>(h, src, dst, n_cells, s, units, blocks, cheb); return true;
+    case 2: line_launch<3, T>(h, src, dst, n_cells, s, units, blocks, cheb); return true;
+    case 3: line_launch<4, T>(h, src, dst, n_cells, s, units, blocks, cheb); return true;
+    case 4: line_launch<5, T>(h, src, dst, n_cells, s, units, blocks, cheb); return true;
+    case 5: line_launch<6, T>(h, src, dst, n_cells, s, units, blocks, cheb); return true;
+    case 6: line_launch<7, T>(h, src, dst, n_cells, s, units, blocks, cheb); return true;
+    default: return false;
+    }
+  }
   switch (degree) {
   case 1: return fused_launch<2, T>(h, src, dst, n_cells, sms, s, units, blocks, cheb, launch);
   case 3: return fused_launch<4, T>(h, src, dst, n_cells, sms, s, units, blocks, cheb, launch);
