@@ -243,6 +243,43 @@ __global__ void coef_interp_kernel(const double *__restrict__ src, const int32_t
   }
 }
 
+// The same between two degrees on one mesh (source cell = target cell): a block per cell, the
+// logarithms of the cell's values and the 1D weights once in shared memory.  One thread per target
+// point took the logarithm of every source value anew, 27 times per value for Q4 -> Q2 (660 us at 32^3).
+__global__ void coef_interp_cell_kernel(const double *__restrict__ src, int nqs, const Gauss8 gs,
+                                        const int32_t *__restrict__ cell_xyz, int64_t n_cells, int nqd, const Gauss8 gd,
+                                        int64_t n0, int64_t n1, int64_t n2, const int32_t *__restrict__ src_lut,
+                                        double *__restrict__ dst) {
+  __shared__ double lg[8 * 8 * 8], L[3][8][8]; // [direction][target point][source point]
+  const int nqd3 = nqd * nqd * nqd, nqs3 = nqs * nqs * nqs;
+  const int64_t ns[3] = {n0, n1, n2};
+  for (int64_t c = blockIdx.x; c < n_cells; c += gridDim.x) {
+    // a target point's cell is the target cell itself (Gauss points lie inside it)
+    const int64_t cell = src_lut[(cell_xyz[3 * c + 2] * ns[1] + cell_xyz[3 * c + 1]) * ns[0] + cell_xyz[3 * c]];
+    for (int q = threadIdx.x; q < nqs3; q += blockDim.x) lg[q] = log(src[cell * nqs3 + q]);
+    for (int t = threadIdx.x; t < 3 * nqd * nqs; t += blockDim.x) {
+      const int d = t / (nqd * nqs), q = (t / nqs) % nqd, a = t % nqs;
+      const double X = (double)cell_xyz[3 * c + d] + gd.x[q], xi = X - (double)cell_xyz[3 * c + d];
+      double l = 1.0;
+      for (int b = 0; b < nqs; ++b)
+        if (b != a) l *= (xi - gs.x[b]) / (gs.x[a] - gs.x[b]);
+      L[d][q][a] = l;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < nqd3; q += blockDim.x) {
+      const int q0 = q % nqd, q1 = (q / nqd) % nqd, q2 = q / (nqd * nqd);
+      double acc = 0.0;
+      for (int k = 0; k < nqs; ++k)
+        for (int j = 0; j < nqs; ++j) {
+          const double ljk = L[1][q1][j] * L[2][q2][k];
+          for (int i = 0; i < nqs; ++i) acc += L[0][q0][i] * ljk * lg[(k * nqs + j) * nqs + i];
+        }
+      dst[c * nqd3 + q] = exp(acc);
+    }
+    __syncthreads();
+  }
+}
+
 } // namespace
 
 const Tables1D &cached_tables(int degree) {
@@ -289,6 +326,14 @@ void coefficient_interpolate(const pmg_operator &src, const pmg_operator &dst, d
   const Tables1D &ts = cached_tables(src.degree), &td = cached_tables(dst.degree);
   for (int q = 0; q < src.nq; ++q) gs.x[q] = ts.xg[q];
   for (int q = 0; q < dst.nq; ++q) gd.x[q] = td.xg[q];
+  if (ratio == 1) {
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(dst.n_cells, (int64_t)dst.sms * 16));
+    coef_interp_cell_kernel<<<grid, 128, 0, s>>>(src.coef_qp.as<double>(), src.nq, gs, dst.cell_xyz.as<int32_t>(),
+                                                 dst.n_cells, dst.nq, gd, src.mesh.n[0], src.mesh.n[1], src.mesh.n[2],
+                                                 src.cell_lut.as<int32_t>(), dst_values);
+    PMG_LAUNCH_CHECK();
+    return;
+  }
   const int64_t n = dst.n_cells * dst.nq * dst.nq * dst.nq;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)dst.sms * 32));
   coef_interp_kernel<<<grid, 256, 0, s>>>(src.coef_qp.as<double>(), src.cell_lut.as<int32_t>(), src.mesh.n[0],
