@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <vector>
 
+#include "mg_tail.hpp"
 #include "pmg_internal.hpp"
 #include "solver.hpp"
 #include "transfer.hpp"
@@ -230,9 +231,15 @@ void mg_setup(pmg_mg &mg, int n_levels, pmg_operator *const *levels, pmg_transfe
     mg.def[l].allocate(bytes);
     mg.t[l].allocate(bytes);
   }
+  mg.tail = mg_tail_plan(mg);
 }
 
-void mg_vcycle(pmg_mg &mg, int l, cudaStream_t s) {
+// the cycle from level l down; levels 0 .. tail (-1: none) run in one kernel
+void mg_vcycle(pmg_mg &mg, int l, int tail, cudaStream_t s) {
+  if (l <= tail) {
+    mg_tail(mg, l, s);
+    return;
+  }
   pmg_operator &op = *mg.levels[l];
   const int dt = op.dtype;
   const int64_t N = op.n_dofs;
@@ -246,7 +253,7 @@ void mg_vcycle(pmg_mg &mg, int l, cudaStream_t s) {
   const vec::Product Ax = operator_product(op, mg.smoothers[l]->Ax.get(), mg.sol[l].get(), s);
   vec::residual(mg.t[l].get(), mg.def[l].get(), mg.sol[l].get(), Ax, mg.def[l - 1].get(), opc.n_dofs, dt, N, s);
   transfer_apply(*mg.transfers[l], 1, mg.def[l - 1].get(), mg.t[l].get(), s);
-  mg_vcycle(mg, l - 1, s);
+  mg_vcycle(mg, l - 1, tail, s);
   transfer_apply(*mg.transfers[l], 0, mg.sol[l].get(), mg.sol[l - 1].get(), s);
   chebyshev_apply(*mg.smoothers[l], mg.sol[l].get(), mg.def[l].get(), false, s);
 }
@@ -277,7 +284,7 @@ void mg_capture(pmg_mg &mg) {
   bool ok = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
   if (ok) {
     try {
-      mg_vcycle(mg, (int)mg.levels.size() - 1, cs);
+      mg_vcycle(mg, (int)mg.levels.size() - 1, mg_tail_top(mg), cs);
     } catch (const Error &) {
       ok = false;
     }
@@ -316,7 +323,7 @@ void mg_vmult(pmg_mg &mg, void *dst, const void *src, int vec_dtype, cudaStream_
   vec::convert(mg.def[L].get(), top.dtype, src, vec_dtype, top.n_dofs, s);
   if (mg.graph_enabled && graphs_allowed() && !prof::enabled() && !mg.graph) mg_capture(mg);
   if (mg.graph && !prof::enabled()) PMG_CUDA(cudaGraphLaunch(mg.graph, s));
-  else mg_vcycle(mg, L, s);
+  else mg_vcycle(mg, L, mg_tail_top(mg), s);
   vec::convert(dst, vec_dtype, mg.sol[L].get(), top.dtype, top.n_dofs, s);
 }
 

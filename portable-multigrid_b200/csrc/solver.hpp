@@ -3,6 +3,7 @@
 
 #include <vector>
 
+#include "mg_tail.hpp"
 #include "pmg_internal.hpp"
 
 struct pmg_chebyshev {
@@ -26,6 +27,7 @@ struct pmg_mg {
   std::vector<pmg_transfer *> transfers;
   std::vector<pmg_chebyshev *> smoothers;
   std::vector<pmg::DeviceBuffer> sol, def, t;
+  std::shared_ptr<pmg::TailPlan> tail; // the coarse levels that run in one kernel, null: none
   // The V-cycle below the finest level's input and output buffers is a fixed sequence of
   // launches on fixed buffers: it is captured once into a CUDA graph and replayed.
   cudaGraphExec_t graph = nullptr;
