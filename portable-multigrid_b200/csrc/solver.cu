@@ -86,12 +86,12 @@ void chebyshev_estimate(pmg_chebyshev &c, cudaStream_t s) {
   // coefficients) keeps them, so repeated estimates allocate nothing
   std::vector<DeviceBuffer> tmp;
   std::vector<DeviceBuffer> &w = c.generation > 0 ? c.est_work : tmp;
-  if (w.size() != 5 || w[0].bytes() != bytes) {
+  if (w.size() != 4 || w[0].bytes() != bytes) {
     w.clear();
-    for (int i = 0; i < 5; ++i) w.emplace_back(bytes);
+    for (int i = 0; i < 4; ++i) w.emplace_back(bytes);
   }
-  DeviceBuffer &x = w[0], &r = w[1], &z = w[2], &p = w[3], &v = w[4];
-  PMG_CUDA(cudaMemsetAsync(x.get(), 0, bytes, s));
+  DeviceBuffer &r = w[0], &z = w[1], &p = w[2], &v = w[3];
+  PMG_CUDA(cudaMemsetAsync(v.get(), 0, bytes, s)); // consumed and cleared by every update
   vec::fill_mod11(r.get(), dt, N, s);
   std::vector<double> diag, offd;
   // The step lengths stay on the device and the host looks at the scalars once every kChunk
@@ -110,12 +110,11 @@ void chebyshev_estimate(pmg_chebyshev &c, cudaStream_t s) {
       const int chunk = std::min(kChunk, c.eig_its - it);
       for (int k = 0; k < chunk; ++k) {
         const int at = it + k + 1; // iteration
-        if (at > 1) sc.xpay(p.get(), z.get(), rho_slot(at - 1), rho_slot(at - 2), dt, N);
-        else PMG_CUDA(cudaMemcpyAsync(p.get(), z.get(), bytes, cudaMemcpyDeviceToDevice, s));
-        operator_vmult(op, v.get(), p.get(), s);
-        sc.dot(kPv + k, p.get(), v.get(), dt, N);
-        sc.cg_update(kRes + k, x.get(), r.get(), p.get(), v.get(), rho_slot(at - 1), kPv + k, dt, N);
-        sc.jacobi_dot(rho_slot(at), z.get(), op.inv_diag.get(), r.get(), dt, N);
+        sc.xpay(p.get(), dt, z.get(), dt, rho_slot(at - 1), at > 1 ? rho_slot(at - 2) : -1, N);
+        const vec::Product Ap = operator_product(op, v.get(), p.get(), s);
+        sc.dot_product(kPv + k, p.get(), Ap, dt, N);
+        sc.cg_update_jacobi(kRes + k, rho_slot(at), r.get(), z.get(), op.inv_diag.get(), p.get(), Ap, rho_slot(at - 1),
+                            kPv + k, dt, N);
       }
       sc.sync();
       if (it == 0 && std::sqrt(sc[kRes0]) <= 1e-10) break;
@@ -302,11 +301,9 @@ void mg_capture(pmg_mg &mg) {
   }
 }
 
-} // namespace
-
-void mg_vmult(pmg_mg &mg, void *dst, const void *src, int vec_dtype, cudaStream_t s) {
+// the V-cycle from mg.def into mg.sol on the finest level
+void mg_cycle(pmg_mg &mg, cudaStream_t s) {
   const int L = (int)mg.levels.size() - 1;
-  const pmg_operator &top = *mg.levels[L];
   for (auto *sm : mg.smoothers)
     if (!sm->estimated) chebyshev_estimate(*sm, s);
   // a graph captured before a smoother was re-estimated holds the old Chebyshev coefficients
@@ -320,10 +317,17 @@ void mg_vmult(pmg_mg &mg, void *dst, const void *src, int vec_dtype, cudaStream_
       mg.graph = nullptr;
     }
   }
-  vec::convert(mg.def[L].get(), top.dtype, src, vec_dtype, top.n_dofs, s);
   if (mg.graph_enabled && graphs_allowed() && !prof::enabled() && !mg.graph) mg_capture(mg);
   if (mg.graph && !prof::enabled()) PMG_CUDA(cudaGraphLaunch(mg.graph, s));
   else mg_vcycle(mg, L, mg_tail_top(mg), s);
+}
+} // namespace
+
+void mg_vmult(pmg_mg &mg, void *dst, const void *src, int vec_dtype, cudaStream_t s) {
+  const int L = (int)mg.levels.size() - 1;
+  const pmg_operator &top = *mg.levels[L];
+  vec::convert(mg.def[L].get(), top.dtype, src, vec_dtype, top.n_dofs, s);
+  mg_cycle(mg, s);
   vec::convert(dst, vec_dtype, mg.sol[L].get(), top.dtype, top.n_dofs, s);
 }
 
@@ -344,13 +348,16 @@ void cg_solve(pmg_operator &A, pmg_mg *mg, void *x, const void *b, double reduce
     A.cg_work.clear();
     for (int i = 0; i < 4; ++i) A.cg_work.emplace_back(bytes);
   }
-  DeviceBuffer &r = A.cg_work[0], &z = A.cg_work[1], &p = A.cg_work[2], &v = A.cg_work[3];
+  DeviceBuffer &r = A.cg_work[0], &p = A.cg_work[1], &v = A.cg_work[2], &z = A.cg_work[3]; // z: Jacobi only
   // r = b - A x and ||r|| in one pass; the step lengths stay on the device, and the host waits once
   // per iteration, for the residual norm (with the scalars it checks)
   enum { kRho = 0, kPv = 2, kRes = 3 }; // kRho, kRho + 1 in turn
   vec::Scalars sc(s);
-  operator_vmult(A, v.get(), x, s);
-  sc.residual_dot(kRes, r.get(), b, v.get(), dt, N);
+  // the residual goes to the V-cycle, and its result to the search direction, as they are produced
+  void *def = mg ? mg->def.back().get() : nullptr;
+  const int mdt = mg ? mg->levels.back()->dtype : dt;
+  PMG_CUDA(cudaMemsetAsync(v.get(), 0, bytes, s)); // consumed and cleared by every update
+  sc.residual_dot(kRes, r.get(), b, x, operator_product(A, v.get(), x, s), def, mdt, dt, N);
   sc.sync();
   double res = std::sqrt(sc[kRes]);
   check_finite(res, "CG residual");
@@ -360,18 +367,19 @@ void cg_solve(pmg_operator &A, pmg_mg *mg, void *x, const void *b, double reduce
   int it = 0;
   while (res > tol && it < max_it) {
     const int rho = kRho + (it & 1), rho_old = kRho + ((it + 1) & 1);
+    const void *dir = z.get();
     if (mg) {
-      mg_vmult(*mg, z.get(), r.get(), dt, s);
-      sc.dot(rho, r.get(), z.get(), dt, N);
+      mg_cycle(*mg, s);
+      dir = mg->sol.back().get();
+      sc.dot_converted(rho, r.get(), dt, dir, mdt, N);
     } else {
       sc.jacobi_dot(rho, z.get(), A.inv_diag.get(), r.get(), dt, N);
     }
-    if (it == 0) PMG_CUDA(cudaMemcpyAsync(p.get(), z.get(), bytes, cudaMemcpyDeviceToDevice, s));
-    else sc.xpay(p.get(), z.get(), rho, rho_old, dt, N);
+    sc.xpay(p.get(), dt, dir, mdt, rho, it > 0 ? rho_old : -1, N);
     ++it;
-    operator_vmult(A, v.get(), p.get(), s);
-    sc.dot(kPv, p.get(), v.get(), dt, N);
-    sc.cg_update(kRes, x, r.get(), p.get(), v.get(), rho, kPv, dt, N);
+    const vec::Product Ap = operator_product(A, v.get(), p.get(), s);
+    sc.dot_product(kPv, p.get(), Ap, dt, N);
+    sc.cg_update(kRes, x, r.get(), p.get(), Ap, rho, kPv, def, mdt, dt, N);
     sc.sync();
     check_finite(sc[rho], "CG preconditioned residual");
     check_finite(sc[kPv], "CG curvature");

@@ -246,7 +246,6 @@ template <typename T> struct Xpay {
   T *p;
   const T *z;
   T beta;
-  const double *rho, *rho_old; // beta = rho / rho_old where given
   template <int W> __device__ void run(int64_t i) {
     const auto a = load<W>(z + i), b = load<W>(p + i);
     Pack<T, W> v;
@@ -255,10 +254,30 @@ template <typename T> struct Xpay {
     store<W>(p + i, v);
   }
 };
-template <int W, typename T> __global__ void __launch_bounds__(kBlock) xpay_k(Xpay<T> f, int64_t n) {
+// p = z + (rho / rho_old) p with the scalars from device memory; rho_old null: p = z
+template <typename T, typename TZ> struct CgDirection {
+  T *p;
+  const TZ *z;
+  const double *rho, *rho_old;
+  T beta;
+  template <int W> __device__ void run(int64_t i) {
+    const auto a = load<W>(z + i);
+    Pack<T, W> v;
+    if (rho_old) {
+      v = load<W>(p + i);
+#pragma unroll
+      for (int k = 0; k < W; ++k) v.v[k] = (T)a.v[k] + beta * v.v[k];
+    } else {
+#pragma unroll
+      for (int k = 0; k < W; ++k) v.v[k] = (T)a.v[k];
+    }
+    store<W>(p + i, v);
+  }
+};
+template <int W, typename F> __global__ void __launch_bounds__(kBlock) cg_direction_k(F f, int64_t n) {
   pdl_trigger();
   pdl_wait();
-  if (f.rho) f.beta = (T)(*f.rho / *f.rho_old);
+  if (f.rho_old) f.beta = static_cast<decltype(f.beta)>(*f.rho / *f.rho_old);
   for_packs<W>(n, f);
 }
 template <typename T> struct Axpy {
@@ -274,12 +293,12 @@ template <typename T> struct Axpy {
   }
 };
 
-// ---- reductions: every block stores a partial sum and the last block to arrive adds the
-// partials in a fixed order (deterministic), into device memory and into host-visible memory ----
+// ---- reductions: every block stores its partial sums (NS of them) and the last block to arrive adds
+// the partials in a fixed order (deterministic), into device memory and into host-visible memory ----
 struct Sum {
-  double *partials;
-  unsigned int *arrived; // 0 between kernels
-  double *device, *host; // the result's places
+  double *partials;       // [NS][kMaxPartials]
+  unsigned int *arrived;  // 0 between kernels
+  double *device[2], *host[2]; // the results' places
 };
 
 __device__ __forceinline__ double block_sum(double v) { // valid in thread 0
@@ -292,23 +311,29 @@ __device__ __forceinline__ double block_sum(double v) { // valid in thread 0
   for (int o = kBlock / 64; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
 }
-__device__ __forceinline__ void finish_sum(double v, const Sum &sum) {
+template <int NS> __device__ __forceinline__ void finish_sum(const double (&acc)[NS], const Sum &sum) {
   __shared__ bool last;
-  v = block_sum(v);
+#pragma unroll
+  for (int k = 0; k < NS; ++k) {
+    const double v = block_sum(acc[k]);
+    if (threadIdx.x == 0) __stcg(sum.partials + k * kMaxPartials + blockIdx.x, v);
+  }
   if (threadIdx.x == 0) {
-    __stcg(sum.partials + blockIdx.x, v);
     __threadfence();
     last = atomicInc(sum.arrived, gridDim.x - 1) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  double w = 0.0;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += kBlock) w += __ldcg(sum.partials + i);
-  w = block_sum(w);
-  if (threadIdx.x == 0) {
-    *sum.device = w;
-    *sum.host = w;
+#pragma unroll
+  for (int k = 0; k < NS; ++k) {
+    double w = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += kBlock) w += __ldcg(sum.partials + k * kMaxPartials + i);
+    w = block_sum(w);
+    if (threadIdx.x == 0) {
+      *sum.device[k] = w;
+      *sum.host[k] = w;
+    }
   }
 }
 template <int W, typename F> __global__ void __launch_bounds__(kBlock) reduce_k(F f, int64_t n, Sum sum) {
@@ -323,32 +348,70 @@ template <int W, typename F> void reduce(const F &f, int64_t n, bool wide, const
   else launch_dependent(reduce_k<1, F>, reduce_grid(n), kBlock, 0, s, f, n, sum);
 }
 
-template <typename T> struct Dot {
-  const T *a, *b;
-  double acc;
+template <typename T, typename TB> struct Dot {
+  const T *a;
+  const TB *b;
+  double acc[1];
   __device__ void begin() {}
   template <int W> __device__ void run(int64_t i) {
-    const auto x = load<W>(a + i), y = load<W>(b + i);
+    const auto x = load<W>(a + i);
+    const auto y = load<W>(b + i);
 #pragma unroll
-    for (int k = 0; k < W; ++k) acc += (double)x.v[k] * (double)y.v[k];
+    for (int k = 0; k < W; ++k) acc[0] += (double)x.v[k] * (double)(T)y.v[k];
   }
 };
-template <typename T> struct CgUpdate {
+template <typename T> struct DotProduct {
+  const T *p;
+  Consumed<T> Ap;
+  double acc[1];
+  __device__ void begin() {}
+  template <int W> __device__ void run(int64_t i) {
+    const auto x = load<W>(p + i), y = Ap.template take<W>(i, x);
+#pragma unroll
+    for (int k = 0; k < W; ++k) acc[0] += (double)x.v[k] * (double)y.v[k];
+  }
+};
+// a copy of a vector in another type, written beside it
+template <typename T, typename TC> struct Copy {
+  TC *to; // null: none
+  template <int W> __device__ void put(int64_t i, const Pack<T, W> &v) const {
+    if (!to) return;
+    Pack<TC, W> c;
+#pragma unroll
+    for (int k = 0; k < W; ++k) c.v[k] = (TC)v.v[k];
+    store<W>(to + i, c);
+  }
+};
+__device__ __forceinline__ bool cg_step(const double *rho, const double *pv, double &alpha) {
+  const double a = *rho, b = *pv;
+  alpha = a / b;
+  return isfinite(a) && isfinite(b) && b > 0.0;
+}
+// The updates of a CG iteration read the operator's product before its identity rows are set and leave
+// it zero, write the residual in the V-cycle's type too and read its result in that type: with a V-cycle
+// three launches less per iteration (two conversions and the product's first pass), 15 instead of 18
+// vectors moved.  Solves with a V-cycle: 16^3 cells of degree 2, FP64, 952 -> 855 us; 48^3 of degree 6,
+// FP64 CG on FP32 levels, 30.4 -> 30.0 ms.  Eigenvalue estimates (CgUpdateJacobi: no iterate, the two sums
+// in one pass; four launches per iteration instead of six) of the eight levels below 32^3 cells of degree
+// 4: 2.3 -> 1.8 ms.
+template <typename T, typename TC> struct CgUpdate {
   T *x, *r;
-  const T *p, *v;
+  const T *p;
+  Consumed<T> Ap;
+  Copy<T, TC> copy;
   const double *rho, *pv;
-  double acc;
+  double acc[1];
   T alpha;
   bool step;
   __device__ void begin() {
-    const double a = *rho, b = *pv;
-    step = isfinite(a) && isfinite(b) && b > 0.0;
-    alpha = (T)(a / b);
+    double a;
+    step = cg_step(rho, pv, a);
+    alpha = (T)a;
   }
   template <int W> __device__ void run(int64_t i) {
     Pack<T, W> rv = load<W>(r + i);
+    const auto pp = load<W>(p + i), vv = Ap.template take<W>(i, pp);
     if (step) {
-      const auto pp = load<W>(p + i), vv = load<W>(v + i);
       auto xv = load<W>(x + i);
 #pragma unroll
       for (int k = 0; k < W; ++k) {
@@ -358,32 +421,66 @@ template <typename T> struct CgUpdate {
       store<W>(x + i, xv);
       store<W>(r + i, rv);
     }
+    copy.template put<W>(i, rv);
 #pragma unroll
-    for (int k = 0; k < W; ++k) acc += (double)rv.v[k] * (double)rv.v[k];
+    for (int k = 0; k < W; ++k) acc[0] += (double)rv.v[k] * (double)rv.v[k];
+    Ap.template done<W>(i);
   }
 };
-// r = b - Ax and r.r
-template <typename T> struct ResidualDot {
+template <typename T> struct CgUpdateJacobi {
+  T *r, *z;
+  const T *invd, *p;
+  Consumed<T> Ap;
+  const double *rho, *pv;
+  double acc[2]; // r.r, r.z
+  T alpha;
+  bool step;
+  __device__ void begin() {
+    double a;
+    step = cg_step(rho, pv, a);
+    alpha = (T)a;
+  }
+  template <int W> __device__ void run(int64_t i) {
+    Pack<T, W> rv = load<W>(r + i), zv;
+    const auto pp = load<W>(p + i), vv = Ap.template take<W>(i, pp), di = load<W>(invd + i);
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      if (step) rv.v[k] = rv.v[k] - alpha * vv.v[k];
+      zv.v[k] = di.v[k] * rv.v[k];
+      acc[0] += (double)rv.v[k] * (double)rv.v[k];
+      acc[1] += (double)rv.v[k] * (double)zv.v[k];
+    }
+    store<W>(r + i, rv);
+    store<W>(z + i, zv);
+    Ap.template done<W>(i);
+  }
+};
+// r = b - A x and r.r
+template <typename T, typename TC> struct ResidualDot {
   T *r;
-  const T *b, *Ax;
-  double acc;
+  const T *b, *x;
+  Consumed<T> Ax;
+  Copy<T, TC> copy;
+  double acc[1];
   __device__ void begin() {}
   template <int W> __device__ void run(int64_t i) {
-    const auto x = load<W>(b + i), y = load<W>(Ax + i);
+    const auto xv = load<W>(x + i), bv = load<W>(b + i), a = Ax.template take<W>(i, xv);
     Pack<T, W> v;
 #pragma unroll
     for (int k = 0; k < W; ++k) {
-      v.v[k] = x.v[k] - y.v[k];
-      acc += (double)v.v[k] * (double)v.v[k];
+      v.v[k] = bv.v[k] - a.v[k];
+      acc[0] += (double)v.v[k] * (double)v.v[k];
     }
     store<W>(r + i, v);
+    copy.template put<W>(i, v);
+    Ax.template done<W>(i);
   }
 };
 // z = invd * r and r.z
 template <typename T> struct JacobiDot {
   T *z;
   const T *invd, *r;
-  double acc;
+  double acc[1];
   __device__ void begin() {}
   template <int W> __device__ void run(int64_t i) {
     const auto d = load<W>(invd + i), a = load<W>(r + i);
@@ -391,7 +488,7 @@ template <typename T> struct JacobiDot {
 #pragma unroll
     for (int k = 0; k < W; ++k) {
       v.v[k] = d.v[k] * a.v[k];
-      acc += (double)a.v[k] * (double)v.v[k];
+      acc[0] += (double)a.v[k] * (double)v.v[k];
     }
     store<W>(z + i, v);
   }
@@ -403,17 +500,17 @@ template <typename T> struct JacobiDot {
 // uses (at most kPool idle ones), so that concurrent users have memory of their own
 struct ScalarSpace {
   int device = 0;
-  DeviceBuffer partials; // kMaxPartials partial sums, kSlots results, the arrival counter
+  DeviceBuffer partials; // 2 kMaxPartials partial sums, kSlots results, the arrival counter
   double *host = nullptr;
   ScalarSpace() = default;
   ~ScalarSpace() {
     if (host) cudaFreeHost(host);
   }
-  Sum sum(int slot) {
-    double *p = partials.as<double>();
-    return Sum{p, reinterpret_cast<unsigned int *>(p + kMaxPartials + Scalars::kSlots), p + kMaxPartials + slot, host + slot};
+  Sum sum(int slot, int second = 0) {
+    double *p = partials.as<double>(), *v = p + 2 * kMaxPartials;
+    return Sum{p, reinterpret_cast<unsigned int *>(v + Scalars::kSlots), {v + slot, v + second}, {host + slot, host + second}};
   }
-  const double *value(int slot) { return partials.as<double>() + kMaxPartials + slot; }
+  const double *value(int slot) { return partials.as<double>() + 2 * kMaxPartials + slot; }
 };
 namespace {
 constexpr size_t kPool = 4;
@@ -443,7 +540,7 @@ Scalars::Scalars(cudaStream_t s) : s_(s) {
   }
   w_ = std::make_unique<ScalarSpace>();
   w_->device = dev;
-  w_->partials.allocate(sizeof(double) * (kMaxPartials + kSlots + 1));
+  w_->partials.allocate(sizeof(double) * (2 * kMaxPartials + kSlots + 1));
   PMG_CUDA(cudaMemset(w_->partials.get(), 0, w_->partials.bytes()));
   PMG_CUDA(cudaDeviceSynchronize());
   PMG_CUDA(cudaMallocHost(&w_->host, sizeof(double) * kSlots));
@@ -549,17 +646,9 @@ void jacobi(void *z, const void *invd, const void *r, int dtype, int64_t n, cuda
   DISPATCH(dtype, map<kW<T>>(Jacobi<T>{io<T>(z), in<T>(invd), in<T>(r)}, n, aligned16(z, invd, r), s));
 }
 
-namespace {
-template <typename T> void xpay_launch(const Xpay<T> &f, int64_t n, cudaStream_t s) {
-  constexpr int W = kW<T>;
-  if (aligned16(f.p, f.z)) launch_dependent(xpay_k<W, T>, grid_for((n + W - 1) / W), kBlock, 0, s, f, n);
-  else launch_dependent(xpay_k<1, T>, grid_for(n), kBlock, 0, s, f, n);
-}
-} // namespace
-
 void xpay(void *p, const void *z, double beta, int dtype, int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
-  DISPATCH(dtype, xpay_launch<T>(Xpay<T>{io<T>(p), in<T>(z), (T)beta, nullptr, nullptr}, n, s));
+  DISPATCH(dtype, map<kW<T>>(Xpay<T>{io<T>(p), in<T>(z), (T)beta}, n, aligned16(p, z), s));
 }
 
 void axpy(void *y, const void *x, double alpha, int dtype, int64_t n, cudaStream_t s) {
@@ -574,30 +663,75 @@ double dot(const void *a, const void *b, int dtype, int64_t n, cudaStream_t s) {
   return v[0];
 }
 
+// f(T, T2) for the types of dtype and dtype2
+#define DISPATCH2(dtype, dtype2, ...)                                                         \
+  DISPATCH(dtype, {                                                                           \
+    if ((dtype2) == PMG_F64) {                                                                \
+      using T2 = double;                                                                      \
+      __VA_ARGS__;                                                                            \
+    } else {                                                                                  \
+      using T2 = float;                                                                       \
+      __VA_ARGS__;                                                                            \
+    }                                                                                         \
+  })
+// entries per pack where vectors of both types are moved
+namespace {
+template <typename T, typename T2> constexpr int kW2 = (sizeof(T) == 8 && sizeof(T2) == 8) ? 2 : 4;
+}
+
 void Scalars::dot(int slot, const void *a, const void *b, int dtype, int64_t n) {
   prof::Scope scope_("vector_reduce", s_);
-  DISPATCH(dtype, reduce<kW<T>>(Dot<T>{in<T>(a), in<T>(b), 0.0}, n, aligned16(a, b), w_->sum(slot), s_));
+  DISPATCH(dtype, reduce<kW<T>>(Dot<T, T>{in<T>(a), in<T>(b), {0.0}}, n, aligned16(a, b), w_->sum(slot), s_));
 }
 
-void Scalars::cg_update(int slot, void *x, void *r, const void *p, const void *v, int rho, int pv, int dtype, int64_t n) {
+void Scalars::dot_converted(int slot, const void *a, int dt_a, const void *b, int dt_b, int64_t n) {
   prof::Scope scope_("vector_reduce", s_);
-  DISPATCH(dtype, reduce<kW<T>>(CgUpdate<T>{io<T>(x), io<T>(r), in<T>(p), in<T>(v), w_->value(rho), w_->value(pv), 0.0, T(0),
-                                            false}, n, aligned16(x, r, p, v), w_->sum(slot), s_));
+  DISPATCH2(dt_a, dt_b, reduce<kW2<T, T2>>(Dot<T, T2>{in<T>(a), in<T2>(b), {0.0}}, n, aligned16(a, b), w_->sum(slot), s_));
 }
 
-void Scalars::residual_dot(int slot, void *r, const void *b, const void *Ax, int dtype, int64_t n) {
+void Scalars::dot_product(int slot, const void *p, const Product &Ap, int dtype, int64_t n) {
   prof::Scope scope_("vector_reduce", s_);
-  DISPATCH(dtype, reduce<kW<T>>(ResidualDot<T>{io<T>(r), in<T>(b), in<T>(Ax), 0.0}, n, aligned16(r, b, Ax), w_->sum(slot), s_));
+  DISPATCH(dtype, reduce<kW<T>>(DotProduct<T>{in<T>(p), consumed<T>(Ap), {0.0}}, n, aligned16(p, Ap.Ax), w_->sum(slot), s_));
+}
+
+void Scalars::cg_update(int slot, void *x, void *r, const void *p, const Product &Ap, int rho, int pv, void *copy,
+                        int dt_copy, int dtype, int64_t n) {
+  prof::Scope scope_("vector_reduce", s_);
+  DISPATCH2(dtype, dt_copy,
+            reduce<kW2<T, T2>>(CgUpdate<T, T2>{io<T>(x), io<T>(r), in<T>(p), consumed<T>(Ap), Copy<T, T2>{io<T2>(copy)},
+                                               w_->value(rho), w_->value(pv), {0.0}, T(0), false}, n,
+                               aligned16(x, r, p, Ap.Ax, copy), w_->sum(slot), s_));
+}
+
+void Scalars::cg_update_jacobi(int slot_rr, int slot_rz, void *r, void *z, const void *invd, const void *p,
+                               const Product &Ap, int rho, int pv, int dtype, int64_t n) {
+  prof::Scope scope_("vector_reduce", s_);
+  DISPATCH(dtype, reduce<kW<T>>(CgUpdateJacobi<T>{io<T>(r), io<T>(z), in<T>(invd), in<T>(p), consumed<T>(Ap), w_->value(rho),
+                                                  w_->value(pv), {0.0, 0.0}, T(0), false}, n, aligned16(r, z, invd, p, Ap.Ax),
+                                w_->sum(slot_rr, slot_rz), s_));
+}
+
+void Scalars::residual_dot(int slot, void *r, const void *b, const void *x, const Product &Ax, void *copy, int dt_copy,
+                           int dtype, int64_t n) {
+  prof::Scope scope_("vector_reduce", s_);
+  DISPATCH2(dtype, dt_copy,
+            reduce<kW2<T, T2>>(ResidualDot<T, T2>{io<T>(r), in<T>(b), in<T>(x), consumed<T>(Ax), Copy<T, T2>{io<T2>(copy)},
+                                                  {0.0}}, n, aligned16(r, b, x, Ax.Ax, copy), w_->sum(slot), s_));
 }
 
 void Scalars::jacobi_dot(int slot, void *z, const void *invd, const void *r, int dtype, int64_t n) {
   prof::Scope scope_("vector_reduce", s_);
-  DISPATCH(dtype, reduce<kW<T>>(JacobiDot<T>{io<T>(z), in<T>(invd), in<T>(r), 0.0}, n, aligned16(z, invd, r), w_->sum(slot), s_));
+  DISPATCH(dtype, reduce<kW<T>>(JacobiDot<T>{io<T>(z), in<T>(invd), in<T>(r), {0.0}}, n, aligned16(z, invd, r), w_->sum(slot), s_));
 }
 
-void Scalars::xpay(void *p, const void *z, int rho, int rho_old, int dtype, int64_t n) {
+void Scalars::xpay(void *p, int dtype, const void *z, int dt_z, int rho, int rho_old, int64_t n) {
   prof::Scope scope_("vector_update", s_);
-  DISPATCH(dtype, xpay_launch<T>(Xpay<T>{io<T>(p), in<T>(z), T(0), w_->value(rho), w_->value(rho_old)}, n, s_));
+  DISPATCH2(dtype, dt_z, {
+    constexpr int W = kW2<T, T2>;
+    const CgDirection<T, T2> f{io<T>(p), in<T2>(z), w_->value(rho), rho_old < 0 ? nullptr : w_->value(rho_old), T(0)};
+    if (aligned16(p, z)) launch_dependent(cg_direction_k<W, CgDirection<T, T2>>, grid_for((n + W - 1) / W), kBlock, 0, s_, f, n);
+    else launch_dependent(cg_direction_k<1, CgDirection<T, T2>>, grid_for(n), kBlock, 0, s_, f, n);
+  });
 }
 
 } // namespace vec

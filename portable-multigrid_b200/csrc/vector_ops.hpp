@@ -52,12 +52,22 @@ public:
   Scalars(const Scalars &) = delete;
   Scalars &operator=(const Scalars &) = delete;
   void dot(int slot, const void *a, const void *b, int dtype, int64_t n);
+  // the same with b of type dt_b, each entry converted to a's type first
+  void dot_converted(int slot, const void *a, int dt_a, const void *b, int dt_b, int64_t n);
+  void dot_product(int slot, const void *p, const Product &Ap, int dtype, int64_t n); // p.(A p), nothing cleared
   void jacobi_dot(int slot, void *z, const void *invd, const void *r, int dtype, int64_t n); // z = invd r; r.z
-  void residual_dot(int slot, void *r, const void *b, const void *Ax, int dtype, int64_t n); // r = b - Ax; r.r
-  // alpha = rho / pv: x += alpha p, r -= alpha v; r.r.  Where rho or pv is not finite or pv <= 0, x
-  // and r stay as they are.
-  void cg_update(int slot, void *x, void *r, const void *p, const void *v, int rho, int pv, int dtype, int64_t n);
-  void xpay(void *p, const void *z, int rho, int rho_old, int dtype, int64_t n); // p = z + (rho / rho_old) p
+  // r = b - A x; r.r; copy (null: none): r in type dt_copy
+  void residual_dot(int slot, void *r, const void *b, const void *x, const Product &Ax, void *copy, int dt_copy,
+                    int dtype, int64_t n);
+  // alpha = rho / pv: x += alpha p, r -= alpha (A p); r.r; copy as above.  Where rho or pv is not
+  // finite or pv <= 0, x and r stay as they are.
+  void cg_update(int slot, void *x, void *r, const void *p, const Product &Ap, int rho, int pv, void *copy, int dt_copy,
+                 int dtype, int64_t n);
+  // the same without x, and z = invd r; r.r and r.z
+  void cg_update_jacobi(int slot_rr, int slot_rz, void *r, void *z, const void *invd, const void *p, const Product &Ap,
+                        int rho, int pv, int dtype, int64_t n);
+  // p = z + (rho / rho_old) p with z of type dt_z; rho_old < 0: p = z
+  void xpay(void *p, int dtype, const void *z, int dt_z, int rho, int rho_old, int64_t n);
   void sync();                  // waits for the stream
   double operator[](int slot) const; // valid after sync()
 
