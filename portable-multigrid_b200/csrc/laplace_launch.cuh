@@ -73,29 +73,25 @@ template <typename K> void allow_smem(K kernel, size_t bytes) {
 // the blocks per SM that registers are allocated for.  The fastest of the shapes measured on
 // B200 (64^3 cells, Q5 and Q6 32^3, Q6 with a coefficient 48^3; time in us with the shape next
 // in line): one warp per pair of Q3 cells needs no block barrier (FP64 full geometry 163; Q4 has
-// 25 lines, which leave 7 lanes of a warp idle, worth it in FP32: 230 against 236 in blocks of
-// five cells, not in FP64: 381 against 376); Q5 and Q6 fill 3 cells' lines into 4 and 5 warps.
-// MINB trades registers for warps: FP64 Q4 full geometry at 4 / 6 / 7 blocks 423 / 376 / 405,
-// Q6 with a coefficient FP64 at 4 / 6 blocks 339 / 328, FP32 at 7 / 8 blocks 220 / 211.
+// 25 lines, which leave 7 lanes of a warp idle: 381 against 376 in blocks of five cells); Q5 and Q6
+// fill 3 cells' lines into 4 and 5 warps.  MINB trades registers for warps: FP64 Q4 full geometry at
+// 4 / 6 / 7 blocks 423 / 376 / 405, Q6 with a coefficient at 4 / 6 blocks 339 / 328.
 template <typename T, int GEOM> constexpr auto line_shape() {
   constexpr bool d = sizeof(T) == 8;
   using kern::LineShape;
   if constexpr (GEOM == 1) { // vmult_box_kernel
     if constexpr (kN == 2) return LineShape<32, 8, 12>{};
     else if constexpr (kN == 3) return LineShape<14, 0, 8>{};
-    else if constexpr (kN == 4) return LineShape<4, 2, 16>{};
-    else if constexpr (kN == 5 && d) return LineShape<2, 1, 12>{};
-    else if constexpr (kN == 5) return LineShape<5, 0, 10>{};
+    else if constexpr (kN == 4) return LineShape<16, 2, 5>{};
+    else if constexpr (kN == 5) return LineShape<2, 1, 12>{};
     else if constexpr (kN == 6) return LineShape<3, 0, 9>{};
-    else return LineShape<3, 0, d ? 6 : 8>{};
+    else return LineShape<3, 0, 6>{};
   } else if constexpr (GEOM == 2) {
     if constexpr (kN == 2) return LineShape<16, 8, 20>{};
-    else if constexpr (kN == 4) return LineShape<4, 2, 12>{};
-    else if constexpr (kN == 5 && d) return LineShape<2, 1, 12>{};
-    else if constexpr (kN == 5) return LineShape<5, 0, 6>{};
-    else if constexpr (kN == 6 && d) return LineShape<3, 0, 9>{};
-    else if constexpr (kN == 6) return LineShape<8, 0, 3>{};
-    else return LineShape<3, 0, d ? 6 : 8>{};
+    else if constexpr (kN == 4) return LineShape<8, 2, 6>{};
+    else if constexpr (kN == 5) return LineShape<2, 1, 12>{};
+    else if constexpr (kN == 6) return LineShape<3, 0, 9>{};
+    else return LineShape<3, 0, 6>{};
   } else {
     if constexpr (kN == 4 && d) return LineShape<2, 2, 24>{};
     else if constexpr (kN == 4) return LineShape<8, 2, 10>{};
@@ -106,27 +102,58 @@ template <typename T, int GEOM> constexpr auto line_shape() {
   }
 }
 
-template <typename T, int GEOM> void line_launch(const SlabLaunch &L) {
-  using SH = decltype(line_shape<T, GEOM>());
-  const int64_t blocks = (L.n_cells + SH::CPB - 1) / SH::CPB;
+// The same for FP32 in pairs of cells (CPB and WC count pairs), degrees 3 to 6.  Half the arithmetic
+// instructions, and the exchanges move 8 bytes per lane.  us, pairs against single cells, 64^3 cells
+// (Q5 32^3, Q6 48^3) with full geometry / a coefficient / neither: Q3 98 / 67 / 48 against 102 / 76 / 75,
+// Q4 226 / 152 / 105 against 234 / 187 / 127, Q5 53 / 34 / 21 against 58 / 41 / 25, Q6 274 / 188 / 113
+// against 285 / 213 / 123 (Q4 without a coefficient in blocks of ten pairs: 105 alone, but 59 against 53 at
+// 64 x 64 x 32, between the updates of a smoother).  On 16^3 cells and fewer both take as long as a launch.
+template <int GEOM> constexpr auto pair_shape() {
+  using kern::LineShape;
+  if constexpr (GEOM == 1) {
+    if constexpr (kN == 4) return LineShape<4, 2, 10>{};
+    else if constexpr (kN == 5) return LineShape<4, 1, 8>{};
+    else if constexpr (kN == 6) return LineShape<3, 0, 5>{};
+    else return LineShape<3, 0, 4>{};
+  } else if constexpr (GEOM == 2) {
+    if constexpr (kN == 4) return LineShape<4, 2, 10>{};
+    else if constexpr (kN == 5) return LineShape<4, 1, 8>{};
+    else if constexpr (kN == 6) return LineShape<8, 0, 2>{};
+    else return LineShape<3, 0, 5>{};
+  } else {
+    if constexpr (kN == 4) return LineShape<2, 2, 20>{};
+    else if constexpr (kN == 5) return LineShape<4, 1, 6>{};
+    else if constexpr (kN == 6) return LineShape<3, 0, 5>{};
+    else return LineShape<3, 0, 3>{};
+  }
+}
+
+template <typename V, int GEOM, typename SH> void line_launch_as(const SlabLaunch &L) {
+  using T = typename kern::Elem<V>::T;
+  constexpr int cells = SH::CPB * kern::Elem<V>::CELLS;
+  const int64_t blocks = (L.n_cells + cells - 1) / cells;
   constexpr int threads = kern::line_threads<kN, SH>();
   const T *src = static_cast<const T *>(L.src);
   T *dst = static_cast<T *>(L.dst);
-  const T c0 = (T)L.affine[0], c1 = (T)L.affine[1], c2 = (T)L.affine[2];
+  const V c0 = (V)L.affine[0], c1 = (V)L.affine[1], c2 = (V)L.affine[2];
   if constexpr (GEOM == 1) {
-    constexpr size_t smem = kern::box_smem<kN, T, SH>();
+    constexpr size_t smem = kern::box_smem<kN, V, SH>();
     static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
-    launch_dependent(kern::vmult_box_kernel<kN, T, SH>, (unsigned)blocks, threads, smem, L.stream, box_tables<kN, T>(), src,
+    launch_dependent(kern::vmult_box_kernel<kN, V, SH>, (unsigned)blocks, threads, smem, L.stream, box_tables<kN, V>(), src,
                      dst, L.idx, c0, c1, c2, L.n_cells);
   } else {
-    constexpr size_t smem = kern::line_smem<kN, T, SH>();
+    constexpr size_t smem = kern::line_smem<kN, V, SH>();
     static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
-    launch_dependent(kern::vmult_line_kernel<kN, T, GEOM, SH>, (unsigned)blocks, threads, smem, L.stream,
-                     line_tables<kN, T>(), src, dst, L.idx, static_cast<const T *>(L.geo),
+    launch_dependent(kern::vmult_line_kernel<kN, V, GEOM, SH>, (unsigned)blocks, threads, smem, L.stream,
+                     line_tables<kN, V>(), src, dst, L.idx, static_cast<const T *>(L.geo),
                      static_cast<const T *>(L.coef), c0, c1, c2, L.n_cells);
   }
   if (L.units) *L.units = L.n_cells;
   if (L.launched) *L.launched = blocks;
+}
+template <typename T, int GEOM> void line_launch(const SlabLaunch &L) {
+  if constexpr (sizeof(T) == 4 && GEOM != 3 && kN >= 4) line_launch_as<kern::F2, GEOM, decltype(pair_shape<GEOM>())>(L);
+  else line_launch_as<T, GEOM, decltype(line_shape<T, GEOM>())>(L);
 }
 
 // ---- slab kernels (degrees 1 and 2) ----

@@ -37,6 +37,61 @@
 namespace pmg {
 namespace kern {
 
+// Two FP32 values moved and computed together, the same place of two neighbouring cells: one packed
+// instruction for two scalar ones, each rounded as the scalar one is.
+struct alignas(8) F2 {
+  float x, y;
+  F2() = default;
+  __host__ __device__ __forceinline__ F2(float a, float b) : x(a), y(b) {}
+  __host__ __device__ __forceinline__ explicit F2(double a) : x((float)a), y((float)a) {}
+  __device__ __forceinline__ static F2 of(unsigned long long b) {
+    F2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(b));
+    return v;
+  }
+  __device__ __forceinline__ unsigned long long bits() const {
+    unsigned long long b;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(x), "f"(y));
+    return b;
+  }
+  friend __device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a.bits()), "l"(b.bits()));
+    return of(d);
+  }
+  friend __device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+    unsigned long long d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a.bits()), "l"(b.bits()));
+    return of(d);
+  }
+  friend __device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a.bits()), "l"(b.bits()));
+    return of(d);
+  }
+  friend __device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a.bits()), "l"(b.bits()), "l"(c.bits()));
+    return of(d);
+  }
+};
+// what a kernel's element V stands for: CELLS cells' values of type T
+template <typename V> struct Elem {
+  using T = V;
+  static constexpr int CELLS = 1;
+  template <typename F> __device__ __forceinline__ static V make(F &&f) { return f(0); }
+  template <typename F> __device__ __forceinline__ static void each(V v, F &&f) { f(0, v); }
+};
+template <> struct Elem<F2> {
+  using T = float;
+  static constexpr int CELLS = 2;
+  template <typename F> __device__ __forceinline__ static F2 make(F &&f) { return F2(f(0), f(1)); }
+  template <typename F> __device__ __forceinline__ static void each(F2 v, F &&f) {
+    f(0, v.x);
+    f(1, v.y);
+  }
+};
+
 // Layouts of the exchange buffers: node (i, j, k) of cell e is at e*CS + i*I + j*J + k*K.
 // Lanes: z lines r = j*N + i, x lines r = k*N + j, y lines r = k*N + i (YK = 0) or i*N + k
 // (YK = 1).  The strides are those with the fewest bank conflicts for the two access patterns
@@ -108,6 +163,12 @@ template <> struct LineLayout<7, double> {
   static constexpr int YK = 0, CS = 353;
 };
 
+// elements of 8 bytes
+template <> struct LineLayout<4, F2> : LineLayout<4, double> {};
+template <> struct LineLayout<5, F2> : LineLayout<5, double> {};
+template <> struct LineLayout<6, F2> : LineLayout<6, double> {};
+template <> struct LineLayout<7, F2> : LineLayout<7, double> {};
+
 // The tables a line kernel reads
 template <int N, typename T> struct LineTab {
   EvenOdd<N, T> eS, eSD, eST, eSDT;
@@ -178,52 +239,59 @@ template <int N, typename T, typename SH> constexpr size_t box_smem() {
 // Full geometry is prefetched into L2 as one bulk request per block, issued before the index
 // map is read, and loaded where it is used: staging it in shared memory takes the room of a
 // block more per SM (FP64 Q4 419 against 376 us, Q3 211 against 163 us at 64^3).
-template <int N, typename T, int GEOM, typename SH>
+template <int N, typename V, int GEOM, typename SH>
 __global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
-    vmult_line_kernel(const __grid_constant__ LineTab<N, T> tab, const T *__restrict__ src, T *__restrict__ dst,
-                      const uint32_t *__restrict__ idx, const T *__restrict__ geo, const T *__restrict__ coef,
-                      T cd0, T cd3, T cd5, int64_t n_cells) {
-  using L = LineLayout<N, T>;
+    vmult_line_kernel(const __grid_constant__ LineTab<N, V> tab, const typename Elem<V>::T *__restrict__ src,
+                      typename Elem<V>::T *__restrict__ dst, const uint32_t *__restrict__ idx,
+                      const typename Elem<V>::T *__restrict__ geo, const typename Elem<V>::T *__restrict__ coef,
+                      V cd0, V cd3, V cd5, int64_t n_cells) {
+  using EL = Elem<V>;
+  using T = typename EL::T;
+  constexpr int CELLS = EL::CELLS;
+  using L = LineLayout<N, V>;
   using E1 = typename L::E1;
   using E2 = typename L::E2;
   constexpr int N2 = N * N, N3 = N2 * N, CPB = SH::CPB, NCOMP = GEOM == 3 ? 10 : 6;
   constexpr int GF = geo_cell_elems<N, T>(NCOMP);
   pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *A0 = reinterpret_cast<T *>(smem_raw), *A1 = A0 + CPB * L::CS, *A2 = A1 + CPB * L::CS;
-  const LinePlace<N, T, SH> at;
+  V *A0 = reinterpret_cast<V *>(smem_raw), *A1 = A0 + CPB * L::CS, *A2 = A1 + CPB * L::CS;
+  const LinePlace<N, V, SH> at;
   const int r = at.r;
-  const int64_t c0 = int64_t(blockIdx.x) * CPB, c = c0 + at.e;
-  const bool in = at.active && c < n_cells;
+  const int64_t c0 = int64_t(blockIdx.x) * (CPB * CELLS), c = c0 + at.e * CELLS; // the first cell of the block, of the element
+  auto in = [&](int m) { return at.active && c + m < n_cells; };
   const uint64_t pol_first = policy_evict_first(), pol_last = policy_evict_last();
   if constexpr (GEOM == 0 || GEOM == 3) {
     if (threadIdx.x == 0) {
       const int64_t left = n_cells - c0;
-      prefetch_l2(geo + c0 * GF, (uint32_t)((left < CPB ? (int)left : CPB) * GF * (int)sizeof(T)), pol_first);
+      prefetch_l2(geo + c0 * GF, (uint32_t)((left < CPB * CELLS ? (int)left : CPB * CELLS) * GF * (int)sizeof(T)), pol_first);
     }
   }
-  uint32_t id[N];
-  line_index<N>(idx, c, r, in, pol_first, id); // (fixed at setup: read before the wait)
+  uint32_t id[CELLS][N];
+#pragma unroll
+  for (int m = 0; m < CELLS; ++m) line_index<N>(idx, c + m, r, in(m), pol_first, id[m]); // (fixed at setup: read before the wait)
   pdl_wait();
   src = pdl_after(src);
   geo = pdl_after(geo);
   coef = pdl_after(coef);
-  T cf[GEOM == 2 ? N : 1]; // the coefficient on the x line, requested before the gather
+  V cf[GEOM == 2 ? N : 1]; // the coefficient on the x line, requested before the gather
   if constexpr (GEOM == 2) {
     const T *cp = coef + c * N3 + r;
 #pragma unroll
-    for (int p = 0; p < N; ++p) cf[p] = in ? ld_keep_early(cp + p * N2, pol_first) : T(0);
+    for (int p = 0; p < N; ++p)
+      cf[p] = EL::make([&](int m) { return in(m) ? ld_keep_early(cp + m * N3 + p * N2, pol_first) : T(0); });
   }
   if (at.active) {
-    T u[N];
+    V u[N];
 #pragma unroll
-    for (int k = 0; k < N; ++k) u[k] = id[k] != kInvalidIdx ? ld_keep(src + id[k], pol_last) : T(0);
-    eo_apply<N, T, 1>(tab.eS, u, [&](int q, T v) { A0[at.z1 + q * E1::K] = v; });
-    eo_apply<N, T, -1>(tab.eSD, u, [&](int q, T v) { A1[at.z1 + q * E1::K] = v; });
+    for (int k = 0; k < N; ++k) 
+      u[k] = EL::make([&](int m) { return id[m][k] != kInvalidIdx ? ld_keep(src + id[m][k], pol_last) : T(0); });
+    eo_apply<N, V, 1>(tab.eS, u, [&](int q, V v) { A0[at.z1 + q * E1::K] = v; });
+    eo_apply<N, V, -1>(tab.eSD, u, [&](int q, V v) { A1[at.z1 + q * E1::K] = v; });
   }
   at.sync();
   {
-    T a[N], z[N];
+    V a[N], z[N];
     if (at.active) {
 #pragma unroll
       for (int j = 0; j < N; ++j) {
@@ -233,81 +301,82 @@ __global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
     }
     at.sync();
     if (at.active) {
-      eo_apply<N, T, 1>(tab.eS, a, [&](int q, T v) { A0[at.y2 + q * E2::J] = v; });
-      eo_apply<N, T, -1>(tab.eSD, a, [&](int q, T v) { A1[at.y2 + q * E2::J] = v; });
-      eo_apply<N, T, 1>(tab.eS, z, [&](int q, T v) { A2[at.y2 + q * E2::J] = v; });
+      eo_apply<N, V, 1>(tab.eS, a, [&](int q, V v) { A0[at.y2 + q * E2::J] = v; });
+      eo_apply<N, V, -1>(tab.eSD, a, [&](int q, V v) { A1[at.y2 + q * E2::J] = v; });
+      eo_apply<N, V, 1>(tab.eS, z, [&](int q, V v) { A2[at.y2 + q * E2::J] = v; });
     }
   }
   at.sync();
   if (at.active) {
     if constexpr (GEOM == 2) {
       // the tensor is diagonal: one direction at a time
-      const T wyz = line_weight<N, T>(tab.W, r % N) * line_weight<N, T>(tab.W, r / N);
+      const V wyz = line_weight<N, V>(tab.W, r % N) * line_weight<N, V>(tab.W, r / N);
 #pragma unroll
-      for (int p = 0; p < N; ++p) cf[p] *= tab.W[p] * wyz;
-      T l[N], d[N];
+      for (int p = 0; p < N; ++p) cf[p] = cf[p] * (tab.W[p] * wyz);
+      V l[N], d[N];
 #pragma unroll
       for (int i = 0; i < N; ++i) l[i] = A0[at.x2 + i * E2::I];
-      eo_apply<N, T, -1>(tab.eSD, l, [&](int q, T v) { d[q] = (cf[q] * cd0) * v; });
-      eo_apply<N, T, -1>(tab.eSDT, d, [&](int q, T v) { A0[at.x2 + q * E2::I] = v; });
+      eo_apply<N, V, -1>(tab.eSD, l, [&](int q, V v) { d[q] = (cf[q] * cd0) * v; });
+      eo_apply<N, V, -1>(tab.eSDT, d, [&](int q, V v) { A0[at.x2 + q * E2::I] = v; });
 #pragma unroll
       for (int i = 0; i < N; ++i) l[i] = A1[at.x2 + i * E2::I];
-      eo_apply<N, T, 1>(tab.eS, l, [&](int q, T v) { d[q] = (cf[q] * cd3) * v; });
-      eo_apply<N, T, 1>(tab.eST, d, [&](int q, T v) { A1[at.x2 + q * E2::I] = v; });
+      eo_apply<N, V, 1>(tab.eS, l, [&](int q, V v) { d[q] = (cf[q] * cd3) * v; });
+      eo_apply<N, V, 1>(tab.eST, d, [&](int q, V v) { A1[at.x2 + q * E2::I] = v; });
 #pragma unroll
       for (int i = 0; i < N; ++i) l[i] = A2[at.x2 + i * E2::I];
-      eo_apply<N, T, 1>(tab.eS, l, [&](int q, T v) { d[q] = (cf[q] * cd5) * v; });
-      eo_apply<N, T, 1>(tab.eST, d, [&](int q, T v) { A2[at.x2 + q * E2::I] = v; });
+      eo_apply<N, V, 1>(tab.eS, l, [&](int q, V v) { d[q] = (cf[q] * cd5) * v; });
+      eo_apply<N, V, 1>(tab.eST, d, [&](int q, V v) { A2[at.x2 + q * E2::I] = v; });
     } else {
-      T dx[N], dy[N], dz[N];
+      V dx[N], dy[N], dz[N];
       {
-        T l[N];
+        V l[N];
 #pragma unroll
         for (int i = 0; i < N; ++i) l[i] = A0[at.x2 + i * E2::I];
-        eo_apply<N, T, -1>(tab.eSD, l, [&](int q, T v) { dx[q] = v; });
+        eo_apply<N, V, -1>(tab.eSD, l, [&](int q, V v) { dx[q] = v; });
 #pragma unroll
         for (int i = 0; i < N; ++i) l[i] = A1[at.x2 + i * E2::I];
-        eo_apply<N, T, 1>(tab.eS, l, [&](int q, T v) { dy[q] = v; });
+        eo_apply<N, V, 1>(tab.eS, l, [&](int q, V v) { dy[q] = v; });
 #pragma unroll
         for (int i = 0; i < N; ++i) l[i] = A2[at.x2 + i * E2::I];
-        eo_apply<N, T, 1>(tab.eS, l, [&](int q, T v) { dz[q] = v; });
+        eo_apply<N, V, 1>(tab.eS, l, [&](int q, V v) { dz[q] = v; });
       }
       const T *gp = geo + c * GF + r;
 #pragma unroll
       for (int p = 0; p < N; ++p) {
-        T g[NCOMP];
+        V g[NCOMP];
 #pragma unroll
-        for (int m = 0; m < NCOMP; ++m) g[m] = in ? ld_keep(gp + (p * NCOMP + m) * N2, pol_first) : T(0);
-        const T x = dx[p], y = dy[p], z = dz[p];
+        for (int m = 0; m < NCOMP; ++m)
+          g[m] = EL::make([&](int k) { return in(k) ? ld_keep(gp + k * GF + (p * NCOMP + m) * N2, pol_first) : T(0); });
+        const V x = dx[p], y = dy[p], z = dz[p];
         if constexpr (GEOM == 0) {
-          dx[p] = g[0] * x + g[1] * y + g[2] * z;
-          dy[p] = g[1] * x + g[3] * y + g[4] * z;
-          dz[p] = g[2] * x + g[4] * y + g[5] * z;
+          dx[p] = fma(g[2], z, fma(g[1], y, g[0] * x));
+          dy[p] = fma(g[4], z, fma(g[3], y, g[1] * x));
+          dz[p] = fma(g[5], z, fma(g[4], y, g[2] * x));
         } else { // J^{-1} row by row, then JxW: the physical gradient, times JxW, and back
-          T gx[3];
+          V gx[3];
 #pragma unroll
-          for (int k = 0; k < 3; ++k) gx[k] = g[NCOMP - 1] * (g[k] * x + g[3 + k] * y + g[(6 + k) % NCOMP] * z);
-          dx[p] = g[0] * gx[0] + g[1] * gx[1] + g[2] * gx[2];
-          dy[p] = g[3] * gx[0] + g[4] * gx[1] + g[5] * gx[2];
-          dz[p] = g[6 % NCOMP] * gx[0] + g[7 % NCOMP] * gx[1] + g[8 % NCOMP] * gx[2];
+          for (int k = 0; k < 3; ++k) gx[k] = g[NCOMP - 1] * fma(g[(6 + k) % NCOMP], z, fma(g[3 + k], y, g[k] * x));
+          dx[p] = fma(g[2], gx[2], fma(g[1], gx[1], g[0] * gx[0]));
+          dy[p] = fma(g[5], gx[2], fma(g[4], gx[1], g[3] * gx[0]));
+          dz[p] = fma(g[8 % NCOMP], gx[2], fma(g[7 % NCOMP], gx[1], g[6 % NCOMP] * gx[0]));
         }
       }
-      eo_apply<N, T, -1>(tab.eSDT, dx, [&](int q, T v) { A0[at.x2 + q * E2::I] = v; });
-      eo_apply<N, T, 1>(tab.eST, dy, [&](int q, T v) { A1[at.x2 + q * E2::I] = v; });
-      eo_apply<N, T, 1>(tab.eST, dz, [&](int q, T v) { A2[at.x2 + q * E2::I] = v; });
+      eo_apply<N, V, -1>(tab.eSDT, dx, [&](int q, V v) { A0[at.x2 + q * E2::I] = v; });
+      eo_apply<N, V, 1>(tab.eST, dy, [&](int q, V v) { A1[at.x2 + q * E2::I] = v; });
+      eo_apply<N, V, 1>(tab.eST, dz, [&](int q, V v) { A2[at.x2 + q * E2::I] = v; });
     }
   }
   at.sync();
   {
-    T a[N], z[N], o[N];
+    V a[N], z[N], o[N];
     if (at.active) {
 #pragma unroll
       for (int j = 0; j < N; ++j) {
         a[j] = A0[at.y2 + j * E2::J];
         z[j] = A1[at.y2 + j * E2::J];
       }
-      eo_apply<N, T, 1>(tab.eST, a, [&](int q, T v) { o[q] = v; });
-      eo_apply<N, T, -1>(tab.eSDT, z, [&](int q, T v) { o[q] += v; });
+      eo_apply<N, V, 1>(tab.eST, a, [&](int q, V v) { o[q] = v; });
+      eo_apply<N, V, -1>(tab.eSDT, z, [&](int q, V v) { o[q] = o[q] + v; });
 #pragma unroll
       for (int j = 0; j < N; ++j) a[j] = A2[at.y2 + j * E2::J];
     }
@@ -315,84 +384,95 @@ __global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
     if (at.active) {
 #pragma unroll
       for (int j = 0; j < N; ++j) A0[at.y1 + j * E1::J] = o[j];
-      eo_apply<N, T, 1>(tab.eST, a, [&](int q, T v) { A1[at.y1 + q * E1::J] = v; });
+      eo_apply<N, V, 1>(tab.eST, a, [&](int q, V v) { A1[at.y1 + q * E1::J] = v; });
     }
   }
   at.sync();
   if (at.active) {
-    T a[N], z[N], o[N];
+    V a[N], z[N], o[N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       a[k] = A0[at.z1 + k * E1::K];
       z[k] = A1[at.z1 + k * E1::K];
     }
-    eo_apply<N, T, 1>(tab.eST, a, [&](int q, T v) { o[q] = v; });
-    eo_apply<N, T, -1>(tab.eSDT, z, [&](int q, T v) { o[q] += v; });
+    eo_apply<N, V, 1>(tab.eST, a, [&](int q, V v) { o[q] = v; });
+    eo_apply<N, V, -1>(tab.eSDT, z, [&](int q, V v) { o[q] = o[q] + v; });
 #pragma unroll
     for (int k = 0; k < N; ++k)
-      if (id[k] != kInvalidIdx) red_keep(dst + id[k], o[k], pol_last);
+      EL::each(o[k], [&](int m, T v) {
+        if (id[m][k] != kInvalidIdx) red_keep(dst + id[m][k], v, pol_last);
+      });
   }
 }
 
 // axis-aligned cells without a coefficient: (cx, cy, cz) = vol / h^2 per direction.  E1, E2 and
 // E3 have buffers of their own (E3 over E1's first), so three barriers order a cell.
-template <int N, typename T, typename SH>
+template <int N, typename V, typename SH>
 __global__ void __launch_bounds__(line_threads<N, SH>(), SH::MINB)
-    vmult_box_kernel(const __grid_constant__ BoxTab<N, T> tab, const T *__restrict__ src, T *__restrict__ dst,
-                     const uint32_t *__restrict__ idx, T cx, T cy, T cz, int64_t n_cells) {
-  using L = LineLayout<N, T>;
+    vmult_box_kernel(const __grid_constant__ BoxTab<N, V> tab, const typename Elem<V>::T *__restrict__ src,
+                     typename Elem<V>::T *__restrict__ dst, const uint32_t *__restrict__ idx, V cx, V cy, V cz,
+                     int64_t n_cells) {
+  using EL = Elem<V>;
+  using T = typename EL::T;
+  constexpr int CELLS = EL::CELLS;
+  using L = LineLayout<N, V>;
   using E1 = typename L::E1;
   using E2 = typename L::E2;
   using E3 = typename L::E3;
   constexpr int CPB = SH::CPB;
   pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *A0 = reinterpret_cast<T *>(smem_raw), *A1 = A0 + CPB * L::CS, *B0 = A1 + CPB * L::CS, *B1 = B0 + CPB * L::CS;
-  const LinePlace<N, T, SH> at;
+  V *A0 = reinterpret_cast<V *>(smem_raw), *A1 = A0 + CPB * L::CS, *B0 = A1 + CPB * L::CS, *B1 = B0 + CPB * L::CS;
+  const LinePlace<N, V, SH> at;
   const int ra = at.r % N, rb = at.r / N;
-  const int64_t c = int64_t(blockIdx.x) * CPB + at.e;
+  const int64_t c = (int64_t(blockIdx.x) * CPB + at.e) * CELLS;
   const uint64_t pol_first = policy_evict_first(), pol_last = policy_evict_last();
-  uint32_t id[N];
-  line_index<N>(idx, c, at.r, at.active && c < n_cells, pol_first, id); // (fixed at setup: read before the wait)
+  uint32_t id[CELLS][N];
+#pragma unroll
+  for (int m = 0; m < CELLS; ++m)
+    line_index<N>(idx, c + m, at.r, at.active && c + m < n_cells, pol_first, id[m]); // (fixed at setup: read before the wait)
   pdl_wait();
   src = pdl_after(src);
   if (at.active) {
-    T u[N];
+    V u[N];
 #pragma unroll
-    for (int k = 0; k < N; ++k) u[k] = id[k] != kInvalidIdx ? ld_keep(src + id[k], pol_last) : T(0);
-    eo_apply<N, T, 1>(tab.eM, u, [&](int q, T v) { A0[at.z1 + q * E1::K] = v; });
-    eo_apply<N, T, 1>(tab.eK, u, [&](int q, T v) { A1[at.z1 + q * E1::K] = cz * v; });
+    for (int k = 0; k < N; ++k) 
+      u[k] = EL::make([&](int m) { return id[m][k] != kInvalidIdx ? ld_keep(src + id[m][k], pol_last) : T(0); });
+    eo_apply<N, V, 1>(tab.eM, u, [&](int q, V v) { A0[at.z1 + q * E1::K] = v; });
+    eo_apply<N, V, 1>(tab.eK, u, [&](int q, V v) { A1[at.z1 + q * E1::K] = cz * v; });
   }
   at.sync();
   if (at.active) {
-    T a[N], b[N], o[N];
+    V a[N], b[N], o[N];
 #pragma unroll
     for (int j = 0; j < N; ++j) {
       a[j] = A0[at.y1 + j * E1::J];
       b[j] = A1[at.y1 + j * E1::J];
     }
-    eo_apply<N, T, 1>(tab.eM, a, [&](int q, T v) { B0[at.y2 + q * E2::J] = v; });
-    eo_apply<N, T, 1>(tab.eK, a, [&](int q, T v) { o[q] = cy * v; });
-    eo_apply<N, T, 1>(tab.eM, b, [&](int q, T v) { B1[at.y2 + q * E2::J] = o[q] + v; });
+    eo_apply<N, V, 1>(tab.eM, a, [&](int q, V v) { B0[at.y2 + q * E2::J] = v; });
+    eo_apply<N, V, 1>(tab.eK, a, [&](int q, V v) { o[q] = v; });
+    eo_apply<N, V, 1>(tab.eM, b, [&](int q, V v) { B1[at.y2 + q * E2::J] = fma(cy, o[q], v); });
   }
   at.sync();
   if (at.active) {
-    T a[N], b[N], o[N];
+    V a[N], b[N], o[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       a[i] = B0[at.x2 + i * E2::I];
       b[i] = B1[at.x2 + i * E2::I];
     }
-    T *x3 = A0 + at.e * L::CS + ra * E3::J + rb * E3::K;
-    eo_apply<N, T, 1>(tab.eK, a, [&](int q, T v) { o[q] = cx * v; });
-    eo_apply<N, T, 1>(tab.eM, b, [&](int q, T v) { x3[q * E3::I] = o[q] + v; });
+    V *x3 = A0 + at.e * L::CS + ra * E3::J + rb * E3::K;
+    eo_apply<N, V, 1>(tab.eK, a, [&](int q, V v) { o[q] = v; });
+    eo_apply<N, V, 1>(tab.eM, b, [&](int q, V v) { x3[q * E3::I] = fma(cx, o[q], v); });
   }
   at.sync();
   if (at.active) {
-    const T *z3 = A0 + at.e * L::CS + ra * E3::I + rb * E3::J;
+    const V *z3 = A0 + at.e * L::CS + ra * E3::I + rb * E3::J;
 #pragma unroll
     for (int k = 0; k < N; ++k)
-      if (id[k] != kInvalidIdx) red_keep(dst + id[k], z3[k * E3::K], pol_last);
+      EL::each(z3[k * E3::K], [&](int m, T v) {
+        if (id[m][k] != kInvalidIdx) red_keep(dst + id[m][k], v, pol_last);
+      });
   }
 }
 
