@@ -12,6 +12,7 @@
 #include "laplace_kernels.cuh"
 #include "line_kernels.cuh"
 #include "line_tables.hpp"
+#include "patch_kernels.cuh"
 #include "pdl.cuh"
 #include "pmg_internal.hpp"
 
@@ -151,7 +152,37 @@ template <typename V, int GEOM, typename SH> void line_launch_as(const SlabLaunc
   if (L.units) *L.units = L.n_cells;
   if (L.launched) *L.launched = blocks;
 }
+// Patches per block (cubes of several small lines share one) and blocks per SM, the fastest measured; cells
+// alone, us, patches against cells (FP64 / FP32; 64^3 cells, Q5 32^3, Q6 48^3): Q2 31 / 21 against 52 / 33,
+// Q3 72 / 45 against 85 / 52, Q4 138 / 84 against 176 / 109, Q5 33 / 23 against 41 / 27, Q6 164 / 101 against
+// 216 / 119.  With a coefficient per point only the nodes are shared, and patches were no faster (Q4
+// 257 / 149 against 267 / 156, Q6 373 / 196 against 335 / 194): cells.
+template <typename T> constexpr auto patch_shape() {
+  [[maybe_unused]] constexpr bool d = sizeof(T) == 8;
+  using kern::PatchShape;
+  if constexpr (kN == 3) return PatchShape<5, 6>{};
+  else if constexpr (kN == 4) return PatchShape<5, d ? 5 : 4>{};
+  else if constexpr (kN == 5) return PatchShape<1, d ? 10 : 8>{};
+  else if constexpr (kN == 6) return PatchShape<1, 8>{};
+  else return PatchShape<1, 4>{};
+}
+template <typename T> void patch_launch(const SlabLaunch &L) {
+  using SH = decltype(patch_shape<T>());
+  constexpr int threads = kern::patch_threads<kN, SH>();
+  constexpr size_t smem = kern::patch_smem<kN, T, SH>();
+  static_assert(smem <= 48 * 1024, "no opt-in for the dynamic shared memory");
+  const int64_t n = L.n_cells / 8, blocks = (n + SH::PPB - 1) / SH::PPB;
+  launch_dependent(kern::vmult_box_patch_kernel<kN, T, SH>, (unsigned)blocks, threads, smem, L.stream, box_tables<kN, T>(),
+                   static_cast<const T *>(L.src), static_cast<T *>(L.dst), L.patch_idx, (T)L.affine[0], (T)L.affine[1],
+                   (T)L.affine[2], n);
+  if (L.units) *L.units = L.n_cells;
+  if (L.launched) *L.launched = blocks;
+}
+
 template <typename T, int GEOM> void line_launch(const SlabLaunch &L) {
+  if constexpr (kern::patch_layout(kN, GEOM)) {
+    if (L.patch_idx) return patch_launch<T>(L);
+  }
   if constexpr (sizeof(T) == 4 && GEOM != 3 && kN >= 4) line_launch_as<kern::F2, GEOM, decltype(pair_shape<GEOM>())>(L);
   else line_launch_as<T, GEOM, decltype(line_shape<T, GEOM>())>(L);
 }

@@ -208,6 +208,30 @@ __global__ void slab_index_kernel(const uint32_t *__restrict__ plain, const uint
   }
 }
 
+// The index map of patches of 2 x 2 x 2 cells, [patch][2N-1][2N-1][2N-1]: cell 8 p + m of the map `idx`
+// (cell by cell) is the half (m & 1, m >> 1 & 1, m >> 2) of patch p.  bad: set where two cells
+// disagree on a node that they would share
+__global__ void patch_index_kernel(const uint32_t *__restrict__ idx, int64_t n_patches, int N, uint32_t *__restrict__ out,
+                                   unsigned int *__restrict__ bad) {
+  const int n1 = 2 * N - 1, n3 = n1 * n1 * n1;
+  const int64_t total = n_patches * n3;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = t / n3;
+    const int l = (int)(t - p * n3), I = l % n1, J = (l / n1) % n1, K = l / (n1 * n1);
+    uint32_t v = 0;
+    bool first = true;
+    for (int m = 0; m < 8; ++m) {
+      const int i = I - (m & 1) * (N - 1), j = J - (m >> 1 & 1) * (N - 1), k = K - (m >> 2) * (N - 1);
+      if (i < 0 || i >= N || j < 0 || j >= N || k < 0 || k >= N) continue;
+      const uint32_t w = idx[(8 * p + m) * (N * N * N) + (k * N + j) * N + i];
+      if (first) v = w;
+      else if (w != v) atomicOr(bad, 1u);
+      first = false;
+    }
+    out[t] = v;
+  }
+}
+
 int grid_for(int64_t n, int sms, int threads = 256) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + threads - 1) / threads, (int64_t)sms * 32));
 }
@@ -297,6 +321,20 @@ void device_slab_index(const uint32_t *plain, const uint8_t *cons, int64_t n_cel
                                                            idx.as<uint32_t>());
     PMG_LAUNCH_CHECK();
   }
+}
+
+void device_patch_index(const uint32_t *idx, int64_t n_cells, int N, int sms, DeviceBuffer &out, cudaStream_t s) {
+  out = DeviceBuffer();
+  if (n_cells <= 0 || n_cells % 8 != 0) return;
+  const int64_t n_patches = n_cells / 8, total = n_patches * (2 * N - 1) * (2 * N - 1) * (2 * N - 1);
+  DeviceBuffer map(sizeof(uint32_t) * total), flag(sizeof(unsigned int));
+  PMG_CUDA(cudaMemsetAsync(flag.get(), 0, flag.bytes(), s));
+  patch_index_kernel<<<grid_for(total, sms), 256, 0, s>>>(idx, n_patches, N, map.as<uint32_t>(), flag.as<unsigned int>());
+  PMG_LAUNCH_CHECK();
+  unsigned int bad = 0;
+  PMG_CUDA(cudaMemcpyAsync(&bad, flag.get(), sizeof(bad), cudaMemcpyDeviceToHost, s));
+  PMG_CUDA(cudaStreamSynchronize(s));
+  if (!bad) out = std::move(map);
 }
 
 } // namespace pmg

@@ -330,6 +330,9 @@ void build_slab_index(pmg_operator &op) {
   op.line = op.kind == PMG_OP_MASS ? kern::mass_line_layout(op.nm) : kern::line_layout(op.nm, geom_code(op));
   device_slab_index(op.dplain.as<uint32_t>(), op.dcons.as<uint8_t>(), op.n_cells, op.nm, op.line, op.cpw, op.lanes,
                     op.n_groups, op.sms, op.idx, nullptr);
+  op.patch_idx = DeviceBuffer();
+  if (op.kind == PMG_OP_LAPLACE && kern::patch_layout(op.nm, geom_code(op)) && kern::patches_fill(op.nm, op.n_cells, op.sms))
+    device_patch_index(op.idx.as<uint32_t>(), op.n_cells, op.nm, op.sms, op.patch_idx, nullptr);
 }
 
 // the constrained DoFs as a list and a bitmask (copy_constrained_values, bk3.h:230)
@@ -703,6 +706,7 @@ void add_product(const pmg_operator &op, void *dst, const void *src, cudaStream_
   SlabLaunch L = slab_launch(op, cached_tables(op.degree), s);
   L.src = src;
   L.dst = dst;
+  L.patch_idx = op.patch_idx.as<uint32_t>();
   L.err = op.err_flag.as<unsigned int>();
   L.units = &op.launch_units[PMG_KERNEL_VMULT_CELL];
   L.launched = &op.launch_par[PMG_KERNEL_VMULT_CELL];

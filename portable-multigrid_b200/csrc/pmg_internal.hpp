@@ -197,6 +197,7 @@ struct pmg_operator {
   mutable pmg::Numbering num;
   mutable bool host_num_valid = false;
   pmg::DeviceBuffer idx;            // uint32, n_groups * cpw cells of nm^3 entries
+  pmg::DeviceBuffer patch_idx;      // uint32, (2 nm - 1)^3 entries per 2 x 2 x 2 cells; empty: no such patches
   pmg::DeviceBuffer geo;            // FULL: 6 (INVJAC: 10) values per point; AFFINE: [C][8]
   pmg::DeviceBuffer coef;           // AFFINE with coefficient: a value per point;
                                     // MASS with mass_geom 0: |det J| w_q (times coefficient)
