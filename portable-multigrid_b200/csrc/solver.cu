@@ -160,7 +160,8 @@ void chebyshev_estimate(pmg_chebyshev &c, cudaStream_t s) {
 // iterate (one vector written per step); the first iterate goes where the parity of the
 // remaining steps puts the last one into dst.  Per element the arithmetic is that of the
 // two-vector form, so results are bit-identical to it.
-void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zero, cudaStream_t s) {
+void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zero, cudaStream_t s, void *zero,
+                     int64_t n_zero) {
   if (!c.estimated) chebyshev_estimate(c, s);
   pmg_operator &op = *c.op;
   const int dt = op.dtype;
@@ -171,7 +172,7 @@ void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zer
   void *cur = nullptr, *prev = nullptr; // x_k and x_{k-1} (null: x_{k-1} = 0)
   if (from_zero) {
     cur = ((d - 1) % 2 == 0) ? A : B;
-    vec::cheb_init(cur, src, op.inv_diag.get(), 1.0 / c.theta, dt, N, s);
+    vec::cheb_init(cur, src, op.inv_diag.get(), 1.0 / c.theta, zero, n_zero, dt, N, s);
   } else {
     const vec::Product Ax = operator_product(op, c.Ax.get(), dst, s);
     if (d % 2 == 0) { // x_1 into xo, x_0 stays in dst as the previous iterate
@@ -230,6 +231,8 @@ void mg_setup(pmg_mg &mg, int n_levels, pmg_operator *const *levels, pmg_transfe
     mg.def[l].allocate(bytes);
     mg.t[l].allocate(bytes);
   }
+  mg.restrict_residual.assign(n_levels, false);
+  for (int l = 1; l < n_levels; ++l) mg.restrict_residual[l] = transfer_restricts_residual(*mg.transfers[l], *mg.levels[l]);
   mg.tail = mg_tail_plan(mg);
 }
 
@@ -247,11 +250,16 @@ void mg_vcycle(pmg_mg &mg, int l, int tail, cudaStream_t s) {
     return;
   }
   pmg_operator &opc = *mg.levels[l - 1];
-  chebyshev_apply(*mg.smoothers[l], mg.sol[l].get(), mg.def[l].get(), true, s);
-  // t = def - A sol, and def[l - 1] = 0 for the restriction (portable_multigrid_solver.h:180-183)
+  // the smoother from zero (its first launch sets def[l - 1] = 0), then def[l - 1] += P^T (def - A sol)
+  // (portable_multigrid_solver.h:180-183)
+  chebyshev_apply(*mg.smoothers[l], mg.sol[l].get(), mg.def[l].get(), true, s, mg.def[l - 1].get(), opc.n_dofs);
   const vec::Product Ax = operator_product(op, mg.smoothers[l]->Ax.get(), mg.sol[l].get(), s);
-  vec::residual(mg.t[l].get(), mg.def[l].get(), mg.sol[l].get(), Ax, mg.def[l - 1].get(), opc.n_dofs, dt, N, s);
-  transfer_apply(*mg.transfers[l], 1, mg.def[l - 1].get(), mg.t[l].get(), s);
+  if (mg.restrict_residual[l]) {
+    transfer_restrict_residual(*mg.transfers[l], mg.def[l - 1].get(), mg.def[l].get(), Ax.Ax, s);
+  } else {
+    vec::residual(mg.t[l].get(), mg.def[l].get(), mg.sol[l].get(), Ax, dt, N, s);
+    transfer_apply(*mg.transfers[l], 1, mg.def[l - 1].get(), mg.t[l].get(), s);
+  }
   mg_vcycle(mg, l - 1, tail, s);
   transfer_apply(*mg.transfers[l], 0, mg.sol[l].get(), mg.sol[l - 1].get(), s);
   chebyshev_apply(*mg.smoothers[l], mg.sol[l].get(), mg.def[l].get(), false, s);

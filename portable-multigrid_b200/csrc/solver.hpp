@@ -27,6 +27,7 @@ struct pmg_mg {
   std::vector<pmg_transfer *> transfers;
   std::vector<pmg_chebyshev *> smoothers;
   std::vector<pmg::DeviceBuffer> sol, def, t;
+  std::vector<char> restrict_residual; // per level: the restriction to the level below takes def - A sol itself
   std::shared_ptr<pmg::TailPlan> tail; // the coarse levels that run in one kernel, null: none
   // The V-cycle below the finest level's input and output buffers is a fixed sequence of
   // launches on fixed buffers: it is captured once into a CUDA graph and replayed.
@@ -41,7 +42,9 @@ struct pmg_mg {
 namespace pmg {
 void chebyshev_setup(pmg_chebyshev &c, pmg_operator &op, const pmg_chebyshev_params &prm);
 void chebyshev_estimate(pmg_chebyshev &c, cudaStream_t s);
-void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zero, cudaStream_t s);
+// zero (null: none) [n_zero], with from_zero: set to zero in the first launch
+void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zero, cudaStream_t s, void *zero = nullptr,
+                     int64_t n_zero = 0);
 void mg_setup(pmg_mg &mg, int n_levels, pmg_operator *const *levels, pmg_transfer *const *transfers,
               pmg_chebyshev *const *smoothers);
 void mg_vmult(pmg_mg &mg, void *dst, const void *src, int vec_dtype, cudaStream_t s);

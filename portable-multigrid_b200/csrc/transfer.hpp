@@ -26,4 +26,8 @@ void transfer_setup_from_maps(pmg_transfer &t, const pmg_operator &coarse, const
                               const pmg_transfer_maps &maps);
 // dir 0: dst_fine += P src_coarse;  dir 1: dst_coarse += P^T src_fine
 void transfer_apply(const pmg_transfer &t, int dir, void *dst, const void *src, cudaStream_t s);
+// whether transfer_restrict_residual may be used for products of the operator `fine` (setup; waits for the device)
+bool transfer_restricts_residual(const pmg_transfer &t, const pmg_operator &fine);
+// dst_coarse += P^T (def - A x) and A x = 0; A x without its identity rows
+void transfer_restrict_residual(const pmg_transfer &t, void *dst, const void *def, void *Ax, cudaStream_t s);
 } // namespace pmg

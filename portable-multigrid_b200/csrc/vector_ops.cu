@@ -223,12 +223,20 @@ template <typename T> struct Zero {
   T *p;
   template <int W> __device__ void run(int64_t i) { store<W>(p + i, Pack<T, W>{}); }
 };
-template <int W, typename T>
-__global__ void __launch_bounds__(kBlock) residual_k(Residual<T> f, int64_t n, Zero<T> z, int64_t n_zero) {
+// f over n entries and zeros over n_zero others
+template <int W, typename T, typename F>
+__global__ void __launch_bounds__(kBlock) map_zero_k(F f, int64_t n, Zero<T> z, int64_t n_zero) {
   pdl_trigger();
   pdl_wait();
   for_packs<W>(n, f);
   for_packs<W>(n_zero, z);
+}
+template <typename T, typename F>
+void map_zero(const F &f, int64_t n, void *zero, int64_t n_zero, bool wide, cudaStream_t s) {
+  const Zero<T> z{static_cast<T *>(zero)};
+  if (!zero) n_zero = 0;
+  if (wide) launch_dependent(map_zero_k<kW<T>, T, F>, grid_for((std::max(n, n_zero) + kW<T> - 1) / kW<T>), kBlock, 0, s, f, n, z, n_zero);
+  else launch_dependent(map_zero_k<1, T, F>, grid_for(std::max(n, n_zero)), kBlock, 0, s, f, n, z, n_zero);
 }
 
 template <typename T> struct Jacobi {
@@ -597,9 +605,11 @@ void init_product(void *dst, const void *src, const uint32_t *bits, int dtype, i
   DISPATCH(dtype, map<kW<T>>(InitProduct<T>{io<T>(dst), in<T>(src), bits}, n, aligned16(dst), s));
 }
 
-void cheb_init(void *dst, const void *src, const void *invd, double scale, int dtype, int64_t n, cudaStream_t s) {
+void cheb_init(void *dst, const void *src, const void *invd, double scale, void *zero, int64_t n_zero, int dtype,
+               int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
-  DISPATCH(dtype, map<kW<T>>(ChebInit<T>{io<T>(dst), in<T>(src), in<T>(invd), (T)scale}, n, aligned16(dst, src, invd), s));
+  DISPATCH(dtype, map_zero<T>(ChebInit<T>{io<T>(dst), in<T>(src), in<T>(invd), (T)scale}, n, zero, n_zero,
+                              aligned16(dst, src, invd, zero), s));
 }
 
 void cheb_first_step(void *out, void *keep, const void *x0, const void *src, const Product &p, const void *invd,
@@ -626,19 +636,9 @@ void cheb_update(void *out, const void *cur, const void *prev, const void *src, 
                                                     in<T>(invd), (T)f1, (T)f2}, n, wide, s));
 }
 
-void residual(void *t, const void *def, const void *x, const Product &p, void *zero, int64_t n_zero, int dtype,
-              int64_t n, cudaStream_t s) {
+void residual(void *t, const void *def, const void *x, const Product &p, int dtype, int64_t n, cudaStream_t s) {
   prof::Scope scope_("vector_update", s);
-  if (!zero) n_zero = 0;
-  const bool wide = aligned16(t, def, x, p.Ax, zero);
-  DISPATCH(dtype, {
-    const Residual<T> f{io<T>(t), in<T>(def), in<T>(x), consumed<T>(p)};
-    const Zero<T> z{io<T>(zero)};
-    if (wide)
-      launch_dependent(residual_k<kW<T>, T>, grid_for((std::max(n, n_zero) + kW<T> - 1) / kW<T>), kBlock, 0, s, f, n, z, n_zero);
-    else
-      launch_dependent(residual_k<1, T>, grid_for(std::max(n, n_zero)), kBlock, 0, s, f, n, z, n_zero);
-  });
+  DISPATCH(dtype, map<kW<T>>(Residual<T>{io<T>(t), in<T>(def), in<T>(x), consumed<T>(p)}, n, aligned16(t, def, x, p.Ax), s));
 }
 
 void jacobi(void *z, const void *invd, const void *r, int dtype, int64_t n, cudaStream_t s) {

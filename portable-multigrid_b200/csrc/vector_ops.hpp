@@ -24,8 +24,9 @@ struct Product {
 // dst = 0 with the identity rows dst_i = src_i of the constrained DoFs
 void init_product(void *dst, const void *src, const uint32_t *bits, int dtype, int64_t n, cudaStream_t s);
 // Chebyshev vector steps (x_{k+1} = x_k + f1 (x_k - x_{k-1}) + f2 D^{-1} (b - A x_k)):
-// cheb_init: dst = scale D^{-1} src
-void cheb_init(void *dst, const void *src, const void *invd, double scale, int dtype, int64_t n, cudaStream_t s);
+// cheb_init: dst = scale D^{-1} src; zero (null: none) [n_zero] is set to zero in the same launch
+void cheb_init(void *dst, const void *src, const void *invd, double scale, void *zero, int64_t n_zero, int dtype,
+               int64_t n, cudaStream_t s);
 // cheb_first_step: out = x0 + scale D^{-1} (src - A x0), and keep = x0 unless null (keep != x0;
 // out == x0 allowed)
 void cheb_first_step(void *out, void *keep, const void *x0, const void *src, const Product &p, const void *invd,
@@ -33,9 +34,8 @@ void cheb_first_step(void *out, void *keep, const void *x0, const void *src, con
 // cheb_update: out = the update from cur and prev (null: zero), out == prev allowed
 void cheb_update(void *out, const void *cur, const void *prev, const void *src, const Product &p, const void *invd,
                  double f1, double f2, int dtype, int64_t n, cudaStream_t s);
-// t = def - A x; zero (null: none) [n_zero] is set to zero in the same launch
-void residual(void *t, const void *def, const void *x, const Product &p, void *zero, int64_t n_zero, int dtype,
-              int64_t n, cudaStream_t s);
+// t = def - A x
+void residual(void *t, const void *def, const void *x, const Product &p, int dtype, int64_t n, cudaStream_t s);
 void jacobi(void *z, const void *invd, const void *r, int dtype, int64_t n, cudaStream_t s);
 void xpay(void *p, const void *z, double beta, int dtype, int64_t n, cudaStream_t s);
 void axpy(void *y, const void *x, double alpha, int dtype, int64_t n, cudaStream_t s); // y += alpha x
