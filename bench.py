@@ -543,7 +543,7 @@ def dg_time_to_solution(torch, pmg, dev, refine=6, repeats=3):
 
 def dg_vmult_rates(torch, pmg, dev, refine=6, launches=20, peak=None):
     """The DG-SIPG Q3 vmult of config 4 alone (64^3 cells), FP32 and FP64: CUDA-event time per
-    vmult (all its kernels: the fused tile kernel where the mesh allows it), GDoF/s and the
+    vmult (all its kernels), GDoF/s and the
     algorithmic bytes 2 s N + 6 s C (src read and dst written once, six geometry values per
     cell; DG indices are implicit) over that time as a fraction of the HBM peak."""
     p = 3
@@ -727,7 +727,7 @@ def gpu_arm(args):
                          "peak_source": ("measured MEASURED_PEAKS.json hbm_gbs" if peak_kind == "measured"
                                          else "fallback 6650 GB/s (MEASURED_PEAKS.json absent)"),
                          "frac_of_same_run_copy": achieved / peaks["copy_gbs"] if peaks else None,
-                         "kernel": "vmult_slab_kernel<5,double,0>",
+                         "kernel": "vmult_line_kernel<5,double,0>",
                          "algorithmic_bytes_per_launch": alg_bytes,
                          "kernel_ms_avg": cell_avg_s * 1e3},
             "e2e": {"value": e2e_value, "unit": "GDoF/s",

@@ -1,6 +1,6 @@
 // Tensor-core variant of the affine (+ coefficient) FP32 cell operator: TF32 mma.sync.
 //
-// The operator is the one of vmult_slab_kernel with GEOM 1 / 2 (axis-aligned cells, the
+// The operator is the one of vmult_box_kernel and vmult_line_kernel<GEOM = 2> (axis-aligned cells, the
 // diagonal cell tensor rr, ss, tt times the Gauss weights and the coefficient per point), the
 // BK3 cell operator of include/kernels/bk3_kokkos_kernel.h:25-746.  Here one warp applies a
 // cell as twelve 1D contractions, each a product of the cell's 64 node lines (8 x 8, the
