@@ -327,6 +327,10 @@ void device_patch_index(const uint32_t *idx, int64_t n_cells, int N, int sms, De
   out = DeviceBuffer();
   if (n_cells <= 0 || n_cells % 8 != 0) return;
   const int64_t n_patches = n_cells / 8, total = n_patches * (2 * N - 1) * (2 * N - 1) * (2 * N - 1);
+  // a second map beside the cells' own: not where memory is short (a quarter of what is free)
+  size_t free_bytes = 0, total_bytes = 0;
+  PMG_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+  if (sizeof(uint32_t) * (size_t)total > free_bytes / 4) return;
   DeviceBuffer map(sizeof(uint32_t) * total), flag(sizeof(unsigned int));
   PMG_CUDA(cudaMemsetAsync(flag.get(), 0, flag.bytes(), s));
   patch_index_kernel<<<grid_for(total, sms), 256, 0, s>>>(idx, n_patches, N, map.as<uint32_t>(), flag.as<unsigned int>());

@@ -27,7 +27,7 @@ void device_slab_index(const uint32_t *plain, const uint8_t *cons, int64_t n_cel
                        int lanes, int64_t n_groups, int sms, DeviceBuffer &idx, cudaStream_t s);
 
 // the nodes of the patches of 2 x 2 x 2 cells from a map cell by cell, where every eight consecutive cells
-// share their nodes as such a patch does (Morton order), else nothing; synchronises s
+// share their nodes as such a patch does (Morton order) and memory is not short, else nothing; synchronises s
 void device_patch_index(const uint32_t *idx, int64_t n_cells, int N, int sms, DeviceBuffer &out, cudaStream_t s);
 
 } // namespace pmg
