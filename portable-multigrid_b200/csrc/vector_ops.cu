@@ -435,6 +435,9 @@ template <typename T, typename TC> struct CgUpdate {
     Ap.template done<W>(i);
   }
 };
+// The step of an eigenvalue estimate is taken whatever the signs: with an indefinite operator (a DG penalty
+// below the coercive one) or a negative one p.Ap < 0 is a step of the Lanczos run like any other.  (CG itself
+// stops there.)
 template <typename T> struct CgUpdateJacobi {
   T *r, *z;
   const T *invd, *p;
@@ -442,18 +445,13 @@ template <typename T> struct CgUpdateJacobi {
   const double *rho, *pv;
   double acc[2]; // r.r, r.z
   T alpha;
-  bool step;
-  __device__ void begin() {
-    double a;
-    step = cg_step(rho, pv, a);
-    alpha = (T)a;
-  }
+  __device__ void begin() { alpha = (T)(*rho / *pv); }
   template <int W> __device__ void run(int64_t i) {
     Pack<T, W> rv = load<W>(r + i), zv;
     const auto pp = load<W>(p + i), vv = Ap.template take<W>(i, pp), di = load<W>(invd + i);
 #pragma unroll
     for (int k = 0; k < W; ++k) {
-      if (step) rv.v[k] = rv.v[k] - alpha * vv.v[k];
+      rv.v[k] = rv.v[k] - alpha * vv.v[k];
       zv.v[k] = di.v[k] * rv.v[k];
       acc[0] += (double)rv.v[k] * (double)rv.v[k];
       acc[1] += (double)rv.v[k] * (double)zv.v[k];
@@ -707,7 +705,7 @@ void Scalars::cg_update_jacobi(int slot_rr, int slot_rz, void *r, void *z, const
                                const Product &Ap, int rho, int pv, int dtype, int64_t n) {
   prof::Scope scope_("vector_reduce", s_);
   DISPATCH(dtype, reduce<kW<T>>(CgUpdateJacobi<T>{io<T>(r), io<T>(z), in<T>(invd), in<T>(p), consumed<T>(Ap), w_->value(rho),
-                                                  w_->value(pv), {0.0, 0.0}, T(0), false}, n, aligned16(r, z, invd, p, Ap.Ax),
+                                                  w_->value(pv), {0.0, 0.0}, T(0)}, n, aligned16(r, z, invd, p, Ap.Ax),
                                 w_->sum(slot_rr, slot_rz), s_));
 }
 

@@ -63,7 +63,7 @@ public:
   // finite or pv <= 0, x and r stay as they are.
   void cg_update(int slot, void *x, void *r, const void *p, const Product &Ap, int rho, int pv, void *copy, int dt_copy,
                  int dtype, int64_t n);
-  // the same without x, and z = invd r; r.r and r.z
+  // the same without x and with every step taken, and z = invd r; r.r and r.z
   void cg_update_jacobi(int slot_rr, int slot_rz, void *r, void *z, const void *invd, const void *p, const Product &Ap,
                         int rho, int pv, int dtype, int64_t n);
   // p = z + (rho / rho_old) p with z of type dt_z; rho_old < 0: p = z
