@@ -353,7 +353,9 @@ typedef struct {
 
 /* initialize(matrix, data) with the operator's inverse diagonal as preconditioner
  * (computed here if needed); the eigenvalue estimate runs on the first use or in
- * pmg_chebyshev_estimate. */
+ * pmg_chebyshev_estimate.  A smoother keeps work vectors that carry state from call to call:
+ * its calls, and those of the V-cycles it belongs to, go to one stream at a time (a change of
+ * stream is ordered by the caller). */
 pmg_status pmg_chebyshev_create(pmg_operator *op, const pmg_chebyshev_params *params,
                                 pmg_chebyshev **smoother);
 pmg_status pmg_chebyshev_destroy(pmg_chebyshev *smoother);

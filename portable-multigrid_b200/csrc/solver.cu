@@ -50,6 +50,17 @@ void check_finite(double v, const char *what) {
   if (!std::isfinite(v)) fail(PMG_ENONFINITE, std::string("non-finite value in ") + what);
 }
 
+// A x in the smoother's work vector; the caller unsets product_open once the consuming update is launched
+vec::Product open_product(pmg_chebyshev &c, const void *x, cudaStream_t s) {
+  c.product_open = true;
+  return operator_product(*c.op, c.Ax.get(), x, s);
+}
+// at the start of a call: the remains of one that failed between a product and its update
+void clear_product(pmg_chebyshev &c, cudaStream_t s) {
+  if (!c.product_open) return;
+  PMG_CUDA(cudaMemsetAsync(c.Ax.get(), 0, c.Ax.bytes(), s));
+  c.product_open = false;
+}
 } // namespace
 
 void chebyshev_setup(pmg_chebyshev &c, pmg_operator &op, const pmg_chebyshev_params &prm) {
@@ -163,6 +174,7 @@ void chebyshev_estimate(pmg_chebyshev &c, cudaStream_t s) {
 void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zero, cudaStream_t s, void *zero,
                      int64_t n_zero) {
   if (!c.estimated) chebyshev_estimate(c, s);
+  clear_product(c, s);
   pmg_operator &op = *c.op;
   const int dt = op.dtype;
   const int64_t N = op.n_dofs;
@@ -174,7 +186,7 @@ void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zer
     cur = ((d - 1) % 2 == 0) ? A : B;
     vec::cheb_init(cur, src, op.inv_diag.get(), 1.0 / c.theta, zero, n_zero, dt, N, s);
   } else {
-    const vec::Product Ax = operator_product(op, c.Ax.get(), dst, s);
+    const vec::Product Ax = open_product(c, dst, s);
     if (d % 2 == 0) { // x_1 into xo, x_0 stays in dst as the previous iterate
       vec::cheb_first_step(B, nullptr, A, src, Ax, op.inv_diag.get(), 1.0 / c.theta, dt, N, s);
       cur = B;
@@ -184,6 +196,7 @@ void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zer
       cur = A;
       prev = B;
     }
+    c.product_open = false;
   }
   if (!more) return;
   double rhok = c.delta / c.theta;
@@ -195,8 +208,9 @@ void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zer
     void *out = prev ? prev : (cur == A ? B : A);
     // DG operators on cell tiles apply the step inside their vmult kernel (A cur never stored)
     if (!operator_vmult_chebyshev(op, out, cur, prev, src, op.inv_diag.get(), f1, f2, s)) {
-      const vec::Product Ax = operator_product(op, c.Ax.get(), cur, s);
+      const vec::Product Ax = open_product(c, cur, s);
       vec::cheb_update(out, cur, prev, src, Ax, op.inv_diag.get(), f1, f2, dt, N, s);
+      c.product_open = false;
     }
     prev = cur;
     cur = out;
@@ -253,13 +267,14 @@ void mg_vcycle(pmg_mg &mg, int l, int tail, cudaStream_t s) {
   // the smoother from zero (its first launch sets def[l - 1] = 0), then def[l - 1] += P^T (def - A sol)
   // (portable_multigrid_solver.h:180-183)
   chebyshev_apply(*mg.smoothers[l], mg.sol[l].get(), mg.def[l].get(), true, s, mg.def[l - 1].get(), opc.n_dofs);
-  const vec::Product Ax = operator_product(op, mg.smoothers[l]->Ax.get(), mg.sol[l].get(), s);
+  const vec::Product Ax = open_product(*mg.smoothers[l], mg.sol[l].get(), s);
   if (mg.restrict_residual[l]) {
     transfer_restrict_residual(*mg.transfers[l], mg.def[l - 1].get(), mg.def[l].get(), Ax.Ax, s);
   } else {
     vec::residual(mg.t[l].get(), mg.def[l].get(), mg.sol[l].get(), Ax, dt, N, s);
     transfer_apply(*mg.transfers[l], 1, mg.def[l - 1].get(), mg.t[l].get(), s);
   }
+  mg.smoothers[l]->product_open = false;
   mg_vcycle(mg, l - 1, tail, s);
   transfer_apply(*mg.transfers[l], 0, mg.sol[l].get(), mg.sol[l - 1].get(), s);
   chebyshev_apply(*mg.smoothers[l], mg.sol[l].get(), mg.def[l].get(), false, s);
@@ -312,8 +327,10 @@ void mg_capture(pmg_mg &mg) {
 // the V-cycle from mg.def into mg.sol on the finest level
 void mg_cycle(pmg_mg &mg, cudaStream_t s) {
   const int L = (int)mg.levels.size() - 1;
-  for (auto *sm : mg.smoothers)
+  for (auto *sm : mg.smoothers) {
     if (!sm->estimated) chebyshev_estimate(*sm, s);
+    clear_product(*sm, s); // (a replayed graph has no such look)
+  }
   // a graph captured before a smoother was re-estimated holds the old Chebyshev coefficients
   if (mg.graph) {
     bool stale = mg.graph_generations.size() != mg.smoothers.size();

@@ -18,6 +18,9 @@ struct pmg_chebyshev {
   double theta = 1, delta = 0, min_ev = 1, max_ev = 1;
   int cg_its = 0;
   pmg::DeviceBuffer xo, Ax;
+  // Ax is zero between calls: a product is added into it and the update that consumes it clears it.
+  // Set while a product waits for its update: still set at the next call, that update never came
+  bool product_open = false;
   std::vector<pmg::DeviceBuffer> est_work; // eigenvalue-estimate vectors kept once re-estimated
 };
 
