@@ -100,7 +100,7 @@ public:
     bytes_ = bytes;
   }
   void release() {
-    if (ptr_) cudaFree(ptr_);
+    if (ptr_ && cudaFree(ptr_) != cudaSuccess) (void)cudaGetLastError(); // (not left for the next call's checks)
     ptr_ = nullptr;
     bytes_ = 0;
   }

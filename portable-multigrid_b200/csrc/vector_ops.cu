@@ -510,7 +510,7 @@ struct ScalarSpace {
   double *host = nullptr;
   ScalarSpace() = default;
   ~ScalarSpace() {
-    if (host) cudaFreeHost(host);
+    if (host && cudaFreeHost(host) != cudaSuccess) (void)cudaGetLastError();
   }
   Sum sum(int slot, int second = 0) {
     double *p = partials.as<double>(), *v = p + 2 * kMaxPartials;
@@ -553,10 +553,17 @@ Scalars::Scalars(cudaStream_t s) : s_(s) {
 }
 // the memory goes back to the pool only once no kernel uses it
 Scalars::~Scalars() {
-  const bool ok = cudaStreamSynchronize(s_) == cudaSuccess;
+  bool unused = cudaStreamSynchronize(s_) == cudaSuccess;
+  if (!unused) {
+    (void)cudaGetLastError(); // raised where it arose: the checks of the next call must not find it again
+    // refused because the stream is being captured: the capture is void, and nothing of it runs
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    unused = cudaStreamIsCapturing(s_, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();
+  }
   Pool &p = pool();
   std::lock_guard<std::mutex> lock(p.mu);
-  if (ok && p.idle.size() < kPool) p.idle.push_back(std::move(w_));
+  if (unused && p.idle.size() < kPool) p.idle.push_back(std::move(w_));
 }
 void Scalars::sync() { PMG_CUDA(cudaStreamSynchronize(s_)); }
 double Scalars::operator[](int slot) const { return w_->host[slot]; }
