@@ -77,10 +77,8 @@ void chebyshev_setup(pmg_chebyshev &c, pmg_operator &op, const pmg_chebyshev_par
   c.xo.allocate(bytes);
   c.Ax.allocate(bytes);
   PMG_CUDA(cudaMemset(c.Ax.get(), 0, bytes)); // every product is consumed and cleared by its update
-  if (!op.has_diag) {
-    operator_compute_inverse_diagonal(op, nullptr);
-    PMG_CUDA(cudaDeviceSynchronize());
-  }
+  if (!op.has_diag) operator_compute_inverse_diagonal(op, nullptr);
+  PMG_CUDA(cudaDeviceSynchronize()); // streams that do not wait for the default one may use the smoother now
 }
 
 // deal.II PreconditionChebyshev::estimate_eigenvalues: at most eig_its CG steps (tolerance
@@ -248,6 +246,7 @@ void mg_setup(pmg_mg &mg, int n_levels, pmg_operator *const *levels, pmg_transfe
   mg.restrict_residual.assign(n_levels, false);
   for (int l = 1; l < n_levels; ++l) mg.restrict_residual[l] = transfer_restricts_residual(*mg.transfers[l], *mg.levels[l]);
   mg.tail = mg_tail_plan(mg);
+  PMG_CUDA(cudaDeviceSynchronize()); // the plan is on the device
 }
 
 // the cycle from level l down; levels 0 .. tail (-1: none) run in one kernel
