@@ -289,6 +289,15 @@ bool graphs_allowed() {
   return on;
 }
 
+std::vector<int> graph_state(const pmg_mg &mg) {
+  std::vector<int> state;
+  for (size_t l = 0; l < mg.smoothers.size(); ++l) {
+    state.push_back(mg.smoothers[l]->generation);
+    state.push_back(mg.levels[l]->tensor_cores);
+  }
+  return state;
+}
+
 // Capture the cycle into a graph on a private stream (the eigenvalue estimates, which
 // synchronise and allocate, must have run before).  Any failure leaves graph == nullptr
 // and the cycle runs as plain launches.
@@ -312,8 +321,7 @@ void mg_capture(pmg_mg &mg) {
     ok = (cudaStreamEndCapture(cs, &g) == cudaSuccess) && ok;
   }
   if (ok) ok = cudaGraphInstantiate(&mg.graph, g, 0) == cudaSuccess;
-  mg.graph_generations.clear();
-  for (auto *sm : mg.smoothers) mg.graph_generations.push_back(sm->generation);
+  mg.graph_state = graph_state(mg);
   if (g) cudaGraphDestroy(g);
   cudaStreamDestroy(cs);
   if (!ok) {
@@ -330,16 +338,12 @@ void mg_cycle(pmg_mg &mg, cudaStream_t s) {
     if (!sm->estimated) chebyshev_estimate(*sm, s);
     clear_product(*sm, s); // (a replayed graph has no such look)
   }
-  // a graph captured before a smoother was re-estimated holds the old Chebyshev coefficients
-  if (mg.graph) {
-    bool stale = mg.graph_generations.size() != mg.smoothers.size();
-    for (size_t l = 0; !stale && l < mg.smoothers.size(); ++l)
-      stale = mg.graph_generations[l] != mg.smoothers[l]->generation;
-    if (stale) {
-      PMG_CUDA(cudaStreamSynchronize(s));
-      cudaGraphExecDestroy(mg.graph);
-      mg.graph = nullptr;
-    }
+  // a graph captured before a smoother was re-estimated holds the old Chebyshev coefficients, one captured
+  // before a level was switched to or from the tensor cores the other kernels
+  if (mg.graph && mg.graph_state != graph_state(mg)) {
+    PMG_CUDA(cudaStreamSynchronize(s));
+    cudaGraphExecDestroy(mg.graph);
+    mg.graph = nullptr;
   }
   if (mg.graph_enabled && graphs_allowed() && !prof::enabled() && !mg.graph) mg_capture(mg);
   if (mg.graph && !prof::enabled()) PMG_CUDA(cudaGraphLaunch(mg.graph, s));

@@ -36,7 +36,7 @@ struct pmg_mg {
   // launches on fixed buffers: it is captured once into a CUDA graph and replayed.
   cudaGraphExec_t graph = nullptr;
   bool graph_enabled = true;
-  std::vector<int> graph_generations; // smoother estimates the graph was captured with
+  std::vector<int> graph_state; // what the captured launches depend on: each level's estimate and tensor-core mode
   ~pmg_mg() {
     if (graph) cudaGraphExecDestroy(graph);
   }
