@@ -241,10 +241,12 @@ void mg_setup(pmg_mg &mg, int n_levels, pmg_operator *const *levels, pmg_transfe
     const size_t bytes = dtype_size(mg.levels[l]->dtype) * mg.levels[l]->n_dofs;
     mg.sol[l].allocate(bytes);
     mg.def[l].allocate(bytes);
-    mg.t[l].allocate(bytes);
   }
   mg.restrict_residual.assign(n_levels, false);
-  for (int l = 1; l < n_levels; ++l) mg.restrict_residual[l] = transfer_restricts_residual(*mg.transfers[l], *mg.levels[l]);
+  for (int l = 1; l < n_levels; ++l) {
+    mg.restrict_residual[l] = transfer_restricts_residual(*mg.transfers[l], *mg.levels[l]);
+    if (!mg.restrict_residual[l]) mg.t[l].allocate(mg.def[l].bytes());
+  }
   mg.tail = mg_tail_plan(mg);
   PMG_CUDA(cudaDeviceSynchronize()); // the plan is on the device
 }

@@ -29,7 +29,7 @@ struct pmg_mg {
   std::vector<pmg_operator *> levels;
   std::vector<pmg_transfer *> transfers;
   std::vector<pmg_chebyshev *> smoothers;
-  std::vector<pmg::DeviceBuffer> sol, def, t;
+  std::vector<pmg::DeviceBuffer> sol, def, t; // t: the residual, where the restriction does not take it itself
   std::vector<char> restrict_residual; // per level: the restriction to the level below takes def - A sol itself
   std::shared_ptr<pmg::TailPlan> tail; // the coarse levels that run in one kernel, null: none
   // The V-cycle below the finest level's input and output buffers is a fixed sequence of
