@@ -1,19 +1,23 @@
-// DG-SIPG face terms on axis-aligned boxes (the interior-penalty operator of
+// The DG-SIPG operator on axis-aligned boxes (the interior-penalty operator of
 // include/operators/portable_laplace_operator_dg.h with the fluxes of
 // include/kernels/laplace_dg_kokkos_kernels.h:833-2026 and
-// source/plain_laplace_solver_dg/program.cc:128-217).
+// source/plain_laplace_solver_dg/program.cc:128-217): launchers, face diagonal, boundary data.
 //
-// The cell stiffness term comes from the continuous slab kernel run on the discontinuous
-// numbering (dof = cell * N^3 + l).  This file adds the face terms with one fused kernel.
-// Where the box is refined at least twice (every 64 consecutive cells form a 4x4x4 cube) a
-// block takes such a tile into shared memory and evaluates each face between two of its
-// cells once, for both cells; the faces on the tile surface take the neighbour's trace from
-// L2.  Elsewhere a block takes a batch of cells, and for each of the six faces of each cell
-// it forms its own trace (the node layer on the face and the reference normal derivative)
-// and the neighbour's trace, recomputed from the neighbour's DoFs straight from L2, so each
-// face is evaluated from both sides.  The reference instead writes every trace to global
-// face buffers and reads them back in three more launches.  In both forms every block
-// writes only its own cells' DoFs: no global atomics and no face buffers.
+// The vmult and the Chebyshev steps run as dg_line_kernel (dg_line.cuh) at every degree and on
+// every mesh.  The environment variables PMG_DG_FACE and PMG_DG_FUSE select older forms for
+// comparison (64^3 cells, degree 3, FP32 / FP64: 84 / 144 us by lines, 178 / 329 by fused tiles):
+//  * the cell stiffness by the continuous cell kernel on the discontinuous numbering (dof =
+//    cell * N^3 + l), then the face terms with one kernel.  Where the box is refined at least
+//    twice (every 64 consecutive cells form a 4x4x4 cube) a block takes such a tile into shared
+//    memory and evaluates each face between two of its cells once, for both cells; the faces on
+//    the tile surface take the neighbour's trace from L2.  Elsewhere a block takes a batch of
+//    cells, and for each of the six faces of each cell it forms its own trace (the node layer on
+//    the face and the reference normal derivative) and the neighbour's trace, recomputed from the
+//    neighbour's DoFs straight from L2, so each face is evaluated from both sides;
+//  * the cell and face terms of a tile in one kernel (degrees 1 and 3).
+// The reference instead writes every trace to global face buffers and reads them back in three
+// more launches.  In every form here a block writes only its own cells' DoFs: no global atomics
+// and no face buffers.
 //
 // On GLL nodes with the (p+1)-point Gauss face rule the face integrals of products of
 // basis functions are exact, so the face quadrature is applied as the 1D GLL mass matrix
@@ -949,10 +953,10 @@ __global__ void __launch_bounds__(TT, 1024 / TT) dg_tile_fused_kernel(const __gr
   }
 }
 
-// the face form: PMG_DG_FACE=0 the face-by-face kernel, 1 the cell-batch kernel, 2 the tile
-// kernel wherever the mesh allows it (comparison switches, read at every launch); unset: the
-// tile kernel where the mesh allows it and the tiles fill the device at least twice, else the
-// cell-batch kernel
+// the form of separate face terms: PMG_DG_FACE=0 the face-by-face kernel, 1 the cell-batch kernel,
+// 2 the tile kernels wherever the mesh allows them (comparison switches, read at every launch);
+// unset, with PMG_DG_FUSE=0: the face tile kernel where the mesh allows it and the tiles fill the
+// device at least twice, else the cell-batch kernel
 int face_form() {
   const char *e = std::getenv("PMG_DG_FACE");
   if (e && (e[0] == '0' || e[0] == '1' || e[0] == '2') && e[1] == 0) return e[0] - '0';
@@ -1102,7 +1106,7 @@ void face_dispatch(int degree, const DGHost &h, const void *src, void *dst, int6
   }
 }
 
-// PMG_DG_FUSE=0 turns the fused tile kernel off (a comparison switch, read at every launch)
+// PMG_DG_FUSE=0: cell and face terms in launches of their own (a comparison switch, read at every launch)
 bool fuse_allowed() {
   const char *e = std::getenv("PMG_DG_FUSE");
   return !(e && e[0] == '0' && e[1] == 0);
@@ -1116,12 +1120,9 @@ bool fused_launch(const DGHost &h, const void *src, void *dst, int64_t n_cells, 
     return false;
   } else {
     constexpr size_t smem = dg_fused_smem<N, T>();
-    const int form = face_form();
-    if (!fuse_allowed() || !(form == 2 || form < 0) || !h.tiles64 || n_cells % 64 != 0 || smem > 200 * 1024)
-      return false;
+    if (!fuse_allowed() || face_form() != 2 || !h.tiles64 || n_cells % 64 != 0 || smem > 200 * 1024) return false;
     const TileShape sh = tile_shape<N, T, true>();
     const int64_t n_tiles = n_cells / 64;
-    if (form < 0 && n_tiles < 2 * (int64_t)sh.blocks_per_sm * sms) return false;
     if (!launch) return true;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(n_tiles, (int64_t)sh.blocks_per_sm * sms));
     if (units) *units = n_tiles;

@@ -1,4 +1,4 @@
-// DG-SIPG face terms (dg.cu).
+// The DG-SIPG operator (dg.cu).
 #pragma once
 
 #include <vector>
@@ -26,10 +26,10 @@ struct DGChebStep {
   const void *prev, *b, *invd;
   double f1, f2;
 };
-// The whole DG vmult (cell stiffness and face terms) in one tile kernel where it applies
-// (degrees 1 and 3, the box refined at least twice, the tiles filling the device twice or
-// PMG_DG_FACE=2; PMG_DG_FUSE=0 turns it off): dst = A src, written once, or with cheb the
-// Chebyshev step from it.  Returns false, with nothing launched, where it does not apply.
+// The whole DG vmult (cell stiffness and face terms) in one kernel: dst = A src, written once, or
+// with cheb the Chebyshev step from it.  By lines on every mesh; with PMG_DG_FACE=2 by 4x4x4 cell
+// tiles where these apply (degrees 1 and 3, the box refined at least twice).  Returns false, with
+// nothing launched, where neither does (PMG_DG_FACE, PMG_DG_FUSE=0).
 bool dg_apply_fused(const DGHost &h, int degree, int dtype, const void *src, void *dst, int64_t n_cells, int sms,
                     cudaStream_t s, int64_t *units = nullptr, int64_t *blocks = nullptr,
                     const DGChebStep *cheb = nullptr);

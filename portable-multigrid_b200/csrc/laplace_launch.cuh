@@ -155,8 +155,9 @@ template <typename V, int GEOM, typename SH> void line_launch_as(const SlabLaunc
 // Patches per block (cubes of several small lines share one) and blocks per SM, the fastest measured; cells
 // alone, us, patches against cells (FP64 / FP32; 64^3 cells, Q5 32^3, Q6 48^3): Q2 31 / 21 against 52 / 33,
 // Q3 72 / 45 against 85 / 52, Q4 138 / 84 against 176 / 109, Q5 33 / 23 against 41 / 27, Q6 164 / 101 against
-// 216 / 119.  With a coefficient per point only the nodes are shared, and patches were no faster (Q4
-// 257 / 149 against 267 / 156, Q6 373 / 196 against 335 / 194): cells.
+// 216 / 119.  With a coefficient per point only the nodes are shared: patches 4 % faster at Q4 (257 / 149
+// against 267 / 156) and slower at Q6 (373 with spills / 196 against 335 / 194), not enough for a kernel
+// of their own: cells.
 template <typename T> constexpr auto patch_shape() {
   [[maybe_unused]] constexpr bool d = sizeof(T) == 8;
   using kern::PatchShape;

@@ -11,6 +11,8 @@
 // a patch is a coarse cell, so the coarse level's own lists sum what the patches hold.
 //
 // The steps and their arithmetic are those of chebyshev_apply and mg_vcycle (solver.cu).
+// Degree 2 with a coefficient or full geometry, and degrees above, run in launches: a line of such a cell
+// needs three exchange arrays more, and what they would gain has not been measured.
 // (Larger levels on a cluster of 16 blocks with vectors in L2 and atomics were measured as well: 60
 // to 90 us per level of 4,913 DoFs against 58 us in separate launches.)
 #include "mg_tail.hpp"

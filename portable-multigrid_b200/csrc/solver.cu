@@ -204,7 +204,7 @@ void chebyshev_apply(pmg_chebyshev &c, void *dst, const void *src, bool from_zer
     const double f1 = rhokp * rhok, f2 = 2.0 * rhokp / c.delta;
     rhok = rhokp;
     void *out = prev ? prev : (cur == A ? B : A);
-    // DG operators on cell tiles apply the step inside their vmult kernel (A cur never stored)
+    // DG operators apply the step inside their vmult kernel (A cur never stored)
     if (!operator_vmult_chebyshev(op, out, cur, prev, src, op.inv_diag.get(), f1, f2, s)) {
       const vec::Product Ax = open_product(c, cur, s);
       vec::cheb_update(out, cur, prev, src, Ax, op.inv_diag.get(), f1, f2, dt, N, s);

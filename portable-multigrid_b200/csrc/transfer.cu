@@ -29,8 +29,8 @@ template <int NC, int NF, typename T> struct TMat {
 
 template <int NC, int NF> struct PatchShape {
   static constexpr int NF2 = NF * NF;
-  // patches per block: lines of several patches fill its warps (at least 90 % of the lanes but for
-  // the patches of 11^2 and 13^2 lines)
+  // patches per block: lines of several patches fill its warps (at least 94 % of the lanes; one patch
+  // of 13^2 lines 88 %)
   static constexpr int PPB = NF == 3 ? 14 : NF == 4 ? 8 : NF == 5 ? 5 : NF == 6 ? 7 : NF == 7 ? 5 : NF == 9 ? 3 : NF == 11 ? 2 : 1;
   static constexpr int THREADS = (PPB * NF2 + 31) / 32 * 32;
   static constexpr int ROW = NF | 1;                 // x lines of the first exchange, odd stride

@@ -492,7 +492,8 @@ class LaplaceOperator:
         return out.reshape(-1, 6, nq3)
 
     def last_launch(self, kernel=KERNEL_VMULT_CELL):
-        """(work units, warps or blocks) of the last launch of one of the operator's kernels."""
+        """(cells, blocks) or (warp groups, warps) of the last launch of one of the operator's kernels,
+        depending on the kernel (pmg_operator_last_launch)."""
         u, p = C.c_int64(), C.c_int64()
         check(lib().pmg_operator_last_launch(self.h, kernel, C.byref(u), C.byref(p)))
         return u.value, p.value
@@ -580,7 +581,7 @@ class Transfer:
         check(lib().pmg_transfer_restrict_and_add(self.h, _ptr(dst_coarse), _ptr(src_fine), _stream()))
 
     def last_launch(self):
-        """(patches, warps) of the last launch."""
+        """(patches, blocks) of the last launch."""
         u, p = C.c_int64(), C.c_int64()
         check(lib().pmg_transfer_last_launch(self.h, C.byref(u), C.byref(p)))
         return u.value, p.value
