@@ -543,7 +543,7 @@ def dg_time_to_solution(torch, pmg, dev, refine=6, repeats=3):
 
 def dg_vmult_rates(torch, pmg, dev, refine=6, launches=20, peak=None):
     """The DG-SIPG Q3 vmult of config 4 alone (64^3 cells), FP32 and FP64: CUDA-event time per
-    vmult (all its kernels), GDoF/s and the
+    vmult (one kernel), GDoF/s and the
     algorithmic bytes 2 s N + 6 s C (src read and dst written once, six geometry values per
     cell; DG indices are implicit) over that time as a fraction of the HBM peak."""
     p = 3
@@ -568,7 +568,7 @@ def dg_vmult_rates(torch, pmg, dev, refine=6, launches=20, peak=None):
         alg = 2 * s * op.m() + 6 * s * mesh.n_cells()
         units, par = op.last_launch(pmg.KERNEL_DG_FACES)
         out[name] = {"vmult_us": t * 1e6, "gdofs": op.m() / t / 1e9, "algorithmic_bytes": alg,
-                     "frac_of_hbm": alg / t / 1e9 / peak, "tiles": units, "blocks": par}
+                     "frac_of_hbm": alg / t / 1e9 / peak, "cells": units, "blocks": par}
         del op, src, dst
     del mesh
     torch.cuda.empty_cache()
